@@ -270,6 +270,13 @@ __device__ __forceinline__ double mdiv(double a, double b, double y) {
 }
 __device__ __forceinline__ float mdiv(float a, float b, float y) { return a * y; }
 
+// a / b given y, an approximation of 1 / b good to a few ulp: the product corrected once with the
+// residual (Markstein), so within half an ulp and a rounding of the quotient.
+__device__ __forceinline__ double cquot(double a, double b, double y) {
+    const double q = a * y;
+    return fma(fma(-q, b, a), y, q);
+}
+
 // Division of FP64 state quantities (RK update, EOS, renormalisation).  The FP64 form divides
 // in IEEE double, as the reference does.  The FP32 form keeps its state in FP64 only so that
 // small increments survive; there a float reciprocal refined by one Newton step and one

@@ -174,17 +174,22 @@ __device__ __forceinline__ R eos_rho(const Consts& C, R T, const R Y[NSP], R fal
     }
     return fallback;
 }
-// The same on the FP64 state, with the state division of the precision form Form.
+// The same on the FP64 state, with the state division of the precision form Form; irho is an
+// approximation of 1 / rho (a product, no second division) for the quotients by rho.  The gas
+// constant of the mixture is multiplied out (rho = p / ((R sum Y_k / M_k) T): one division
+// instead of three).
 template <typename Form>
-__device__ __forceinline__ double eos_rho_state(const Consts& C, double T, const double Y[NSP], double fallback) {
-    double syw = 0.0;
+__device__ __forceinline__ double eos_rho_state(const Consts& C, double T, const double Y[NSP], double fallback,
+                                                double& irho) {
+    double syw = Y[0] * C.d_mwk[0].r;
 #pragma unroll
-    for (int s = 0; s < NSP; s++) syw += cdv(Y[s], C.d_mwk[s]);
+    for (int s = 1; s < NSP; s++) syw = fma(Y[s], C.d_mwk[s].r, syw);
     if (syw > 1e-9 && T > 1.0) {
-        double W = sdiv<Form>(1.0, syw);
-        double Rm = sdiv<Form>(R_UNIV, W);
-        return sdiv<Form>(P_CONST, Rm * T);
+        const double z = (R_UNIV * syw) * T;
+        irho = z * (1.0 / P_CONST);
+        return sdiv<Form>(P_CONST, z);
     }
+    irho = sdiv<Form>(1.0, fallback);
     return fallback;
 }
 
@@ -647,49 +652,58 @@ __device__ __forceinline__ R weno5_grad(const Consts& C, const R* __restrict__ q
     return cdv(ph - mh, dx);
 }
 
-// superbee_limiter (:2017-2028)
+// MUSCL-superbee (:2017-2028, :2058-2094).  Half the limited slope of a face,
+// 0.5 * superbee(a / b) * b, with a the difference across the face behind and b across the face
+// itself, as the reference defines it: b where |b| < SMALL (it sets r = 1e9, :2064), 0 where a
+// and b differ in sign, otherwise the middle form of superbee without the quotient:
+// superbee(a / b) |b| = min(2 min(|a|, |b|), max(|a|, |b|)).  Exact apart from the reference's
+// rounding of (a / b) * b; a NaN in a alone gives b, as superbee(NaN) = 2 does.
 template <typename R>
-__device__ __forceinline__ R superbee(R r) {
-    if (r <= R(0.0)) return R(0.0);
-    R t1 = fmin(R(2.0) * r, R(1.0));
-    R t2 = fmin(r, R(2.0));
-    return fmax(t1, t2);
+__device__ __forceinline__ R half_slope(R a, R b) {
+    const bool sm = fabs(a) < fabs(b);
+    const R lo = sm ? a : b, hh = R(0.5) * (sm ? b : a);
+    R x = fabs(lo) >= fabs(hh) ? hh : lo;
+    x = (a * b <= R(0.0)) ? R(0.0) : x;
+    return fabs(b) < R(SMALL) ? b : x;
 }
 
-// superbee(dup / ddn) as the reference evaluates it (r = 1e9 when |ddn| < SMALL, :2064),
-// dividing only where the limiter depends on the quotient's value.  For quotients <= 0, in
-// (0.5, 1] or >= 2 the limiter is exactly 0, 1 or 2 whatever the rounding (division is
-// monotonic and 0.5, 1, 2 are representable), and exact comparisons of |dup| with |ddn|
-// decide those cases; NaN operands take the division.
+// One field around a cell, along each axis in the direction of the velocity there: the cell, its
+// upstream and downstream neighbours and the cell two upstream.  Mirrored for a negative
+// velocity, the reference's two branches are the same expression, so the flux difference needs
+// no selects and four values per axis instead of five.
 template <typename R>
-__device__ __forceinline__ R superbee_of(R dup, R ddn) {
-    const R addn = fabs(ddn);
-    if (addn < R(SMALL)) return R(2.0);                   // superbee(1e9)
-    const R adup = fabs(dup);
-    if (adup == adup && addn == addn) {
-        if (dup == R(0) || ((dup > R(0)) != (ddn > R(0)))) return R(0.0);
-        if (adup >= R(2.0) * addn) return R(2.0);
-        if (adup <= addn && adup > R(0.5) * addn) return R(1.0);
+struct Star {
+    R c, up[3], dn[3], uu[3];
+};
+
+// What the advection-diffusion of every scalar of a cell shares.
+template <typename R>
+struct StarCoef {
+    R av[3];            // |velocity| / spacing
+    R gu[3], gd[3];     // (nu_t + nu_t of the neighbour) / (2 Sc_t) / spacing^2, up- and downstream face
+    R lim;              // 1, or 0 in the band where the scheme is first-order upwind (:2043-2052)
+};
+
+// relax * (target - phi) - advection + div((g + D) grad phi) (:2037-2159, :2853-2865, :2932-2944):
+// the face differences are formed once, and feed the limiter, the advection and the diffusion.
+// Differences of neighbours instead of reconstructed face values keep the cancellation exact
+// where the reference rounds face values first.  gr scales the shared SGS coefficients (1 for
+// the mass fractions, Sc_t / Pr_t for the temperature).
+template <typename R, bool UNIT>
+__device__ __forceinline__ R star_rhs(const Star<R>& q, const StarCoef<R>& K, R gr, R D, const R (&ih2)[3], R src) {
+    R k = src;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const R d1 = q.up[a] - q.uu[a], d2 = q.c - q.up[a], d3 = q.dn[a] - q.c;
+        const R t = fma(K.lim, half_slope<R>(d2, d3) - half_slope<R>(d1, d2), d2);
+        const R Dh = D * ih2[a];
+        const R cu = UNIT ? K.gu[a] + Dh : fma(K.gu[a], gr, Dh);
+        const R cd = UNIT ? K.gd[a] + Dh : fma(K.gd[a], gr, Dh);
+        k = fma(-K.av[a], t, k);
+        k = fma(cd, d3, k);
+        k = fma(-cu, d2, k);
     }
-    return superbee<R>(qdiv(dup, ddn));
-}
-
-// MUSCL-superbee along one axis (:2058-2094); values at offsets -2..+2.  Both faces have
-// the same ddn for either sign of the velocity; the sign only selects the upwind value and
-// dup, so the two branches of the reference become selects (base + x or base - x, the same
-// roundings as the reference's two expressions).
-template <typename R>
-__device__ __forceinline__ R muscl_axis(R vel, R pm2, R pm1, R p0, R pp1, R pp2, const DCT<R>& d) {
-    const bool pos = vel >= R(0.0);
-    const R ddn_m = p0 - pm1;
-    const R dup_m = pos ? (pm1 - pm2) : (pp1 - p0);
-    const R x_m = R(0.5) * superbee_of<R>(dup_m, ddn_m) * ddn_m;
-    const R phi_imh = pos ? pm1 + x_m : p0 - x_m;
-    const R ddn_p = pp1 - p0;
-    const R dup_p = pos ? (p0 - pm1) : (pp2 - pp1);
-    const R x_p = R(0.5) * superbee_of<R>(dup_p, ddn_p) * ddn_p;
-    const R phi_iph = pos ? p0 + x_p : pp1 - x_p;
-    return cdv(vel * (phi_iph - phi_imh), d);
+    return k;
 }
 
 // Stencil access to one field around the current cell, q(di, dj, dk): global memory (the
@@ -707,16 +721,6 @@ __device__ __forceinline__ GAcc<R> gacc(const R* p, ptrdiff_t sI, ptrdiff_t sJ) 
     a.p = p; a.sI = sI; a.sJ = sJ;
     return a;
 }
-// NP planes centred on the cell (di in [-NP/2, NP/2]); pl[d] points at the cell's (j, k) in
-// plane i + d - NP/2, rows bw apart.  Every call site passes constant offsets, so pl[] stays
-// in registers.
-template <typename R, int NP>
-struct SAcc {
-    const R* pl[NP];
-    int bw;
-    __device__ __forceinline__ R operator()(int di, int dj, int dk) const { return pl[di + NP / 2][dj * bw + dk]; }
-};
-
 // First-order upwind fallback used by the non-conservative schemes near faces
 // (:642-651, :2043-2052).
 template <typename R, typename A>
@@ -730,17 +734,6 @@ __device__ __forceinline__ R upwind3(const Consts& C, const A& q, R u, R v, R w)
     if (w >= R(0.0)) f += cdv(w * (q(0, 0, 0) - q(0, 0, -1)), K.d_dz);
     else f += cdv(w * (q(0, 0, 1) - q(0, 0, 0)), K.d_dz);
     return f;
-}
-
-// calculate_convection_muscl (:2037-2159)
-template <typename R, typename A>
-__device__ __forceinline__ R conv_muscl(const Consts& C, const A& q, bool band2, R u, R v, R w) {
-    const auto& K = kc<R>(C);
-    if (band2) return upwind3<R>(C, q, u, v, w);
-    R cx = muscl_axis<R>(u, q(-2, 0, 0), q(-1, 0, 0), q(0, 0, 0), q(1, 0, 0), q(2, 0, 0), K.d_dx);
-    R cy = muscl_axis<R>(v, q(0, -2, 0), q(0, -1, 0), q(0, 0, 0), q(0, 1, 0), q(0, 2, 0), K.d_dy);
-    R cz = muscl_axis<R>(w, q(0, 0, -2), q(0, 0, -1), q(0, 0, 0), q(0, 0, 1), q(0, 0, 2), K.d_dz);
-    return cx + cy + cz;
 }
 
 // Face-averaged SGS diffusion div((nu_t/Sc) grad phi) (:2751-2760, :2853-2860, :2932-2939).
@@ -964,16 +957,38 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
 // C2: species (:2837-2904) and temperature (:2912-2962), then the RK4 bookkeeping.
 // stage: 0,1,2 -> intermediate stage with coefficient 0.5/0.5/1.0, 3 -> final combine.
 // Where the scalar pass reads its stencil fields (filtered T and Y_k, nu_t): global memory,
-// or the shared-memory tile of the staged kernel (les_tma.cuh).
+// or the shared-memory tile of the staged kernel (les_tma.cuh).  Element indices are 32-bit: a
+// grid whose fields fit the device has fewer than 2^31 cells.
 template <typename R>
 struct GSrc {
     const R* T;
     const R* Y[NSP];
     const R* nut;
-    ptrdiff_t sI, sJ;
-    __device__ __forceinline__ GAcc<R> y(int s) const { return gacc(Y[s], sI, sJ); }
-    __device__ __forceinline__ GAcc<R> t() const { return gacc(T, sI, sJ); }
-    __device__ __forceinline__ GAcc<R> nu() const { return gacc(nut, sI, sJ); }
+    int id, s[3], up[3], uu[3];         // the cell, the strides, its neighbours upstream
+    __device__ __forceinline__ void orient(const bool (&pos)[3], bool far) {
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const int o = pos[a] ? -s[a] : s[a];
+            up[a] = o;
+            uu[a] = far ? 2 * o : o;    // the band's cells have no second neighbour
+        }
+    }
+    __device__ __forceinline__ void star(const R* p, Star<R>& q) const {
+        q.c = p[id];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            q.up[a] = p[id + up[a]];
+            q.dn[a] = p[id - up[a]];
+            q.uu[a] = p[id + uu[a]];
+        }
+    }
+    __device__ __forceinline__ void y(int sp, Star<R>& q) const { star(Y[sp], q); }
+    __device__ __forceinline__ void t(Star<R>& q) const { star(T, q); }
+    __device__ __forceinline__ void nu(R& c, R (&u)[3], R (&d)[3]) const {
+        c = nut[id];
+#pragma unroll
+        for (int a = 0; a < 3; a++) { u[a] = nut[id + up[a]]; d[a] = nut[id - up[a]]; }
+    }
 };
 
 // One cell of the scalar pass (the body shared by both read paths).
@@ -982,7 +997,7 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
                                                 const PropBuf<R>& P, const F11<RS>& S0, const F11<R>& St,
                                                 const AccBuf<R>& acc, const KFlow<R>& kf, const KDbg<R>& kd,
                                                 const Scalars* __restrict__ Sc, int stage, int i, int j, int k,
-                                                const Src& src, const R relax) {
+                                                Src& src, const R relax) {
     const auto& K = kc<R>(C);
     const int nx = C.nx, ny = C.ny, nz = C.nz;
     const size_t id = cid(i, j, k, ny, nz);
@@ -999,12 +1014,14 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
                 if (q != 5) St.p[q][id] = R(S0.p[q][id]);
 #pragma unroll
             for (int s = 0; s < NSP; s++) Y0[s] = S0.p[6 + s][id];
-            if (a == 2) St.p[5][id] = R(eos_rho_state<R>(C, S0.p[3][id], Y0, S0.p[5][id]));
+            RS unused;
+            if (a == 2) St.p[5][id] = R(eos_rho_state<R>(C, S0.p[3][id], Y0, S0.p[5][id], unused));
         } else if (stage == 3 && a == 2) {
             RS Y0[NSP];
 #pragma unroll
             for (int s = 0; s < NSP; s++) Y0[s] = S0.p[6 + s][id];
-            S0.p[5][id] = eos_rho_state<R>(C, S0.p[3][id], Y0, S0.p[5][id]);
+            RS unused;
+            S0.p[5][id] = eos_rho_state<R>(C, S0.p[3][id], Y0, S0.p[5][id], unused);
         }
         if (kd.p[0]) {
 #pragma unroll
@@ -1013,29 +1030,36 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
         return;
     }
 
-    const R u0 = F.p[0][id], v0 = F.p[1][id], w0 = F.p[2][id];
+    const R vel[3] = {F.p[0][id], F.p[1][id], F.p[2][id]};
     const bool band2 = (i < 2 || i >= nx - 2 || j < 2 || j >= ny - 2 || k < 2 || k >= nz - 2);
     R kv[NACC];
     R g = F.p[4][id];
     if (g < R(0.0)) g = R(0.0);
     if (g > R(1.0)) g = R(1.0);
-    // Temperature; in the FP64 form ahead of the species, which leaves the register allocator
-    // fewer values live across the species loop (spills 100/260 -> 44/148 bytes per thread),
-    // in the FP32 form after them (fewer spills that way round).  Either order gives the same
-    // bits: the two are independent.
-    auto temperature = [&]() {
-        const auto qT = src.t();
-        R conv = conv_muscl<R>(C, qT, band2, u0, v0, w0);
-        R mol = ld_stream(P.aT + id) * lap3<R>(C, qT);
-        const SgsFaces<R> gt = sgs_faces<R>(src.nu(), K.d_prt2);
-        R sgs = sgs_div<R>(C, qT, gt);
-        R Tt = (R)K.t_in + g * (R)K.t_burnt_span;
-        R nud = relax * (Tt - qT(0, 0, 0));
-        kv[3] = -conv + mol + sgs + nud;
-    };
-    constexpr bool kF32s = std::is_same<R, float>::value;
-    if constexpr (!kF32s) temperature();
-    const SgsFaces<R> gs = sgs_faces<R>(src.nu(), K.d_sct2);
+    const bool pos[3] = {vel[0] >= R(0.0), vel[1] >= R(0.0), vel[2] >= R(0.0)};
+    src.orient(pos, !band2);
+    const R ih2[3] = {K.d_dxx.r, K.d_dyy.r, K.d_dzz.r};
+    StarCoef<R> co;
+    co.lim = band2 ? R(0.0) : R(1.0);
+    co.av[0] = fabs(vel[0]) * K.d_dx.r;
+    co.av[1] = fabs(vel[1]) * K.d_dy.r;
+    co.av[2] = fabs(vel[2]) * K.d_dz.r;
+    {
+        R n0, nu[3], nd[3];
+        src.nu(n0, nu, nd);
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const R c = K.d_sct2.r * ih2[q];
+            co.gu[q] = (nu[q] + n0) * c;
+            co.gd[q] = (nd[q] + n0) * c;
+        }
+    }
+    {
+        Star<R> q;
+        src.t(q);
+        const R Tt = fma(g, (R)K.t_burnt_span, (R)K.t_in);
+        kv[3] = star_rhs<R, false>(q, co, K.d_sct2.c * K.d_prt2.r, ld_stream(P.aT + id), ih2, relax * (Tt - q.c));
+    }
 #pragma unroll
     for (int s = 0; s < NSP; s++) {
         R tgt;
@@ -1044,14 +1068,10 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
         else if (s == CO2) tgt = (R)K.inletYk[CO2] + (R)K.prod_co2 * g;
         else if (s == H2O) tgt = (R)K.inletYk[H2O] + (R)K.prod_h2o * g;
         else tgt = (R)K.inletYk[N2];
-        const auto qY = src.y(s);
-        R conv = conv_muscl<R>(C, qY, band2, u0, v0, w0);
-        R mol = ld_stream(P.D[s] + id) * lap3<R>(C, qY);
-        R sgs = sgs_div<R>(C, qY, gs);
-        R nud = relax * (tgt - qY(0, 0, 0));
-        kv[5 + s] = -conv + mol + sgs + nud;
+        Star<R> q;
+        src.y(s, q);
+        kv[5 + s] = star_rhs<R, true>(q, co, R(1.0), ld_stream(P.D[s] + id), ih2, relax * (tgt - q.c));
     }
-    if constexpr (kF32s) temperature();
     kv[0] = ld_stream(kf.p[0] + id);
     kv[1] = ld_stream(kf.p[1] + id);
     kv[2] = ld_stream(kf.p[2] + id);
@@ -1082,11 +1102,11 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
     // the state's FP32 ulp are not rounded away step after step.
     const RS cdt = fin ? (RS)(dt / 6.0) : (RS)((stage == 2 ? 1.0 : 0.5) * dt);
     const RS rho_n = ld_stream(S0.p[5] + id);
-    RS Tn = ld_stream(S0.p[3] + id) + cdt * (RS)incr[3];
-    RS Gn = ld_stream(S0.p[4] + id) + cdt * (RS)incr[4];
+    RS Tn = fma(cdt, (RS)incr[3], ld_stream(S0.p[3] + id));
+    RS Gn = fma(cdt, (RS)incr[4], ld_stream(S0.p[4] + id));
     RS Y[NSP];
 #pragma unroll
-    for (int s = 0; s < NSP; s++) Y[s] = ld_stream(S0.p[6 + s] + id) + cdt * (RS)incr[5 + s];
+    for (int s = 0; s < NSP; s++) Y[s] = fma(cdt, (RS)incr[5 + s], ld_stream(S0.p[6 + s] + id));
     Tn = fmax(RS(200.0), fmin(RS(3000.0), Tn));
     Gn = fmax(RS(0.0), fmin(RS(1.0), Gn));
     RS sy = RS(0);
@@ -1095,26 +1115,29 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
         Y[s] = fmax(RS(0.0), fmin(RS(1.0), Y[s]));
         sy += Y[s];
     }
+    // One reciprocal per divisor; the quotients sharing it are corrected with one fma each.
     if (sy > RS(SMALL)) {
+        const RS y = sdiv<R>(RS(1.0), sy);
 #pragma unroll
-        for (int s = 0; s < NSP; s++) Y[s] = sdiv<R>(Y[s], sy);
+        for (int s = 0; s < NSP; s++) Y[s] = cquot(Y[s], sy, y);
     }
-    RS rn = eos_rho_state<R>(C, Tn, Y, rho_n);
-    RS vel[3];
+    RS irn;
+    const RS rn = eos_rho_state<R>(C, Tn, Y, rho_n, irn);
+    RS vn[3];
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-        RS m = rho_n * ld_stream(S0.p[q] + id) + cdt * (RS)incr[q];   // rhou = rho*u after the BC (:3146)
-        vel[q] = (rn > RS(SMALL)) ? sdiv<R>(m, rn) : RS(0);
+        RS m = fma(cdt, (RS)incr[q], rho_n * ld_stream(S0.p[q] + id));   // rhou = rho*u after the BC (:3146)
+        vn[q] = (rn > RS(SMALL)) ? cquot(m, rn, irn) : RS(0);
     }
     if (fin) {
         RS* const* out = S0.p;
-        out[0][id] = vel[0]; out[1][id] = vel[1]; out[2][id] = vel[2];
+        out[0][id] = vn[0]; out[1][id] = vn[1]; out[2][id] = vn[2];
         out[3][id] = Tn; out[4][id] = Gn; out[5][id] = rn;
 #pragma unroll
         for (int s = 0; s < NSP; s++) out[6 + s][id] = Y[s];
     } else {
         R* const* out = St.p;
-        out[0][id] = R(vel[0]); out[1][id] = R(vel[1]); out[2][id] = R(vel[2]);
+        out[0][id] = R(vn[0]); out[1][id] = R(vn[1]); out[2][id] = R(vn[2]);
         out[3][id] = R(Tn); out[4][id] = R(Gn); out[5][id] = R(rn);
 #pragma unroll
         for (int s = 0; s < NSP; s++) out[6 + s][id] = R(Y[s]);
@@ -1152,12 +1175,14 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
     if (k >= nz || j >= ny || i >= C.nx) return;
     const size_t id = cid(i, j, k, ny, nz);
     GSrc<R> src;
-    src.sI = (ptrdiff_t)ny * nz;
-    src.sJ = (ptrdiff_t)nz;
-    src.T = F.p[3] + id;
+    src.id = (int)id;
+    src.s[0] = ny * nz;
+    src.s[1] = nz;
+    src.s[2] = 1;
+    src.T = F.p[3];
 #pragma unroll
-    for (int s = 0; s < NSP; s++) src.Y[s] = F.p[6 + s] + id;
-    src.nut = P.nu_t + id;
+    for (int s = 0; s < NSP; s++) src.Y[s] = F.p[6 + s];
+    src.nut = P.nu_t;
     rhs_scalar_cell<R, RS>(C, attr, F, P, S0, St, acc, kf, kd, Sc, stage, i, j, k, src, relax);
 }
 

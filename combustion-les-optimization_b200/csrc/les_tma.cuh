@@ -48,13 +48,43 @@ struct TmaMaps {
     CUtensorMap nut;
 };
 
-template <typename R, int NP>
-struct SSrcPlanes {
-    SAcc<R, 5> Yv[NSP], Tv;
-    SAcc<R, 3> Nv;
-    __device__ __forceinline__ const SAcc<R, 5>& y(int s) const { return Yv[s]; }
-    __device__ __forceinline__ const SAcc<R, 5>& t() const { return Tv; }
-    __device__ __forceinline__ const SAcc<R, 3>& nu() const { return Nv; }
+// The staged planes as the source of a cell's stars: five planes of each field and three of
+// nu_t, centred on the cell, rows BW values apart.  The axis across planes picks its plane by the
+// sign of the velocity, the other two their offset.
+template <typename R>
+struct SSrc {
+    const R *T[5], *Y[NSP][5], *nut[3];
+    bool pos0, far;
+    int o1, o2;                         // offsets of the upstream neighbours in a plane
+    __device__ __forceinline__ void orient(const bool (&pos)[3], bool f) {
+        pos0 = pos[0];
+        far = f;
+        o1 = pos[1] ? -TmaGeom<R>::BW : TmaGeom<R>::BW;
+        o2 = pos[2] ? -1 : 1;
+    }
+    __device__ __forceinline__ void star(const R* const (&pl)[5], Star<R>& q) const {
+        q.c = pl[2][0];
+        q.up[0] = *(pos0 ? pl[1] : pl[3]);
+        q.dn[0] = *(pos0 ? pl[3] : pl[1]);
+        q.uu[0] = *(pos0 ? (far ? pl[0] : pl[1]) : (far ? pl[4] : pl[3]));
+        q.up[1] = pl[2][o1];
+        q.dn[1] = pl[2][-o1];
+        q.uu[1] = pl[2][far ? 2 * o1 : o1];
+        q.up[2] = pl[2][o2];
+        q.dn[2] = pl[2][-o2];
+        q.uu[2] = pl[2][far ? 2 * o2 : o2];
+    }
+    __device__ __forceinline__ void y(int sp, Star<R>& q) const { star(Y[sp], q); }
+    __device__ __forceinline__ void t(Star<R>& q) const { star(T, q); }
+    __device__ __forceinline__ void nu(R& c, R (&u)[3], R (&d)[3]) const {
+        c = nut[1][0];
+        u[0] = *(pos0 ? nut[0] : nut[2]);
+        d[0] = *(pos0 ? nut[2] : nut[0]);
+        u[1] = nut[1][o1];
+        d[1] = nut[1][-o1];
+        u[2] = nut[1][o2];
+        d[2] = nut[1][-o2];
+    }
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -184,25 +214,21 @@ __global__ void __launch_bounds__(TMA_TK* TMA_TJ, (sizeof(R) == 8) ? 2 : 3)
             for (int q = 0; q < 5; q++) asm volatile("prefetch.global.L2 [%0];" ::"l"(F.p[q] + idn));
         }
         if (k < C.nz && j < C.ny) {
-            SSrcPlanes<R, 5> src;
+            SSrc<R> src;
 #pragma unroll
             for (int d = 0; d < 5; d++) {
                 const int slot = (rc - 2 + d) % TMA_RING;
                 const int off = (jl + 2) * G::BW + (kl + G::KOFF);
 #pragma unroll
-                for (int s = 0; s < NSP; s++) src.Yv[s].pl[d] = fring + (size_t)(s * TMA_RING + slot) * (G::FBYTES / sizeof(R)) + off;
-                src.Tv.pl[d] = fring + (size_t)(NSP * TMA_RING + slot) * (G::FBYTES / sizeof(R)) + off;
+                for (int s = 0; s < NSP; s++) src.Y[s][d] = fring + (size_t)(s * TMA_RING + slot) * (G::FBYTES / sizeof(R)) + off;
+                src.T[d] = fring + (size_t)(NSP * TMA_RING + slot) * (G::FBYTES / sizeof(R)) + off;
             }
-#pragma unroll
-            for (int s = 0; s < NSP; s++) src.Yv[s].bw = G::BW;
-            src.Tv.bw = G::BW;
 #pragma unroll
             for (int d = 0; d < 3; d++) {
                 const int nslot = (rc - 1 + d + 1) % TMA_NRING;   // nu plane i-1+d arrived with step rc-1+d+1
-                src.Nv.pl[d] = reinterpret_cast<const R*>(nbase + nslot * G::NSTRIDE) + (jl + 1) * G::BW +
-                               (kl + G::KOFF);
+                src.nut[d] = reinterpret_cast<const R*>(nbase + nslot * G::NSTRIDE) + (jl + 1) * G::BW +
+                             (kl + G::KOFF);
             }
-            src.Nv.bw = G::BW;
             rhs_scalar_cell<R, RS>(C, attr, F, P, S0, St, acc, kf, kd, Sc, stage, i, j, k, src, (R)kc<R>(C).relax);
         }
         __syncthreads();                            // the plane of step rc - 2 is free
