@@ -53,6 +53,60 @@ int cuda_fail(lesgpu_ctx* c, cudaError_t e, const char* where) {
 
 bool all_zero4(const double* c) { return c[0] == 0.0 && c[1] == 0.0 && c[2] == 0.0 && c[3] == 0.0; }
 
+// The property constants of ordinary cells, formed in extended precision and rounded once, and
+// whether the kernels may use them: the binary fits symmetric, one T_mid, no all-zero fit (the
+// reference takes 0 for those), and over FIT_TMIN..FIT_TMAX every fit smooth between samples and
+// small enough for exp2_fit, and every D_ab well inside (1e-12, 1e2), where the reference's skip
+// rules cannot apply.
+void build_fits(const lesgpu_species& sp, les::Consts& C) {
+    const long double step = (long double)les::EXP_STEPS / logl(2.0L);
+    bool ok = C.dco_sym != 0;
+    auto set = [&](double (&f)[4], const double* c, long double power, long double ln_unit) {
+        for (int q = 0; q < 4; q++) f[q] = (double)(power * step * ((long double)c[q] + (q == 0 ? ln_unit : 0.0L)));
+        const double l0 = log(les::FIT_TMIN), l1 = log(les::FIT_TMAX);
+        double last = 0.0;
+        for (int n = 0; n <= 1024; n++) {
+            const double L = l0 + (l1 - l0) * n / 1024.0;
+            const double v = c[0] + L * (c[1] + L * (c[2] + L * c[3]));
+            if (!(fabs(v) < 300.0) || (n > 0 && !(fabs(v - last) < 0.5))) ok = false;
+            last = v;
+        }
+    };
+    auto between = [&](const double* c, double lo, double hi) {
+        const double l0 = log(les::FIT_TMIN), l1 = log(les::FIT_TMAX);
+        for (int n = 0; n <= 1024; n++) {
+            const double L = l0 + (l1 - l0) * n / 1024.0;
+            const double v = c[0] + L * (c[1] + L * (c[2] + L * c[3]));
+            if (!(v > lo && v < hi)) ok = false;
+        }
+    };
+    int p = 0;
+    for (int a = 0; a < les::NSP; a++) {
+        if (C.eta_zero[a] || C.lam_zero[a] || sp.t_mid[a] != sp.t_mid[0] || !(C.mwk[a] >= 1e-9)) ok = false;
+        set(C.f_smu[a], sp.eta[a], 0.5L, logl(0.1L));
+        set(C.f_lam[a], sp.lambda[a], 1.0L, logl(1e-5L));
+        between(sp.eta[a], -60.0, 30.0);
+        between(sp.lambda[a], -60.0, 60.0);
+        for (int b = a + 1; b < les::NSP; b++, p++) {
+            if (C.dco_zero[a][b]) ok = false;
+            set(C.f_idif[p], sp.dcoef[a][b], -1.0L, -logl(1e4L));
+            between(sp.dcoef[a][b], log(1e-8) + 1.0, log(1e6) - 1.0);      // cm^2/s
+        }
+        for (int b = 0; b < les::NSP; b++) {
+            const long double rs = 1.0L / sqrtl((long double)C.wden[a][b]);
+            C.w0[a][b] = (double)rs;
+            C.w1[a][b] = (double)((long double)C.wpow[a][b] * rs);
+        }
+        for (int q = 0; q < 5; q++) {
+            C.cp_high[a][q] = (double)((long double)sp.nasa_high[a][q] * (long double)les::R_UNIV / (long double)C.mwk[a]);
+            C.cp_low[a][q] = (double)((long double)sp.nasa_low[a][q] * (long double)les::R_UNIV / (long double)C.mwk[a]);
+        }
+    }
+    C.t_split = sp.t_mid[0];
+    for (int j = 0; j < les::EXP_STEPS; j++) C.exp_tab[j] = (double)exp2l((long double)j / les::EXP_STEPS);
+    C.fit_ok = ok ? 1 : 0;
+}
+
 // Constant table: grid spacings and the species/model constants in the form the kernels use.
 void build_consts(const lesgpu_config& g, const lesgpu_species& sp, les::Consts& C) {
     memset(&C, 0, sizeof(C));
@@ -141,6 +195,7 @@ void build_consts(const lesgpu_config& g, const lesgpu_species& sp, les::Consts&
         C.d_tenows[q] = dc(q == 0 ? 1.0 : ws);
     }
     C.ssr_exp = 2.0 - C.d3;                                             // :1946
+    build_fits(sp, C);
     les::fill_float_consts(C);
 }
 

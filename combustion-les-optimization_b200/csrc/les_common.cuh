@@ -13,6 +13,7 @@ namespace les {
 constexpr int NSP = 5;
 constexpr int C3H8 = 0, O2 = 1, N2 = 2, CO2 = 3, H2O = 4;   // :129-133
 constexpr int NSTATE = 11;                                  // u v w T G rho Y0..Y4
+constexpr int NPAIR = NSP * (NSP - 1) / 2;                  // unordered species pairs
 constexpr int NACC = 10;                                    // rhou rhov rhow T G Y0..Y4
 // thread-block shape of the per-cell passes: 32 consecutive k-cells x 8 j-rows
 constexpr int BX = 32, BY = 8, NT = BX * BY;
@@ -30,6 +31,11 @@ constexpr double TENO_CUT = 1.0e-6;
 constexpr double FORCE_LIMIT = 500.0;
 constexpr double RAMP_DIST = 0.03;
 constexpr double SSR_A = 0.2340, SSR_B = 0.2187;
+
+// The temperatures over which the property fits are checked when a context is made; cells
+// outside them take the general path.
+constexpr double FIT_TMIN = 150.0, FIT_TMAX = 4000.0;
+constexpr int EXP_STEPS = 16;           // table steps per octave of exp2_fit
 
 // A divisor with its reciprocal rounded to nearest.  x / c is evaluated as q = x*r followed
 // by one fma correction q + (x - q*c)*r (Markstein's iteration), which returns the
@@ -62,7 +68,9 @@ struct ModelK {
     X(u_in, ) X(noise_amp, )                                                                     \
     XD(d_dx, ) XD(d_dy, ) XD(d_dz, ) XD(d_2dx, ) XD(d_2dy, ) XD(d_2dz, ) XD(d_dxx, ) XD(d_dyy, ) \
     XD(d_dzz, ) XD(d_six, ) XD(d_filter, ) XD(d_sct2, ) XD(d_prt2, ) XD(d_ramp, ) XD(d_w2, )      \
-    XD(d_tau_sl, ) XD(d_mwk, [NSP]) XD(d_wden, [NSP][NSP]) XD(d_tenows, [8])
+    XD(d_tau_sl, ) XD(d_mwk, [NSP]) XD(d_wden, [NSP][NSP]) XD(d_tenows, [8])                     \
+    X(t_split, ) X(cp_high, [NSP][5]) X(cp_low, [NSP][5]) X(w0, [NSP][NSP]) X(w1, [NSP][NSP])                  \
+    X(f_smu, [NSP][4]) X(f_lam, [NSP][4]) X(f_idif, [NPAIR][4])
 
 struct ConstsF {
 #define LES_DECL_F(name, dims) float name dims;
@@ -112,6 +120,17 @@ struct Consts {
     double u_in, noise_amp;             // INLET_VELOCITY, 0.10*INLET_VELOCITY
     double ti_rms;                      // INLET_VELOCITY * INLET_TURBULENCE_INTENSITY
     double ssr_exp;                     // 2.0 - D3, the SSR-SGS wrinkling exponent
+    // Mixture properties of an ordinary cell (les_kernels.cuh, cell_props): the fits as cubics in
+    // ln T of the base-2 exponent times EXP_STEPS, unit factors included.
+    int fit_ok;                         // the fits are tame over FIT_TMIN..FIT_TMAX and symmetric
+    int pad2;
+    double t_split;                     // the T_mid of all species
+    double cp_high[NSP][5], cp_low[NSP][5];   // NASA-7 cp coefficients times R / M_k
+    double w0[NSP][NSP], w1[NSP][NSP];  // Wilke: wden^-1/2 and wpow wden^-1/2
+    double f_smu[NSP][4];               // sqrt(mu_k)
+    double f_lam[NSP][4];               // lambda_k
+    double f_idif[NPAIR][4];            // 1 / D_ab, pairs (a < b) in ascending order
+    double exp_tab[16];                 // 2^(j/16)
     ConstsF f;                          // float copies for the FP32 form
 };
 
@@ -156,6 +175,14 @@ inline void fill_float_consts(Consts& C) {
 #define LES_CONV(name, dims) to_float(C.f.name, C.name);
     LES_FCONSTS(LES_CONV, LES_CONV)
 #undef LES_CONV
+    // the FP32 form's fits are plain base-2 exponents (ex2.approx)
+    for (int q = 0; q < 4; q++) {
+        for (int s = 0; s < NSP; s++) {
+            C.f.f_smu[s][q] = (float)(C.f_smu[s][q] / EXP_STEPS);
+            C.f.f_lam[s][q] = (float)(C.f_lam[s][q] / EXP_STEPS);
+        }
+        for (int p = 0; p < NPAIR; p++) C.f.f_idif[p][q] = (float)(C.f_idif[p][q] / EXP_STEPS);
+    }
 }
 
 // A batched launch (les_launch.cuh, batch_stages) steps several members of one grid shape in
@@ -291,6 +318,44 @@ __device__ __forceinline__ double sdiv<float>(double a, double b) {
     y = fma(y, fma(-b, y, 1.0), y);
     const double q = a * y;
     return fma(fma(-q, b, a), y, q);
+}
+
+// 1 / x for a positive x far from the ends of the range: the hardware's approximation (about 20
+// bits) and one third-order Newton (Householder) step, y (1 + e + e^2) with e = 1 - x y: 2^-60 and
+// the rounding, in 4 instructions without the general division's checks and branch.
+__device__ __forceinline__ double frcp(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ float frcp(float x) { return __fdividef(1.0f, x); }
+__device__ __forceinline__ float cquot(float a, float b, float y) { return a * y; }
+
+// 2^(t / EXP_STEPS) for |t| < 16000, t a fit's value: Tang's table-driven method (ACM TOMS 15,
+// 1989) in base 2.  t = k + r with an integer k and |r| <= 1/2, both exact, so no constant has to
+// be subtracted in two parts; 2^(k/16) is a table entry and an exponent, 2^(r/16) - 1 a
+// degree-6 polynomial (Chebyshev interpolation, error 1.5e-17).  The table is one shared-memory
+// line of 16 banks, so a warp reads it without conflicts.  Error within 1.1 ulp of 2^(t/16).
+__device__ __forceinline__ double exp2_fit(double t, const double* tab) {
+    const double magic = 6755399441055744.0;                     // 1.5 * 2^52: rounds to an integer
+    const double s = t + magic;
+    const int k = __double2loint(s);
+    const double r = t - (s - magic);
+    double p = 9.181334960907254e-12;
+    p = fma(p, r, 1.2716085030349987e-09);
+    p = fma(p, r, 1.4676100321837672e-07);
+    p = fma(p, r, 1.355080777749983e-05);
+    p = fma(p, r, 0.0009383847928089873);
+    p = fma(p, r, 0.04332169878499661);
+    const double v = tab[k & (EXP_STEPS - 1)];
+    const double y = fma(v, p * r, v);
+    return __hiloint2double(__double2hiint(y) + ((k >> 4) << 20), __double2loint(y));
+}
+__device__ __forceinline__ float exp2_fit(float t, const double*) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(t));
+    return y;
 }
 
 // x^3 and x^4 rounded once: glibc pow() returns the correctly rounded power for these

@@ -193,13 +193,23 @@ __device__ __forceinline__ double eos_rho_state(const Consts& C, double T, const
     return fallback;
 }
 
-// Cell-local mixture properties of one fluid cell (attr == 3).
-// The diffusivities D_k are handed to store_d as soon as they are known (before the mixing
-// rules, so that they and the fit polynomial's powers of ln T are not held across them).
-template <typename R, typename StoreD>
-__device__ __forceinline__ void cell_props(const Consts& C, R Tl, const R Yf[NSP], R rhof, R& mu_mix, R& nu,
-                                           const StoreD& store_d, R& aT, R& cp_out, R& lam_out, R& alpha) {
+// What the properties of a cell are kept in.
+template <typename R>
+struct CellProps {
+    R D[NSP], mu_mix, nu, aT, cp, lam, alpha;
+};
+
+// Cell-local mixture properties of one fluid cell (attr == 3), general path: any temperature, any
+// composition, any fits, by the reference's own rules term by term.  Called, not inlined: ordinary
+// cells (cell_props_fast) never come here, and the instructions of this path in their way cost the
+// pass instruction-cache misses.
+template <typename R>
+__device__ __noinline__ void cell_props_any(const Consts& C, R Tl, const R* Yf, R rhof, CellProps<R>* out) {
     const auto& K = kc<R>(C);
+    R &mu_mix = out->mu_mix, &nu = out->nu, &aT = out->aT, &cp_out = out->cp, &lam_out = out->lam, &alpha = out->alpha;
+    auto store_d = [&](const R* D) {
+        for (int s = 0; s < NSP; s++) out->D[s] = D[s];
+    };
     R X[NSP];
     R syw = R(0);
     bool tpos = Tl > R(0);
@@ -376,6 +386,112 @@ __device__ __forceinline__ void cell_props(const Consts& C, R Tl, const R Yf[NSP
     aT = q;
 }
 
+// The same for an ordinary cell: FIT_TMIN < T < FIT_TMAX, some mass, no pure species, fits that
+// passed the host's check.  False where the cell is not one.  No branches but the choice of
+// NASA range: species below the reference's X = 1e-12 take part with weight 0, which is what its
+// skips amount to.  Against the general path per cell: 20 exponentials of 17 instructions
+// instead of about 35 each (exp2_fit; the unit factors and 1/2 of the square roots are in the
+// fits), no square roots, Wilke's denominators folded into two constants a pair, cp as one
+// polynomial of the mixture, and reciprocals without the general division's checks.
+// The diffusivities go to store_d as soon as they are known, so that they are not held across the
+// mixing rules.
+template <typename R, typename StoreD>
+__device__ __forceinline__ bool cell_props_fast(const Consts& C, const double* tab, R Tl, const R* Yf, R rhof,
+                                                const StoreD& store_d, CellProps<R>& o) {
+    const auto& K = kc<R>(C);
+    R X[NSP];
+    R syw = R(0);
+#pragma unroll
+    for (int s = 0; s < NSP; s++) {
+        X[s] = Yf[s] * K.d_mwk[s].r;
+        syw += X[s];
+    }
+    if (!(C.fit_ok && Tl > R(FIT_TMIN) && Tl < R(FIT_TMAX) && syw >= R(1e-9) && syw < R(1e9) && rhof > R(1e-3) &&
+          rhof < R(1e9)))
+        return false;
+    const R isyw = frcp(syw);
+    bool pure = false;
+#pragma unroll
+    for (int s = 0; s < NSP; s++) {
+        X[s] *= isyw;
+        pure = pure || fabs(R(1.0) - X[s]) < R(1e-9);
+    }
+    if (pure) return false;
+    const R L = qlog(Tl);
+    auto fit = [&](const auto& c) { return exp2_fit(fma(fma(fma((R)c[3], L, (R)c[2]), L, (R)c[1]), L, (R)c[0]), tab); };
+    R w[NSP];
+#pragma unroll
+    for (int s = 0; s < NSP; s++) w[s] = X[s] > R(1e-12) ? X[s] : R(0);
+    {
+        // Hirschfelder-Curtiss (:1716-1749), sums over b != a in ascending b; the pressure factor
+        // PATM / (p0 + P_f) (:1743-1746) is exactly 1, P being identically zero in the reference
+        R sx[NSP];
+#pragma unroll
+        for (int s = 0; s < NSP; s++) sx[s] = R(0);
+        int p = 0;
+#pragma unroll
+        for (int a = 0; a < NSP; a++)
+#pragma unroll
+            for (int b = a + 1; b < NSP; b++, p++) {
+                const R y = fit(K.f_idif[p]);
+                sx[a] = fma(w[b], y, sx[a]);
+                sx[b] = fma(w[a], y, sx[b]);
+            }
+#pragma unroll
+        for (int s = 0; s < NSP; s++) {
+            const R d = (R(1.0) - X[s]) * frcp(sx[s]);
+            o.D[s] = fmax(R(1e-9), fmin(R(1e-2), sx[s] > R(1e-12) ? d : R(1e-5)));
+        }
+        store_d(o.D);
+    }
+    // cp (:1772-1786)
+    R c[5];
+#pragma unroll
+    for (int q = 0; q < 5; q++) c[q] = R(0);
+    if (Tl > K.t_split) {
+#pragma unroll
+        for (int s = 0; s < NSP; s++)
+#pragma unroll
+            for (int q = 0; q < 5; q++) c[q] = fma(Yf[s], (R)K.cp_high[s][q], c[q]);
+    } else {
+#pragma unroll
+        for (int s = 0; s < NSP; s++)
+#pragma unroll
+            for (int q = 0; q < 5; q++) c[q] = fma(Yf[s], (R)K.cp_low[s][q], c[q]);
+    }
+    const R Cp = fmax(R(100.0), fma(fma(fma(fma(c[4], Tl, c[3]), Tl, c[2]), Tl, c[1]), Tl, c[0]));
+    // Wilke (:1530-1546) and Wassiljew (:1842-1863): the same phi_ab, skip rule and order of
+    // summation, so one denominator serves both; phi_ab = (w0 + w1 sqrt(mu_a / mu_b))^2, phi_aa = 1
+    R smu[NSP], ismu[NSP];
+#pragma unroll
+    for (int s = 0; s < NSP; s++) {
+        smu[s] = fit(K.f_smu[s]);
+        ismu[s] = frcp(smu[s]);
+    }
+    R mu = R(0), lam = R(0);
+#pragma unroll
+    for (int a = 0; a < NSP; a++) {
+        R den = w[a];
+#pragma unroll
+        for (int b = 0; b < NSP; b++) {
+            if (b == a) continue;
+            const R t = fma(smu[a] * ismu[b], (R)K.w1[a][b], (R)K.w0[a][b]);
+            den = fma(w[b] * t, t, den);
+        }
+        const R q = den > R(1e-9) ? w[a] * frcp(den) : R(0);
+        mu = fma(q * smu[a], smu[a], mu);
+        lam = fma(q, fit(K.f_lam[a]), lam);
+    }
+    o.cp = Cp;
+    o.mu_mix = fmax(R(1e-7), mu);
+    o.lam = fmax(R(1e-3), lam);
+    const R rc = rhof * Cp, irc = frcp(rc);
+    o.nu = fmax(R(1e-7), cquot(o.mu_mix, rhof, Cp * irc));
+    o.aT = cquot(o.lam, rc, irc);
+    o.alpha = fmax(R(1e-7), o.aT);
+    return true;
+}
+
 // ------------------------------------------------------------------ pass A: filter + props
 
 template <typename R, typename RI = R, bool BATCH = false>
@@ -385,6 +501,7 @@ __global__ void __launch_bounds__(NT, MinBlocks<R>::filter)
     const auto& K = kc<R>(C);
     __shared__ double sh[NT / 32];
     __shared__ bool last;
+    __shared__ double tab[EXP_STEPS];
     int bz = blockIdx.z;
     if constexpr (BATCH) {
         const int m = blockIdx.z / B.gz;
@@ -403,37 +520,54 @@ __global__ void __launch_bounds__(NT, MinBlocks<R>::filter)
     const int i = bz * blockDim.z + threadIdx.z;
     const int tid = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
     const ptrdiff_t sI = (ptrdiff_t)ny * nz, sJ = (ptrdiff_t)nz;
+    if (std::is_same<R, double>::value && tid < EXP_STEPS) tab[tid] = C.exp_tab[tid];
     double mass = 0.0, mnu = 0.0, mal = 0.0;
-    if (k < nz && j < ny && i < C.nx) {
-        const size_t id = cid(i, j, k, ny, nz);
-        const int a = attr[id];
+    const bool here = k < nz && j < ny && i < C.nx;
+    const size_t id = here ? cid(i, j, k, ny, nz) : 0;
+    const int a = here ? attr[id] : 0;
+    R f[NSTATE];
+    if (here) {
         const bool filt = (a == 3) && i >= 1 && i < nx - 1 && j >= 1 && j < ny - 1 && k >= 1 && k < nz - 1;
-        R f[NSTATE];
+        // (50 x + six neighbours) / 56 (:1307-1470) as x + (neighbours - 6 x) / 56: fewer roundings
+        // at the size of x, and a uniform field stays exactly what it is.  In the input's type:
+        // the FP32 form's first stage reads the FP64 state and converts one value instead of seven.
 #pragma unroll
         for (int q = 0; q < NSTATE; q++) {
             const RI* __restrict__ x = in.p[q] + id;
-            if (filt) {
-                f[q] = cdv(R(x[-sI]) + R(x[-sJ]) + R(x[-1]) + R(FILTER_W) * R(x[0]) + R(x[1]) + R(x[sJ]) + R(x[sI]),
-                           K.d_filter);
-            } else {
-                f[q] = R(x[0]);
-            }
-            F.p[q][id] = f[q];
+            const RI x0 = x[0];
+            RI v = x0;
+            if (filt) v = fma(fma(RI(-6.0), x0, x[-sI] + x[-sJ] + x[-1] + x[1] + x[sJ] + x[sI]), RI(1.0 / 56.0), x0);
+            f[q] = R(v);
         }
+        // stored after the last load: a store may alias the next field's loads as far as the
+        // compiler knows, and would make them wait for this field's
+#pragma unroll
+        for (int q = 0; q < NSTATE; q++) F.p[q][id] = f[q];
+    }
+    if constexpr (std::is_same<R, double>::value) __syncthreads();   // exp2_fit's table
+    if (here) {
         if (a == 1 || a == 2 || a == 3 || a == 5) mass = (((double)f[5] * C.dx) * C.dy) * C.dz;
         if (a == 3) {
-            R mu_mix, nu, aT, cp, lam, alpha;
+            CellProps<R> o;
             auto store_d = [&](const R* D) {
 #pragma unroll
                 for (int s = 0; s < NSP; s++) P.D[s][id] = D[s];
             };
-            cell_props<R>(C, f[3], &f[6], f[5], mu_mix, nu, store_d, aT, cp, lam, alpha);
-            P.mu_mix[id] = mu_mix;
-            P.nu[id] = nu;
-            P.aT[id] = aT;
-            if (P.dbg_cp) { P.dbg_cp[id] = cp; P.dbg_lam[id] = lam; P.dbg_alpha[id] = alpha; }
-            mnu = (double)nu;
-            mal = (double)alpha;
+            if (!cell_props_fast<R>(C, tab, f[3], &f[6], f[5], store_d, o)) {
+                CellProps<R> g;
+                R Yf[NSP];
+#pragma unroll
+                for (int s = 0; s < NSP; s++) Yf[s] = f[6 + s];
+                cell_props_any<R>(C, f[3], Yf, f[5], &g);
+                store_d(g.D);
+                o = g;
+            }
+            P.mu_mix[id] = o.mu_mix;
+            P.nu[id] = o.nu;
+            P.aT[id] = o.aT;
+            if (P.dbg_cp) { P.dbg_cp[id] = o.cp; P.dbg_lam[id] = o.lam; P.dbg_alpha[id] = o.alpha; }
+            mnu = (double)o.nu;
+            mal = (double)o.alpha;
         } else if (P.dbg_cp) {
             // property values of non-fluid cells are never read by the step; they are filled
             // only for inspection, with the reference's defaults
