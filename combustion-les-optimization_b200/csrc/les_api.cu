@@ -485,7 +485,10 @@ int lesgpu_create(const lesgpu_config* cfg, const lesgpu_species* sp, lesgpu_ctx
     for (int s = 0; s < les::NSP; s++) d.D[s] = take();
     d.aT = take(); d.nu_t = take(); d.S_mag = take(); d.ST = take(); d.mu_eff = take();
     for (int q = 0; q < les::NACC; q++) d.acc[q] = take();
-    for (int q = 0; q < 4; q++) d.kflow[q] = take();
+    // the FP64 density handed from the scalar to the flow pass; four fields of the form's type, so
+    // that it fits and a context's size per cell is what admission by memory has always counted
+    d.rn = take();
+    for (int q = 0; q < 3; q++) (void)take();
     // per-block partials: 3 per block of the per-cell grid (filter pass, any tile shape) and
     // 6 per block of the monitor grid
     size_t nb = les::max_cell_blocks(d.nx, d.ny, d.nz);
@@ -1367,8 +1370,7 @@ bool batchable(const DevCtx& a, const DevCtx& b) {
             return false;
     for (int q = 0; q < les::NACC; q++)
         if (off(a, a.acc[q]) != off(b, b.acc[q])) return false;
-    for (int q = 0; q < 4; q++)
-        if (off(a, a.kflow[q]) != off(b, b.kflow[q])) return false;
+    if (off(a, a.rn) != off(b, b.rn)) return false;
     if (off(a, a.mu_mix) != off(b, b.mu_mix) || off(a, a.nu_t) != off(b, b.nu_t) || off(a, a.mu_eff) != off(b, b.mu_eff))
         return false;
     const les::Consts ca = masked_consts(a.hC), cb = masked_consts(b.hC);

@@ -70,7 +70,7 @@ struct DevCtx {
     void* ST = nullptr;
     void* mu_eff = nullptr;
     void* acc[NACC] = {};
-    void* kflow[4] = {};                // momentum and G right-hand sides of the stage
+    void* rn = nullptr;                 // new density of the stage (FP64), scalar pass to flow pass
     void* dbg_cp = nullptr;             // optional inspection buffers (lesgpu_get_field)
     void* dbg_lam = nullptr;
     void* dbg_alpha = nullptr;

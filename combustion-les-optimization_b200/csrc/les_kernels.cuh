@@ -9,9 +9,11 @@
 //                       :1762, update_lambda_mix_alpha :1798); partial sums for <rho_f>.
 //   B  k_strain       : resolved strain, G-dependent Smagorinsky nu_t (calculate_nu_t
 //                       :1569), SSR-SGS flame speed (:1913) and mu_eff = mu + rho_f nu_t.
-//   C1 k_rhs_flow     : momentum and G right-hand sides (calculate_RHS :2552-2825).
-//   C2 k_rhs_scalar   : species and temperature right-hand sides (:2837-2962) fused with
-//                       the RK4 stage update (:4432-4455) or the final combine (:4517-4544).
+//   C1 k_rhs_scalar   : species and temperature right-hand sides (:2837-2962) fused with
+//                       the RK4 stage update (:4432-4455) or the final combine (:4517-4544)
+//                       of T, Y_k and rho; the new density is handed to C2.
+//   C2 k_rhs_flow     : momentum and G right-hand sides (calculate_RHS :2552-2825) fused with
+//                       the same update of u, v, w and G.
 // After the fourth stage the boundary kernels replay apply_boundary_conditions
 // (:2967-3161) in the reference's face order.
 //
@@ -54,10 +56,6 @@ template <typename R>
 struct KDbg {                // optional (nullptr): the stage's k-arrays for inspection
     R* p[NACC];
 };
-template <typename R>
-struct KFlow {               // momentum and G right-hand sides handed from C1 to C2
-    R* p[4];                 // k_rhou k_rhov k_rhow k_G
-};
 
 #define LES_KERNEL_CONSTS const __grid_constant__ Consts C
 
@@ -85,12 +83,11 @@ __device__ __forceinline__ void shift_props(PropBuf<R>& P, long long d) {
     P.grad_g = nullptr;
 }
 
-// Minimum resident blocks per SM requested from the register allocator (filter / flow /
-// scalar).  These kernels are latency-bound; swept on B200 at 256x128x128: FP64 5/4/4 (the
-// scalar pass at 3 blocks 3.41 ms, at 4 3.17 ms; the filter at 4 3.14 ms, at 5 3.02 ms; the
-// flow pass at 5 slower), FP32 8/8/6/6 for filter/strain/flow/scalar (the scalar pass at 4
-// blocks 2.01 ms, at 5 1.84 ms, at 6 1.76 ms; the flow pass at 8 0.616 ms, at 7 0.616, at 6
-// 0.597).
+// Minimum resident blocks per SM requested from the register allocator (filter / strain / flow /
+// scalar).  Swept on B200 at 256x128x128, ms per step (four launches): FP64 flow 0.95 at 5 blocks,
+// 0.91 at 4, 1.01 at 3, 1.29 at 2; scalar 1.40 at 5, 1.38 at 4, 1.51 at 3 and 2; FP32 flow
+// 0.617 at 7, 0.610 at 6 and 5 (at 96x48x48 0.0775, 0.0729, 0.0705), 0.658 at 4; scalar 1.06 at 7,
+// 1.04 at 6, 0.91 at 5, 0.88 at 4.
 #ifndef LES_MINB_FILTER
 #define LES_MINB_FILTER 5
 #endif
@@ -110,10 +107,10 @@ __device__ __forceinline__ void shift_props(PropBuf<R>& P, long long d) {
 #define LES_MINB_STRAIN_F32 8
 #endif
 #ifndef LES_MINB_FLOW_F32
-#define LES_MINB_FLOW_F32 6
+#define LES_MINB_FLOW_F32 5
 #endif
 #ifndef LES_MINB_SCALAR_F32
-#define LES_MINB_SCALAR_F32 6
+#define LES_MINB_SCALAR_F32 4
 #endif
 template <typename R>
 struct MinBlocks {
@@ -174,22 +171,15 @@ __device__ __forceinline__ R eos_rho(const Consts& C, R T, const R Y[NSP], R fal
     }
     return fallback;
 }
-// The same on the FP64 state, with the state division of the precision form Form; irho is an
-// approximation of 1 / rho (a product, no second division) for the quotients by rho.  The gas
+// The same on the FP64 state, with the state division of the precision form Form.  The gas
 // constant of the mixture is multiplied out (rho = p / ((R sum Y_k / M_k) T): one division
 // instead of three).
 template <typename Form>
-__device__ __forceinline__ double eos_rho_state(const Consts& C, double T, const double Y[NSP], double fallback,
-                                                double& irho) {
+__device__ __forceinline__ double eos_rho_state(const Consts& C, double T, const double Y[NSP], double fallback) {
     double syw = Y[0] * C.d_mwk[0].r;
 #pragma unroll
     for (int s = 1; s < NSP; s++) syw = fma(Y[s], C.d_mwk[s].r, syw);
-    if (syw > 1e-9 && T > 1.0) {
-        const double z = (R_UNIV * syw) * T;
-        irho = z * (1.0 / P_CONST);
-        return sdiv<Form>(P_CONST, z);
-    }
-    irho = sdiv<Form>(1.0, fallback);
+    if (syw > 1e-9 && T > 1.0) return sdiv<Form>(P_CONST, (R_UNIV * syw) * T);
     return fallback;
 }
 
@@ -706,84 +696,63 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::strain, NTB))
 
 // ------------------------------------------------------------------ pass C: right-hand sides
 
-// teno5_reconstruct (:2190-2236)
+// TENO5 (:2190-2295) and the WENO5 gradient (:735-827) of one axis, in the differences between
+// neighbouring cells.  With f, g the two differences of three consecutive values (a, b, c), the
+// reference's smoothness differences are a - 2b + c = g - f and a - 4b + 3c = 3g - f (seen from
+// the right end), a - c = -(f + g) (from the middle), 3a - 4b + c = g - 3f (from the left end).
 template <typename R>
-__device__ __forceinline__ R teno5_rec(const Consts& C, R v0, R v1, R v2, R v3, R v4) {
-    const auto& K = kc<R>(C);
-    R a0 = v0 - R(2.0) * v1 + v2, b0 = v0 - R(4.0) * v1 + R(3.0) * v2;
-    R a1 = v1 - R(2.0) * v2 + v3, b1 = v1 - v3;
-    R a2 = v2 - R(2.0) * v3 + v4, b2 = R(3.0) * v2 - R(4.0) * v3 + v4;
-    R is0 = R(13.0 / 12.0) * (a0 * a0) + R(1.0 / 4.0) * (b0 * b0);
-    R is1 = R(13.0 / 12.0) * (a1 * a1) + R(1.0 / 4.0) * (b1 * b1);
-    R is2 = R(13.0 / 12.0) * (a2 * a2) + R(1.0 / 4.0) * (b2 * b2);
-    int d0 = (is0 < R(TENO_CUT)) ? 1 : 0, d1 = (is1 < R(TENO_CUT)) ? 1 : 0, d2 = (is2 < R(TENO_CUT)) ? 1 : 0;
-    R p0 = cdv(R(2.0) * v0 - R(7.0) * v1 + R(11.0) * v2, K.d_six);
-    R p1 = cdv(-v1 + R(5.0) * v2 + R(2.0) * v3, K.d_six);
-    R p2 = cdv(R(2.0) * v2 + R(5.0) * v3 - v4, K.d_six);
-    if (d0 + d1 + d2 == 0) {
-        if (is0 <= is1 && is0 <= is2) return p0;
-        else if (is1 <= is0 && is1 <= is2) return p1;
-        else return p2;
-    }
-    R w0 = (R)d0 * R(0.1), w1 = (R)d1 * R(0.6), w2 = (R)d2 * R(0.3);
-    R ws = w0 + w1 + w2;
-    if (ws < R(1e-40)) return p1;
-    // ws takes one of seven values: divide by the tabulated divisor (same bits as x / ws)
-    return cdv(w0 * p0 + w1 * p1 + w2 * p2, K.d_tenows[d0 + 2 * d1 + 4 * d2]);
+__device__ __forceinline__ R smooth(R s2, R b) { return fma(R(1.0 / 4.0) * b, b, s2); }   // s2 = 13/12 (g - f)^2
+
+// 6 x (reconstructed value - its cell) from the three candidates q0, q1, q2 (:2212-2236): the
+// smooth ones by their linear weights, or the smoothest where none is smooth.
+template <typename R>
+__device__ __forceinline__ R teno_pick(R is0, R is1, R is2, R q0, R q1, R q2) {
+    const R w0 = is0 < R(TENO_CUT) ? R(0.1) : R(0.0), w1 = is1 < R(TENO_CUT) ? R(0.6) : R(0.0),
+            w2 = is2 < R(TENO_CUT) ? R(0.3) : R(0.0);
+    const R ws = w0 + w1 + w2;
+    const R best = (is0 <= is1 && is0 <= is2) ? q0 : ((is1 <= is0 && is1 <= is2) ? q1 : q2);
+    const R sum = fma(w2, q2, fma(w1, q1, w0 * q0));
+    return ws > R(0.0) ? sum * frcp(ws > R(0.0) ? ws : R(1.0)) : best;
 }
 
-// One axis of the TENO5 G-advection (:2258-2295).
+// Difference of the two reconstructed face values along the velocity, f1..f5 the differences of
+// the six values from three upstream to two downstream: mirrored for a negative velocity the
+// reference's two branches are this one expression, and the two faces share three stencils.
 template <typename R>
-__device__ __forceinline__ R teno_axis(const Consts& C, R vel, const R* __restrict__ q, ptrdiff_t s, const DCT<R>& d) {
-    R q0 = q[-3 * s], q1 = q[-2 * s], q2 = q[-s], q3 = q[0], q4 = q[s], q5 = q[2 * s], q6 = q[3 * s];
-    if (vel >= R(0.0)) {
-        R ph = teno5_rec<R>(C, q1, q2, q3, q4, q5);
-        R mh = teno5_rec<R>(C, q0, q1, q2, q3, q4);
-        return cdv(vel * (ph - mh), d);
-    } else {
-        R mh = teno5_rec<R>(C, q5, q4, q3, q2, q1);
-        R ph = teno5_rec<R>(C, q6, q5, q4, q3, q2);
-        return cdv(vel * (ph - mh), d);
-    }
+__device__ __forceinline__ R teno_faces(R f1, R f2, R f3, R f4, R f5) {
+    const R s1 = f2 - f1, s2 = f3 - f2, s3 = f4 - f3, s4 = f5 - f4;
+    const R c = R(13.0 / 12.0);
+    const R t1 = c * s1 * s1, t2 = c * s2 * s2, t3 = c * s3 * s3, t4 = c * s4 * s4;
+    const R m = teno_pick<R>(smooth(t1, fma(R(3.0), f2, -f1)), smooth(t2, f2 + f3), smooth(t3, fma(R(-3.0), f3, f4)),
+                             fma(R(5.0), f2, R(-2.0) * f1), fma(R(2.0), f3, f2), fma(R(4.0), f3, -f4));
+    const R p = teno_pick<R>(smooth(t2, fma(R(3.0), f3, -f2)), smooth(t3, f3 + f4), smooth(t4, fma(R(-3.0), f4, f5)),
+                             fma(R(5.0), f3, R(-2.0) * f2), fma(R(2.0), f4, f3), fma(R(4.0), f4, -f5));
+    return fma(p - m, R(1.0 / 6.0), f3);
 }
 
-// calculate_weno5_smoothness + calculate_weno5_gradient_1d (:735-827)
+// The WENO5 gradient (:735-827, on the cells -2..+3 whatever the velocity) times the spacing, e1..e5 the
+// differences of its six values.  The weights gamma_k / (eps + IS_k)^2 are brought to one
+// denominator: one reciprocal per half instead of three quotients and three shares of their sum.
 template <typename R>
-__device__ __forceinline__ void weno_is(R v1, R v2, R v3, R v4, R v5, R& is0, R& is1, R& is2) {
-    R a0 = v1 - R(2.0) * v2 + v3, b0 = v1 - R(4.0) * v2 + R(3.0) * v3;
-    R a1 = v2 - R(2.0) * v3 + v4, b1 = v2 - v4;
-    R a2 = v3 - R(2.0) * v4 + v5, b2 = R(3.0) * v3 - R(4.0) * v4 + v5;
-    is0 = R(13.0 / 12.0) * (a0 * a0) + R(1.0 / 4.0) * (b0 * b0);
-    is1 = R(13.0 / 12.0) * (a1 * a1) + R(1.0 / 4.0) * (b1 * b1);
-    is2 = R(13.0 / 12.0) * (a2 * a2) + R(1.0 / 4.0) * (b2 * b2);
-}
-template <typename R>
-__device__ __forceinline__ R weno5_grad(const Consts& C, const R* __restrict__ q, ptrdiff_t s, const DCT<R>& dx) {
-    const auto& K = kc<R>(C);
-    R p0 = q[-2 * s], p1 = q[-s], p2 = q[0], p3 = q[s], p4 = q[2 * s], p5 = q[3 * s];
+__device__ __forceinline__ R weno_half(R i0, R i1, R i2, R g0, R g1, R g2, R q0, R q1, R q2) {
     const R eps = R(1.0e-6);
-    R i0, i1, i2;
-    weno_is<R>(p1, p2, p3, p4, p5, i0, i1, i2);
-    R e0 = eps + i0, e1 = eps + i1, e2 = eps + i2;
-    R a0 = qdiv(R(3.0 / 10.0), e0 * e0), a1 = qdiv(R(6.0 / 10.0), e1 * e1), a2 = qdiv(R(1.0 / 10.0), e2 * e2);
-    R sa = a0 + a1 + a2;
-    R ysa = qdiv(R(1.0), sa);
-    R w0 = mdiv(a0, sa, ysa), w1 = mdiv(a1, sa, ysa), w2 = mdiv(a2, sa, ysa);
-    R s0 = cdv(R(2.0) * p1 - R(7.0) * p2 + R(11.0) * p3, K.d_six);
-    R s1 = cdv(-p2 + R(5.0) * p3 + R(2.0) * p4, K.d_six);
-    R s2 = cdv(R(2.0) * p3 + R(5.0) * p4 - p5, K.d_six);
-    R ph = w0 * s0 + w1 * s1 + w2 * s2;
-    weno_is<R>(p0, p1, p2, p3, p4, i0, i1, i2);
-    e0 = eps + i0; e1 = eps + i1; e2 = eps + i2;
-    a0 = qdiv(R(1.0 / 10.0), e0 * e0); a1 = qdiv(R(6.0 / 10.0), e1 * e1); a2 = qdiv(R(3.0 / 10.0), e2 * e2);
-    sa = a0 + a1 + a2;
-    ysa = qdiv(R(1.0), sa);
-    w0 = mdiv(a0, sa, ysa); w1 = mdiv(a1, sa, ysa); w2 = mdiv(a2, sa, ysa);
-    R m0 = cdv(-p0 + R(5.0) * p1 + R(2.0) * p2, K.d_six);
-    R m1 = cdv(R(2.0) * p1 + R(5.0) * p2 - p3, K.d_six);
-    R m2 = cdv(R(11.0) * p2 - R(7.0) * p3 + R(2.0) * p4, K.d_six);
-    R mh = w0 * m0 + w1 * m1 + w2 * m2;
-    return cdv(ph - mh, dx);
+    const R a0 = eps + i0, a1 = eps + i1, a2 = eps + i2;
+    const R e0 = a0 * a0, e1 = a1 * a1, e2 = a2 * a2;
+    const R w0 = g0 * (e1 * e2), w1 = g1 * (e0 * e2), w2 = g2 * (e0 * e1);
+    return fma(w2, q2, fma(w1, q1, w0 * q0)) * frcp(w0 + w1 + w2);
+}
+template <typename R>
+__device__ __forceinline__ R weno_diff(R e1, R e2, R e3, R e4, R e5) {
+    const R s1 = e2 - e1, s2 = e3 - e2, s3 = e4 - e3, s4 = e5 - e4;
+    const R c = R(13.0 / 12.0);
+    const R t1 = c * s1 * s1, t2 = c * s2 * s2, t3 = c * s3 * s3, t4 = c * s4 * s4;
+    const R p = weno_half<R>(smooth(t2, fma(R(3.0), e3, -e2)), smooth(t3, e3 + e4), smooth(t4, fma(R(-3.0), e4, e5)),
+                             R(0.3), R(0.6), R(0.1), fma(R(5.0), e3, R(-2.0) * e2), fma(R(2.0), e4, e3),
+                             fma(R(4.0), e4, -e5));
+    const R m = weno_half<R>(smooth(t1, fma(R(3.0), e2, -e1)), smooth(t2, e2 + e3), smooth(t3, fma(R(-3.0), e3, e4)),
+                             R(0.1), R(0.6), R(0.3), fma(R(2.0), e2, e1), fma(R(4.0), e2, -e3),
+                             fma(R(2.0), e4, fma(R(-5.0), e3, R(6.0) * e2)));
+    return fma(p - m, R(1.0 / 6.0), e2 + e3);
 }
 
 // MUSCL-superbee (:2017-2028, :2058-2094).  Half the limited slope of a face,
@@ -840,255 +809,7 @@ __device__ __forceinline__ R star_rhs(const Star<R>& q, const StarCoef<R>& K, R 
     return k;
 }
 
-// Stencil access to one field around the current cell, q(di, dj, dk): global memory (the
-// cell's address and the i/j strides) or the shared-memory planes of a staged tile.  The
-// helpers below take either, so both read paths run the same arithmetic.
-template <typename R>
-struct GAcc {
-    const R* __restrict__ p;
-    ptrdiff_t sI, sJ;
-    __device__ __forceinline__ R operator()(int di, int dj, int dk) const { return p[di * sI + dj * sJ + dk]; }
-};
-template <typename R>
-__device__ __forceinline__ GAcc<R> gacc(const R* p, ptrdiff_t sI, ptrdiff_t sJ) {
-    GAcc<R> a;
-    a.p = p; a.sI = sI; a.sJ = sJ;
-    return a;
-}
-// First-order upwind fallback used by the non-conservative schemes near faces
-// (:642-651, :2043-2052).
-template <typename R, typename A>
-__device__ __forceinline__ R upwind3(const Consts& C, const A& q, R u, R v, R w) {
-    const auto& K = kc<R>(C);
-    R f;
-    if (u >= R(0.0)) f = cdv(u * (q(0, 0, 0) - q(-1, 0, 0)), K.d_dx);
-    else f = cdv(u * (q(1, 0, 0) - q(0, 0, 0)), K.d_dx);
-    if (v >= R(0.0)) f += cdv(v * (q(0, 0, 0) - q(0, -1, 0)), K.d_dy);
-    else f += cdv(v * (q(0, 1, 0) - q(0, 0, 0)), K.d_dy);
-    if (w >= R(0.0)) f += cdv(w * (q(0, 0, 0) - q(0, 0, -1)), K.d_dz);
-    else f += cdv(w * (q(0, 0, 1) - q(0, 0, 0)), K.d_dz);
-    return f;
-}
-
-// Face-averaged SGS diffusion div((nu_t/Sc) grad phi) (:2751-2760, :2853-2860, :2932-2939).
-// The six face coefficients depend only on nu_t, so they are computed once per cell.
-template <typename R>
-struct SgsFaces {
-    R iph, imh, jph, jmh, kph, kmh;
-};
-template <typename R, typename A>
-__device__ __forceinline__ SgsFaces<R> sgs_faces(const A& nut, const DCT<R>& c2) {
-    R n0 = nut(0, 0, 0);
-    SgsFaces<R> g;
-    g.iph = cdv(nut(1, 0, 0) + n0, c2); g.imh = cdv(n0 + nut(-1, 0, 0), c2);
-    g.jph = cdv(nut(0, 1, 0) + n0, c2); g.jmh = cdv(n0 + nut(0, -1, 0), c2);
-    g.kph = cdv(nut(0, 0, 1) + n0, c2); g.kmh = cdv(n0 + nut(0, 0, -1), c2);
-    return g;
-}
-template <typename R, typename A>
-__device__ __forceinline__ R sgs_div(const Consts& C, const A& q, const SgsFaces<R>& g) {
-    const auto& K = kc<R>(C);
-    R p0 = q(0, 0, 0);
-    R sx = cdv(cdv(g.iph * (q(1, 0, 0) - p0), K.d_dx) - cdv(g.imh * (p0 - q(-1, 0, 0)), K.d_dx), K.d_dx);
-    R sy = cdv(cdv(g.jph * (q(0, 1, 0) - p0), K.d_dy) - cdv(g.jmh * (p0 - q(0, -1, 0)), K.d_dy), K.d_dy);
-    R sz = cdv(cdv(g.kph * (q(0, 0, 1) - p0), K.d_dz) - cdv(g.kmh * (p0 - q(0, 0, -1)), K.d_dz), K.d_dz);
-    return sx + sy + sz;
-}
-
-template <typename R, typename A>
-__device__ __forceinline__ R lap3(const Consts& C, const A& q) {
-    const auto& K = kc<R>(C);
-    R p0 = q(0, 0, 0);
-    R a = cdv(q(1, 0, 0) - R(2.0) * p0 + q(-1, 0, 0), K.d_dxx);
-    R b = cdv(q(0, 1, 0) - R(2.0) * p0 + q(0, -1, 0), K.d_dyy);
-    R c = cdv(q(0, 0, 1) - R(2.0) * p0 + q(0, 0, -1), K.d_dzz);
-    return a + b + c;
-}
-
-// C1: momentum (:2552-2697) with calculate_convection_conservative (:683-727) and the G
-// equation (:2706-2825).  Writes k_rhou, k_rhov, k_rhow, k_G of fluid cells.
-template <typename R, bool BATCH = false, int NTB = NT>
-__global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
-    k_rhs_flow(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, KFlow<R> kf,
-               KDbg<R> kd, const Scalars* __restrict__ Sc, Batch B) {
-    const auto& K = kc<R>(C);
-    int bz = blockIdx.z;
-    ModelK<R> M;
-    if constexpr (BATCH) {
-        const int m = blockIdx.z / B.gz;
-        bz = blockIdx.z - m * B.gz;
-        const MemberTab& e = B.mt[m];
-        shift_all(F, e.delta);
-        shift_props(P, e.delta);
-        shift_all(kf, e.delta);
-#pragma unroll
-        for (int q = 0; q < NACC; q++) kd.p[q] = nullptr;
-        attr = e.attr;
-        Sc = e.S;
-        M = member_model<R>(e);
-    } else {
-        M = model_of<R>(C);
-    }
-    const int nx = C.nx, ny = C.ny, nz = C.nz;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i = bz * blockDim.z + threadIdx.z;
-    if (k >= nz || j >= ny || i >= C.nx) return;
-    const ptrdiff_t sI = (ptrdiff_t)ny * nz, sJ = (ptrdiff_t)nz;
-    const size_t id = cid(i, j, k, ny, nz);
-    if (attr[id] != 3) return;
-    const R* __restrict__ uf = F.p[0] + id;
-    const R* __restrict__ vf = F.p[1] + id;
-    const R* __restrict__ wf = F.p[2] + id;
-    const R* __restrict__ Gf = F.p[4] + id;
-    const R* __restrict__ rf = F.p[5] + id;
-    const R u0 = uf[0], v0 = vf[0], w0 = wf[0];
-    const bool band2 = (i < 2 || i >= nx - 2 || j < 2 || j >= ny - 2 || k < 2 || k >= nz - 2);
-    const bool band3 = (i < 3 || i >= nx - 3 || j < 3 || j >= ny - 3 || k < 3 || k >= nz - 3);
-    R kmom[3];
-    {
-        const R r0 = rf[0];
-        // face mass fluxes; in the near-face band the reference writes 0.5*(a+b)*0.5*(c+d),
-        // in the interior (0.5*(a+b))*(0.5*(c+d)) -- equal values, since scaling by 0.5 is exact
-        R mf_iph = (R(0.5) * (rf[sI] + r0)) * (R(0.5) * (uf[sI] + u0));
-        R mf_imh = (R(0.5) * (r0 + rf[-sI])) * (R(0.5) * (u0 + uf[-sI]));
-        R mf_jph = (R(0.5) * (rf[sJ] + r0)) * (R(0.5) * (vf[sJ] + v0));
-        R mf_jmh = (R(0.5) * (r0 + rf[-sJ])) * (R(0.5) * (v0 + vf[-sJ]));
-        R mf_kph = (R(0.5) * (rf[1] + r0)) * (R(0.5) * (wf[1] + w0));
-        R mf_kmh = (R(0.5) * (r0 + rf[-1])) * (R(0.5) * (w0 + wf[-1]));
-        const R mu_eff = P.mu_eff[id];
-        const R* comps[3] = {uf, vf, wf};
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const R* __restrict__ ph = comps[q];
-            R pc = ph[0];
-            R p_iph, p_imh, p_jph, p_jmh, p_kph, p_kmh;
-            if (band2) {
-                p_iph = (mf_iph > R(0)) ? pc : ph[sI];
-                p_imh = (mf_imh > R(0)) ? ph[-sI] : pc;
-                p_jph = (mf_jph > R(0)) ? pc : ph[sJ];
-                p_jmh = (mf_jmh > R(0)) ? ph[-sJ] : pc;
-                p_kph = (mf_kph > R(0)) ? pc : ph[1];
-                p_kmh = (mf_kmh > R(0)) ? ph[-1] : pc;
-            } else {
-                // With the reference's face coefficients UW2 = 0, UW1 = DW1 = 0.5 (:164-166)
-                // both upwind branches give 0.5*phi_L + 0.5*phi_R, so no branch is taken.
-                p_iph = R(0.5) * pc + R(0.5) * ph[sI];
-                p_imh = R(0.5) * ph[-sI] + R(0.5) * pc;
-                p_jph = R(0.5) * pc + R(0.5) * ph[sJ];
-                p_jmh = R(0.5) * ph[-sJ] + R(0.5) * pc;
-                p_kph = R(0.5) * pc + R(0.5) * ph[1];
-                p_kmh = R(0.5) * ph[-1] + R(0.5) * pc;
-            }
-            R conv = cdv(mf_iph * p_iph - mf_imh * p_imh, K.d_dx) + cdv(mf_jph * p_jph - mf_jmh * p_jmh, K.d_dy) +
-                     cdv(mf_kph * p_kph - mf_kmh * p_kmh, K.d_dz);
-            kmom[q] = -conv + mu_eff * lap3<R>(C, gacc(ph, sI, sJ));
-        }
-        R grav = (r0 - (R)Sc->rho_avg) * R(G_GRAVITY);
-        R fx = R(0), fy = R(0), fz = R(0);
-        if (C.flame_accel) {
-            R Gl = Gf[0];
-            if (Gl > R(0.01) && Gl < R(0.99)) {
-                R dGx = cdv(Gf[sI] - Gf[-sI], K.d_2dx);
-                R dGy = cdv(Gf[sJ] - Gf[-sJ], K.d_2dy);
-                R dGz = cdv(Gf[1] - Gf[-1], K.d_2dz);
-                if (dGx < R(0.0)) dGx = R(0.0);
-                if (dGy < R(0.0)) dGy = R(0.0);
-                R zrel = ((R)k * (R)K.dz) - (R)K.inlet_center_z;
-                if (zrel > R(0.0)) {
-                    if (dGz < R(0.0)) dGz = R(0.0);
-                } else {
-                    if (dGz > R(0.0)) dGz = R(0.0);
-                }
-                R df = Gl - M.accel_center;
-                R window = qexp(cdv(-(df * df), M.d_w2));
-                // tip_mask is the literal 1.0 in the momentum source (:2638)
-                R cf = M.accel_strength * r0 * window * R(1.0);
-                fx = cf * dGx * R(0.05);
-                fy = cf * dGy * R(1.0);
-                fz = cf * dGz * R(1.0);
-                R zp = (R)k * (R)K.dz, ramp = R(1.0);
-                if (zp < R(RAMP_DIST)) ramp = cdv(zp, K.d_ramp);
-                fx *= ramp; fy *= ramp; fz *= ramp;
-            }
-        }
-        const R lim = R(FORCE_LIMIT);
-        if (fx > lim) fx = lim;
-        if (fx < -lim) fx = -lim;
-        if (fy > lim) fy = lim;
-        if (fy < -lim) fy = -lim;
-        if (fz > lim) fz = lim;
-        if (fz < -lim) fz = -lim;
-        kmom[0] = kmom[0] + grav + fx;
-        kmom[1] = kmom[1] + fy;
-        kmom[2] = kmom[2] + fz;
-    }
-    R kG;
-    {
-        R conv;
-        if (band3) {
-            if (band2) {
-                conv = upwind3<R>(C, gacc(Gf, sI, sJ), u0, v0, w0);
-            } else {
-                // calculate_convection_non_conservative interior branch (:652-677); the
-                // zero UW2 coefficient again makes both upwind branches identical.
-                R pc = Gf[0];
-                R p_iph = R(0.5) * pc + R(0.5) * Gf[sI], p_imh = R(0.5) * Gf[-sI] + R(0.5) * pc;
-                R p_jph = R(0.5) * pc + R(0.5) * Gf[sJ], p_jmh = R(0.5) * Gf[-sJ] + R(0.5) * pc;
-                R p_kph = R(0.5) * pc + R(0.5) * Gf[1], p_kmh = R(0.5) * Gf[-1] + R(0.5) * pc;
-                R cx = cdv(u0 * (p_iph - p_imh), K.d_dx);
-                R cy = cdv(v0 * (p_jph - p_jmh), K.d_dy);
-                R cz = cdv(w0 * (p_kph - p_kmh), K.d_dz);
-                conv = cx + cy + cz;
-            }
-        } else {
-            R fxa = teno_axis<R>(C, u0, Gf, sI, K.d_dx);
-            R fya = teno_axis<R>(C, v0, Gf, sJ, K.d_dy);
-            R fza = teno_axis<R>(C, w0, Gf, 1, K.d_dz);
-            conv = fxa + fya + fza;
-        }
-        SgsFaces<R> gf = sgs_faces<R>(gacc<R>(P.nu_t + id, sI, sJ), K.d_sct2);
-        R sgs = sgs_div<R>(C, gacc(Gf, sI, sJ), gf);
-        R gx, gy, gz;
-        if (Sc->t_loop >= C.weno_step && !band3) {
-            gx = weno5_grad<R>(C, Gf, sI, K.d_dx);
-            gy = weno5_grad<R>(C, Gf, sJ, K.d_dy);
-            gz = weno5_grad<R>(C, Gf, 1, K.d_dz);
-        } else {
-            gx = cdv(Gf[sI] - Gf[-sI], K.d_2dx);
-            gy = cdv(Gf[sJ] - Gf[-sJ], K.d_2dy);
-            gz = cdv(Gf[1] - Gf[-1], K.d_2dz);
-        }
-        R gmag = qsqrt(gx * gx + gy * gy + gz * gz);
-        if (P.grad_g) P.grad_g[id] = gmag;   // grad_G_magnitude_for_debug (:2783)
-        R prop = P.ST[id] * gmag;
-        R art = R(0);
-        if (C.flame_accel) {
-            R Gl = Gf[0];
-            if (Gl > R(0.1) && Gl < R(0.99)) {
-                R df = Gl - M.accel_center;
-                R window = qexp(cdv(-(df * df), M.d_w2));
-                // tip_mask = 1 - exp(-r^2 / 0^2) is exactly 1 for every fluid cell (j >= 1)
-                // because TIP_PROTECTION_RADIUS is 0.0 (:234, :2806-2807).
-                R adc = R(5.0) * (P.nu_t[id] + R(1.0e-5)) * window * R(1.0);
-                art = adc * lap3<R>(C, gacc(Gf, sI, sJ));
-            }
-        }
-        kG = -conv + prop + sgs + art;
-    }
-    kf.p[0][id] = kmom[0];
-    kf.p[1][id] = kmom[1];
-    kf.p[2][id] = kmom[2];
-    kf.p[3][id] = kG;
-    if (kd.p[0]) {
-        kd.p[0][id] = kmom[0];
-        kd.p[1][id] = kmom[1];
-        kd.p[2][id] = kmom[2];
-        kd.p[4][id] = kG;
-    }
-}
-
-// C2: species (:2837-2904) and temperature (:2912-2962), then the RK4 bookkeeping.
+// C1: species (:2837-2904) and temperature (:2912-2962), then their RK4 bookkeeping.
 // stage: 0,1,2 -> intermediate stage with coefficient 0.5/0.5/1.0, 3 -> final combine.
 // Where the scalar pass reads its stencil fields (filtered T and Y_k, nu_t): global memory,
 // or the shared-memory tile of the staged kernel (les_tma.cuh).  Element indices are 32-bit: a
@@ -1125,37 +846,36 @@ struct GSrc {
     }
 };
 
+// The RK stages as the scalar pass sees them: the first starts the running sum, the last ends it.
+enum { RK_FIRST = 0, RK_MIDDLE = 1, RK_LAST = 2 };
+
 // One cell of the scalar pass (the body shared by both read paths).
-template <typename R, typename RS, typename Src>
+template <int PART, typename R, typename RS, typename Src>
 __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* __restrict__ attr, const F11<R>& F,
                                                 const PropBuf<R>& P, const F11<RS>& S0, const F11<R>& St,
-                                                const AccBuf<R>& acc, const KFlow<R>& kf, const KDbg<R>& kd,
+                                                const AccBuf<R>& acc, RS* __restrict__ rn, const KDbg<R>& kd,
                                                 const Scalars* __restrict__ Sc, int stage, int i, int j, int k,
                                                 Src& src, const R relax) {
     const auto& K = kc<R>(C);
     const int nx = C.nx, ny = C.ny, nz = C.nz;
     const size_t id = cid(i, j, k, ny, nz);
     const int a = attr[id];
-
     if (a != 3) {
-        // non-fluid cells: the temp state is Phi_n with the current velocity (:4444, :4454);
-        // rho_temp is only ever written on outlet/fluid cells (:1893), so it stays 0 on
-        // inlet/wall/symmetry cells.  These values are the same for all stages of a step.
-        if (stage == 0) {
-            RS Y0[NSP];
+        // non-fluid cells: the temp state is Phi_n (:4444, :4454); rho_temp is only ever written on
+        // outlet/fluid cells (:1893), so it stays 0 on inlet/wall/symmetry cells.  These values
+        // are the same for all stages of a step.
+        RS Y0[NSP];
+        const RS T0 = S0.p[3][id], r0 = S0.p[5][id];
 #pragma unroll
-            for (int q = 0; q < NSTATE; q++)
-                if (q != 5) St.p[q][id] = R(S0.p[q][id]);
+        for (int s = 0; s < NSP; s++) Y0[s] = S0.p[6 + s][id];
+        if (PART == RK_FIRST) {
+            const RS r = eos_rho_state<R>(C, T0, Y0, r0);
+            St.p[3][id] = R(T0);
 #pragma unroll
-            for (int s = 0; s < NSP; s++) Y0[s] = S0.p[6 + s][id];
-            RS unused;
-            if (a == 2) St.p[5][id] = R(eos_rho_state<R>(C, S0.p[3][id], Y0, S0.p[5][id], unused));
-        } else if (stage == 3 && a == 2) {
-            RS Y0[NSP];
-#pragma unroll
-            for (int s = 0; s < NSP; s++) Y0[s] = S0.p[6 + s][id];
-            RS unused;
-            S0.p[5][id] = eos_rho_state<R>(C, S0.p[3][id], Y0, S0.p[5][id], unused);
+            for (int s = 0; s < NSP; s++) St.p[6 + s][id] = R(Y0[s]);
+            if (a == 2) St.p[5][id] = R(r);
+        } else if (PART == RK_LAST && a == 2) {
+            rn[id] = eos_rho_state<R>(C, T0, Y0, r0);
         }
         if (kd.p[0]) {
 #pragma unroll
@@ -1165,9 +885,10 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
     }
 
     const R vel[3] = {F.p[0][id], F.p[1][id], F.p[2][id]};
-    const bool band2 = (i < 2 || i >= nx - 2 || j < 2 || j >= ny - 2 || k < 2 || k >= nz - 2);
-    R kv[NACC];
     R g = F.p[4][id];
+    // the right-hand sides and running sums of T, Y0..Y4 in this order, fields 3 and 5..9 of acc
+    R kv[1 + NSP];
+    const bool band2 = (i < 2 || i >= nx - 2 || j < 2 || j >= ny - 2 || k < 2 || k >= nz - 2);
     if (g < R(0.0)) g = R(0.0);
     if (g > R(1.0)) g = R(1.0);
     const bool pos[3] = {vel[0] >= R(0.0), vel[1] >= R(0.0), vel[2] >= R(0.0)};
@@ -1192,7 +913,7 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
         Star<R> q;
         src.t(q);
         const R Tt = fma(g, (R)K.t_burnt_span, (R)K.t_in);
-        kv[3] = star_rhs<R, false>(q, co, K.d_sct2.c * K.d_prt2.r, ld_stream(P.aT + id), ih2, relax * (Tt - q.c));
+        kv[0] = star_rhs<R, false>(q, co, K.d_sct2.c * K.d_prt2.r, ld_stream(P.aT + id), ih2, relax * (Tt - q.c));
     }
 #pragma unroll
     for (int s = 0; s < NSP; s++) {
@@ -1204,84 +925,63 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
         else tgt = (R)K.inletYk[N2];
         Star<R> q;
         src.y(s, q);
-        kv[5 + s] = star_rhs<R, true>(q, co, R(1.0), ld_stream(P.D[s] + id), ih2, relax * (tgt - q.c));
+        kv[1 + s] = star_rhs<R, true>(q, co, R(1.0), ld_stream(P.D[s] + id), ih2, relax * (tgt - q.c));
     }
-    kv[0] = ld_stream(kf.p[0] + id);
-    kv[1] = ld_stream(kf.p[1] + id);
-    kv[2] = ld_stream(kf.p[2] + id);
-    kv[4] = ld_stream(kf.p[3] + id);
-    if (kd.p[0]) {
-        kd.p[3][id] = kv[3];
-#pragma unroll
-        for (int s = 0; s < NSP; s++) kd.p[5 + s][id] = kv[5 + s];
-    }
-
     // ---- RK4 bookkeeping.  acc holds k1, k1 + 2k2, (k1 + 2k2) + 2k3: exactly the
-    // left-to-right partial sums of k1 + 2.0*k2 + 2.0*k3 + k4 (:4520).
-    const bool fin = (stage == 3);
-    const double dt = Sc->dt;
-    R incr[NACC];
-    if (stage == 0) {
+    // left-to-right partial sums of k1 + 2.0*k2 + 2.0*k3 + k4 (:4520).  All loads come before the
+    // first store: a store in between may alias them as far as the compiler knows, and each load
+    // after it would wait for that store's operand, one trip to memory after another; for the
+    // same reason the part of the step is a template parameter, not a branch.
+    RS sn[2 + NSP];                     // T, Y0..Y4, rho
+    R ac[1 + NSP];
 #pragma unroll
-        for (int q = 0; q < NACC; q++) { incr[q] = kv[q]; st_stream(acc.p[q] + id, kv[q]); }
-    } else if (stage < 3) {
-#pragma unroll
-        for (int q = 0; q < NACC; q++) { incr[q] = kv[q]; st_stream(acc.p[q] + id, ld_stream(acc.p[q] + id) + R(2.0) * kv[q]); }
-    } else {
-#pragma unroll
-        for (int q = 0; q < NACC; q++) incr[q] = ld_stream(acc.p[q] + id) + kv[q];
+    for (int q = 0; q < 1 + NSP; q++) {
+        sn[q] = ld_stream(S0.p[q == 0 ? 3 : 5 + q] + id);
+        ac[q] = PART != RK_FIRST ? ld_stream(acc.p[q == 0 ? 3 : 4 + q] + id) : R(0);
     }
+    const RS rho_n = ld_stream(S0.p[5] + id);
+    const double dt = Sc->dt;
     // The update itself runs in the state's type: in the FP32 form the right-hand sides are
     // FP32 and Phi_n, the stage update and the final combine FP64, so increments far below
     // the state's FP32 ulp are not rounded away step after step.
-    const RS cdt = fin ? (RS)(dt / 6.0) : (RS)((stage == 2 ? 1.0 : 0.5) * dt);
-    const RS rho_n = ld_stream(S0.p[5] + id);
-    RS Tn = fma(cdt, (RS)incr[3], ld_stream(S0.p[3] + id));
-    RS Gn = fma(cdt, (RS)incr[4], ld_stream(S0.p[4] + id));
-    RS Y[NSP];
+    const RS cdt = PART == RK_LAST ? (RS)(dt / 6.0) : (RS)((PART == RK_MIDDLE && stage == 2 ? 1.0 : 0.5) * dt);
+    RS up[1 + NSP], sy = RS(0);
 #pragma unroll
-    for (int s = 0; s < NSP; s++) Y[s] = fma(cdt, (RS)incr[5 + s], ld_stream(S0.p[6 + s] + id));
-    Tn = fmax(RS(200.0), fmin(RS(3000.0), Tn));
-    Gn = fmax(RS(0.0), fmin(RS(1.0), Gn));
-    RS sy = RS(0);
-#pragma unroll
-    for (int s = 0; s < NSP; s++) {
-        Y[s] = fmax(RS(0.0), fmin(RS(1.0), Y[s]));
-        sy += Y[s];
+    for (int q = 0; q < 1 + NSP; q++) {
+        const R incr = PART == RK_LAST ? ac[q] + kv[q] : kv[q];
+        ac[q] = PART == RK_FIRST ? kv[q] : fma(R(2.0), kv[q], ac[q]);
+        up[q] = fma(cdt, (RS)incr, sn[q]);
+        up[q] = q == 0 ? fmax(RS(200.0), fmin(RS(3000.0), up[q])) : fmax(RS(0.0), fmin(RS(1.0), up[q]));
+        if (q > 0) sy += up[q];
     }
-    // One reciprocal per divisor; the quotients sharing it are corrected with one fma each.
+    // one reciprocal, the quotients sharing it corrected with one fma each
     if (sy > RS(SMALL)) {
         const RS y = sdiv<R>(RS(1.0), sy);
 #pragma unroll
-        for (int s = 0; s < NSP; s++) Y[s] = cquot(Y[s], sy, y);
+        for (int s = 1; s < 1 + NSP; s++) up[s] = cquot(up[s], sy, y);
     }
-    RS irn;
-    const RS rn = eos_rho_state<R>(C, Tn, Y, rho_n, irn);
-    RS vn[3];
+    const RS rho = eos_rho_state<R>(C, up[0], up + 1, rho_n);
+    if (kd.p[0]) {
 #pragma unroll
-    for (int q = 0; q < 3; q++) {
-        RS m = fma(cdt, (RS)incr[q], rho_n * ld_stream(S0.p[q] + id));   // rhou = rho*u after the BC (:3146)
-        vn[q] = (rn > RS(SMALL)) ? cquot(m, rn, irn) : RS(0);
+        for (int q = 0; q < 1 + NSP; q++) kd.p[q == 0 ? 3 : 4 + q][id] = kv[q];
     }
-    if (fin) {
-        RS* const* out = S0.p;
-        out[0][id] = vn[0]; out[1][id] = vn[1]; out[2][id] = vn[2];
-        out[3][id] = Tn; out[4][id] = Gn; out[5][id] = rn;
+    st_stream(rn + id, rho);
+    if (PART != RK_LAST) St.p[5][id] = R(rho);
 #pragma unroll
-        for (int s = 0; s < NSP; s++) out[6 + s][id] = Y[s];
-    } else {
-        R* const* out = St.p;
-        out[0][id] = R(vn[0]); out[1][id] = R(vn[1]); out[2][id] = R(vn[2]);
-        out[3][id] = R(Tn); out[4][id] = R(Gn); out[5][id] = R(rn);
-#pragma unroll
-        for (int s = 0; s < NSP; s++) out[6 + s][id] = R(Y[s]);
+    for (int q = 0; q < 1 + NSP; q++) {
+        if (PART != RK_LAST) {
+            st_stream(acc.p[q == 0 ? 3 : 4 + q] + id, ac[q]);
+            St.p[q == 0 ? 3 : 5 + q][id] = R(up[q]);
+        } else {
+            S0.p[q == 0 ? 3 : 5 + q][id] = up[q];
+        }
     }
 }
 
-template <typename R, typename RS = R, bool BATCH = false, int NTB = NT>
+template <int PART, typename R, typename RS = R, bool BATCH = false, int NTB = NT>
 __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
     k_rhs_scalar(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, F11<RS> S0, F11<R> St,
-                 AccBuf<R> acc, KFlow<R> kf, KDbg<R> kd, const Scalars* __restrict__ Sc, int stage, Batch B) {
+                 AccBuf<R> acc, RS* __restrict__ rn, KDbg<R> kd, const Scalars* __restrict__ Sc, int stage, Batch B) {
     int bz = blockIdx.z;
     R relax;
     if constexpr (BATCH) {
@@ -1293,7 +993,7 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
         shift_all(S0, e.delta);
         shift_all(St, e.delta);
         shift_all(acc, e.delta);
-        shift_all(kf, e.delta);
+        rn = shifted(rn, e.delta);
 #pragma unroll
         for (int q = 0; q < NACC; q++) kd.p[q] = nullptr;
         attr = e.attr;
@@ -1317,7 +1017,199 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
 #pragma unroll
     for (int s = 0; s < NSP; s++) src.Y[s] = F.p[6 + s];
     src.nut = P.nu_t;
-    rhs_scalar_cell<R, RS>(C, attr, F, P, S0, St, acc, kf, kd, Sc, stage, i, j, k, src, relax);
+    rhs_scalar_cell<PART, R, RS>(C, attr, F, P, S0, St, acc, rn, kd, Sc, stage, i, j, k, src, relax);
+}
+
+// C2: momentum (:2552-2697) with calculate_convection_conservative (:683-727) and the G
+// equation (:2706-2825), then the RK4 bookkeeping of u, v, w and G with the density the scalar
+// pass left in rn.  Measured at 256x128x128, both passes together: handing the density over
+// (8 bytes a cell) instead of four right-hand sides, with this pass updating what it computes,
+// moves 48 bytes a cell less and takes the loads of half the update out of the scalar pass,
+// which waits for memory, into this one, which computes.
+// Everything is in differences across the six faces: a conservative flux m p with the face
+// value p = p0 + d/2 (first-order upwind next to the boundary: p0 or p0 + d by the sign of m),
+// so convection and diffusion of all three components are two coefficients a face.
+template <int PART, typename R, typename RS = R, bool BATCH = false, int NTB = NT>
+__global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
+    k_rhs_flow(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, F11<RS> S0, F11<R> St,
+               AccBuf<R> acc, RS* __restrict__ rn, KDbg<R> kd, const Scalars* __restrict__ Sc, int stage, Batch B) {
+    const auto& K = kc<R>(C);
+    int bz = blockIdx.z;
+    ModelK<R> M;
+    if constexpr (BATCH) {
+        const int m = blockIdx.z / B.gz;
+        bz = blockIdx.z - m * B.gz;
+        const MemberTab& e = B.mt[m];
+        shift_all(F, e.delta);
+        shift_props(P, e.delta);
+        shift_all(S0, e.delta);
+        shift_all(St, e.delta);
+        shift_all(acc, e.delta);
+        rn = shifted(rn, e.delta);
+#pragma unroll
+        for (int q = 0; q < NACC; q++) kd.p[q] = nullptr;
+        attr = e.attr;
+        Sc = e.S;
+        M = member_model<R>(e);
+    } else {
+        M = model_of<R>(C);
+    }
+    const int nx = C.nx, ny = C.ny, nz = C.nz;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = bz * blockDim.z + threadIdx.z;
+    if (k >= nz || j >= ny || i >= C.nx) return;
+    const int id = (int)cid(i, j, k, ny, nz);
+    const int a = attr[id];
+    if (a != 3) {
+        // as in the scalar pass: the stage state of other cells is Phi_n, and only outlet cells
+        // get a new density
+        if (PART == RK_FIRST) {
+#pragma unroll
+            for (int q = 0; q < 5; q++)
+                if (q != 3) St.p[q][id] = R(S0.p[q][id]);
+        } else if (PART == RK_LAST && a == 2) {
+            S0.p[5][id] = rn[id];
+        }
+        return;
+    }
+    const int st[3] = {ny * nz, nz, 1};
+    const R ih[3] = {K.d_dx.r, K.d_dy.r, K.d_dz.r}, ih2[3] = {K.d_dxx.r, K.d_dyy.r, K.d_dzz.r};
+    const bool band2 = (i < 2 || i >= nx - 2 || j < 2 || j >= ny - 2 || k < 2 || k >= nz - 2);
+    const bool band3 = (i < 3 || i >= nx - 3 || j < 3 || j >= ny - 3 || k < 3 || k >= nz - 3);
+    const R p0[3] = {F.p[0][id], F.p[1][id], F.p[2][id]};
+    const R r0 = F.p[5][id], G0 = F.p[4][id], n0 = P.nu_t[id], mu = P.mu_eff[id];
+    R km[3];
+    {
+        R out = R(0);
+#pragma unroll
+        for (int q = 0; q < 3; q++) km[q] = R(0);
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            const R* __restrict__ rho = F.p[5];
+            const R* __restrict__ va = F.p[x];
+            const R mp = (R(0.5) * (rho[id + st[x]] + r0)) * (R(0.5) * (va[id + st[x]] + p0[x]));
+            const R mm = (R(0.5) * (rho[id - st[x]] + r0)) * (R(0.5) * (va[id - st[x]] + p0[x]));
+            const R up = band2 ? (mp > R(0) ? R(0) : mp) : R(0.5) * mp;
+            const R um = band2 ? (mm > R(0) ? mm : R(0)) : R(0.5) * mm;
+            const R v = mu * ih2[x];
+            const R cp = fma(-ih[x], up, v), cm = fma(ih[x], um, v);
+            out = fma(ih[x], mp - mm, out);
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const R* __restrict__ ph = F.p[q];
+                km[q] = fma(cp, ph[id + st[x]] - p0[q], km[q]);
+                km[q] = fma(-cm, p0[q] - ph[id - st[x]], km[q]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++) km[q] = fma(-out, p0[q], km[q]);
+    }
+    R kG, grad[3], lap = R(0);
+    {
+        const R* __restrict__ G = F.p[4];
+        R adv = R(0), sgs = R(0);
+        R e3[3];
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            const bool pos = p0[x] >= R(0.0);
+            const int o = pos ? -st[x] : st[x];
+            const R U = G[id + o], Dn = G[id - o];
+            const R f3 = G0 - U, f4 = Dn - G0;
+            R d = f3;                                   // first-order upwind (:642-651)
+            if (!band3) {
+                const R UU = G[id + 2 * o], U3 = G[id + 3 * o], DD = G[id - 2 * o];
+                d = teno_faces<R>(UU - U3, U - UU, f3, f4, DD - Dn);
+            } else if (!band2) {
+                // central faces (:652-677): the zero UW2 coefficient makes both upwind branches identical
+                d = R(0.5) * (f3 + f4);
+            }
+            adv = fma(fabs(p0[x]) * ih[x], d, adv);
+            const R gu = (P.nu_t[id + o] + n0) * K.d_sct2.r, gd = (P.nu_t[id - o] + n0) * K.d_sct2.r;
+            sgs = fma(ih2[x], fma(gd, f4, -gu * f3), sgs);
+            lap = fma(ih2[x], f4 - f3, lap);
+            e3[x] = pos ? f3 + f4 : -(f3 + f4);
+            grad[x] = R(0.5) * ih[x] * e3[x];
+        }
+        kG = sgs - adv;
+    }
+    R art = R(0), fo[3] = {R(0), R(0), R(0)};
+    if (C.flame_accel && G0 > R(0.01) && G0 < R(0.99)) {
+        const R df = G0 - M.accel_center;
+        const R window = qexp(-(df * df) * M.d_w2.r);
+        const R zp = (R)k * (R)K.dz;
+        const R ramp = zp < R(RAMP_DIST) ? zp * K.d_ramp.r : R(1.0);
+        // tip_mask is the literal 1.0 in the momentum source (:2638)
+        const R cf = M.accel_strength * r0 * window * ramp;
+        fo[0] = cf * R(0.05) * fmax(grad[0], R(0.0));
+        fo[1] = cf * fmax(grad[1], R(0.0));
+        fo[2] = cf * (zp - (R)K.inlet_center_z > R(0.0) ? fmax(grad[2], R(0.0)) : fmin(grad[2], R(0.0)));
+        // tip_mask = 1 - exp(-r^2 / 0^2) is exactly 1 for every fluid cell (j >= 1)
+        // because TIP_PROTECTION_RADIUS is 0.0 (:234, :2806-2807).
+        if (G0 > R(0.1)) art = R(5.0) * (n0 + R(1.0e-5)) * window * lap;
+    }
+    const R lim = R(FORCE_LIMIT);
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        R f = fo[q];
+        if (f > lim) f = lim;
+        if (f < -lim) f = -lim;
+        km[q] += f;
+    }
+    km[0] = fma(r0 - (R)Sc->rho_avg, R(G_GRAVITY), km[0]);
+    if (Sc->t_loop >= C.weno_step && !band3) {
+        const R* __restrict__ G = F.p[4];
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            const R q0 = G[id - 2 * st[x]], q1 = G[id - st[x]], q3 = G[id + st[x]], q4 = G[id + 2 * st[x]],
+                    q5 = G[id + 3 * st[x]];
+            grad[x] = ih[x] * weno_diff<R>(q1 - q0, G0 - q1, q3 - G0, q4 - q3, q5 - q4);
+        }
+    }
+    const R gmag = qsqrt(fma(grad[2], grad[2], fma(grad[1], grad[1], grad[0] * grad[0])));
+    if (P.grad_g) P.grad_g[id] = gmag;   // grad_G_magnitude_for_debug (:2783)
+    kG = fma(P.ST[id], gmag, kG) + art;
+
+    // ---- RK4 bookkeeping (see rhs_scalar_cell); every load ahead of the first store
+    const R kv[4] = {km[0], km[1], km[2], kG};
+    constexpr int qa[4] = {0, 1, 2, 4};
+    RS sn[4];
+    R ac[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        sn[q] = ld_stream(S0.p[qa[q]] + id);
+        ac[q] = PART != RK_FIRST ? ld_stream(acc.p[qa[q]] + id) : R(0);
+    }
+    const RS rho_n = ld_stream(S0.p[5] + id), rho = ld_stream(rn + id);
+    const double dt = Sc->dt;
+    const RS cdt = PART == RK_LAST ? (RS)(dt / 6.0) : (RS)((PART == RK_MIDDLE && stage == 2 ? 1.0 : 0.5) * dt);
+    const RS irho = sdiv<R>(RS(1.0), rho);
+    RS out[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const R incr = PART == RK_LAST ? ac[q] + kv[q] : kv[q];
+        ac[q] = PART == RK_FIRST ? kv[q] : fma(R(2.0), kv[q], ac[q]);
+        if (q < 3) {
+            const RS m = fma(cdt, (RS)incr, rho_n * sn[q]);             // rhou = rho*u after the BC (:3146)
+            out[q] = rho > RS(SMALL) ? cquot(m, rho, irho) : RS(0);
+        } else {
+            out[q] = fmax(RS(0.0), fmin(RS(1.0), fma(cdt, (RS)incr, sn[q])));
+        }
+    }
+    if (kd.p[0]) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) kd.p[qa[q]][id] = kv[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        if (PART != RK_LAST) {
+            st_stream(acc.p[qa[q]] + id, ac[q]);
+            St.p[qa[q]][id] = R(out[q]);
+        } else {
+            S0.p[qa[q]][id] = out[q];
+        }
+    }
+    if (PART == RK_LAST) S0.p[5][id] = rho;
 }
 
 // ------------------------------------------------------------------ boundary conditions
@@ -1439,26 +1331,20 @@ __global__ void __launch_bounds__(NT) k_bc_eos(LES_KERNEL_CONSTS, const uint8_t*
         R Y[NSP];
 #pragma unroll
         for (int s = 0; s < NSP; s++) Y[s] = S.p[6 + s][id];
-        R T = S.p[3][id];
-        R syw = R(0);
-#pragma unroll
-        for (int s = 0; s < NSP; s++) syw += cdv(Y[s], K.d_mwk[s]);
-        R rho = (syw > R(1e-9) && T > R(1.0)) ? sdiv<Form>(P_CONST, sdiv<Form>(R_UNIV, sdiv<Form>(1.0, syw)) * T)
-                                              : R(1.2);
-        S.p[5][id] = rho;
+        const R T = S.p[3][id];
+        const R u = S.p[0][id], v = S.p[1][id], w = S.p[2][id];
+        S.p[5][id] = eos_rho_state<Form>(C, T, Y, R(1.2));
         if (a == 3 || a == 2 || a == 5) {
             R sy = R(0);
 #pragma unroll
             for (int s = 0; s < NSP; s++) sy += Y[s];
             if (sy > R(1e-6)) {
+                const R y = sdiv<Form>(R(1.0), sy);
 #pragma unroll
-                for (int s = 0; s < NSP; s++) S.p[6 + s][id] = sdiv<Form>(Y[s], sy);
+                for (int s = 0; s < NSP; s++) S.p[6 + s][id] = cquot(Y[s], sy, y);
             }
         }
-        if (a == 1 || a == 3) {
-            R u = S.p[0][id], v = S.p[1][id], w = S.p[2][id];
-            vmax = (double)sqrt(u * u + v * v + w * w);
-        }
+        if (a == 1 || a == 3) vmax = (double)sqrt(u * u + v * v + w * w);
     }
     const unsigned nblk = gridDim.x * gridDim.y * gridDim.z;
     const unsigned bid = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;

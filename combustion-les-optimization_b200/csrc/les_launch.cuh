@@ -53,22 +53,44 @@ static inline void launch_strain(dim3 g, dim3 b, cudaStream_t st, const Consts& 
     if (b.x * b.y * b.z == 512) k_strain<R, BATCH, 512><<<g, b, 0, st>>>(hC, attr, F, P, B);
     else k_strain<R, BATCH><<<g, b, 0, st>>>(hC, attr, F, P, B);
 }
-template <typename R, bool BATCH>
-static inline void launch_flow(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
-                               const F11<R>& F, const PropBuf<R>& P, const KFlow<R>& kf, const KDbg<R>& kd,
-                               Scalars* dS, const Batch& B) {
-    if (b.x * b.y * b.z == 512) k_rhs_flow<R, BATCH, 512><<<g, b, 0, st>>>(hC, attr, F, P, kf, kd, dS, B);
-    else k_rhs_flow<R, BATCH><<<g, b, 0, st>>>(hC, attr, F, P, kf, kd, dS, B);
+template <int PART, typename R, bool BATCH>
+static inline void launch_scalar_part(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
+                                      const F11<R>& F, const PropBuf<R>& P, const F11<RS>& S, const F11<R>& St,
+                                      const AccBuf<R>& acc, RS* rn, const KDbg<R>& kd, Scalars* dS,
+                                      int stage, const Batch& B) {
+    if (b.x * b.y * b.z == 512)
+        k_rhs_scalar<PART, R, RS, BATCH, 512><<<g, b, 0, st>>>(hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    else
+        k_rhs_scalar<PART, R, RS, BATCH><<<g, b, 0, st>>>(hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
 }
 template <typename R, bool BATCH>
 static inline void launch_scalar(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
                                  const F11<R>& F, const PropBuf<R>& P, const F11<RS>& S, const F11<R>& St,
-                                 const AccBuf<R>& acc, const KFlow<R>& kf, const KDbg<R>& kd, Scalars* dS,
+                                 const AccBuf<R>& acc, RS* rn, const KDbg<R>& kd, Scalars* dS,
                                  int stage, const Batch& B) {
+    if (stage == 0) launch_scalar_part<RK_FIRST, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    else if (stage < 3) launch_scalar_part<RK_MIDDLE, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    else launch_scalar_part<RK_LAST, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+}
+
+template <int PART, typename R, bool BATCH>
+static inline void launch_flow_part(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
+                                      const F11<R>& F, const PropBuf<R>& P, const F11<RS>& S, const F11<R>& St,
+                                      const AccBuf<R>& acc, RS* rn, const KDbg<R>& kd, Scalars* dS,
+                                      int stage, const Batch& B) {
     if (b.x * b.y * b.z == 512)
-        k_rhs_scalar<R, RS, BATCH, 512><<<g, b, 0, st>>>(hC, attr, F, P, S, St, acc, kf, kd, dS, stage, B);
+        k_rhs_flow<PART, R, RS, BATCH, 512><<<g, b, 0, st>>>(hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
     else
-        k_rhs_scalar<R, RS, BATCH><<<g, b, 0, st>>>(hC, attr, F, P, S, St, acc, kf, kd, dS, stage, B);
+        k_rhs_flow<PART, R, RS, BATCH><<<g, b, 0, st>>>(hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+}
+template <typename R, bool BATCH>
+static inline void launch_flow(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
+                                 const F11<R>& F, const PropBuf<R>& P, const F11<RS>& S, const F11<R>& St,
+                                 const AccBuf<R>& acc, RS* rn, const KDbg<R>& kd, Scalars* dS,
+                                 int stage, const Batch& B) {
+    if (stage == 0) launch_flow_part<RK_FIRST, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    else if (stage < 3) launch_flow_part<RK_MIDDLE, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    else launch_flow_part<RK_LAST, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
 }
 
 // Every launch that writes per-block partials checks the buffer first: `per_block` values
@@ -135,8 +157,7 @@ cudaError_t step_impl(DevCtx& c, double dt, int t_loop, bool device_mode) {
     for (int q = 0; q < NACC; q++) kd.p[q] = c.debug ? (R*)c.kd[q] : nullptr;
     KDbg<R> knone;
     for (int q = 0; q < NACC; q++) knone.p[q] = nullptr;
-    KFlow<R> kf;
-    for (int q = 0; q < 4; q++) kf.p[q] = (R*)c.kflow[q];
+    RS* rn = (RS*)c.rn;
 
     int tm = tmark_begin(c, 0);
     if (device_mode) loop_pre(c);
@@ -165,12 +186,12 @@ cudaError_t step_impl(DevCtx& c, double dt, int t_loop, bool device_mode) {
         tmark_end(c, tm);
         // the k-arrays of the first stage are kept for inspection when requested
         const KDbg<R>& kds = (s == 0) ? kd : knone;
-        tm = tmark_begin(c, 3);
-        launch_flow<R, false>(gC, bC, st, c.hC, c.attr, F, P, kf, kds, c.dS, Batch{});
-        tmark_end(c, tm);
         tm = tmark_begin(c, 5);
-        if (c.scalar_tma && c.tma_ok) launch_scalar_tma<R, RS>(c, st, F, P, S, St, acc, kf, kds, s);
-        else launch_scalar<R, false>(gD, bD, st, c.hC, c.attr, F, P, S, St, acc, kf, kds, c.dS, s, Batch{});
+        if (c.scalar_tma && c.tma_ok) launch_scalar_tma<R, RS>(c, st, F, P, S, St, acc, rn, kds, s);
+        else launch_scalar<R, false>(gD, bD, st, c.hC, c.attr, F, P, S, St, acc, rn, kds, c.dS, s, Batch{});
+        tmark_end(c, tm);
+        tm = tmark_begin(c, 3);
+        launch_flow<R, false>(gC, bC, st, c.hC, c.attr, F, P, S, St, acc, rn, kds, c.dS, s, Batch{});
         tmark_end(c, tm);
     }
     // apply_boundary_conditions (:2967-3161)
@@ -226,14 +247,13 @@ cudaError_t batch_stages(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t
     for (int q = 0; q < NACC; q++) acc.p[q] = (R*)c0.acc[q];
     KDbg<R> knone;
     for (int q = 0; q < NACC; q++) knone.p[q] = nullptr;
-    KFlow<R> kf;
-    for (int q = 0; q < 4; q++) kf.p[q] = (R*)c0.kflow[q];
+    RS* rn = (RS*)c0.rn;
     for (int s = 0; s < 4; s++) {
         if (s == 0) k_filter_props<R, RS, true><<<gA, bA, 0, st>>>(c0.hC, c0.attr, S, F, P, c0.part, c0.dS, 0, BA);
         else k_filter_props<R, R, true><<<gA, bA, 0, st>>>(c0.hC, c0.attr, St, F, P, c0.part, c0.dS, s == 3 ? 1 : 0, BA);
         launch_strain<R, true>(gB, bB, st, c0.hC, c0.attr, F, P, BB);
-        launch_flow<R, true>(gC, bC, st, c0.hC, c0.attr, F, P, kf, knone, c0.dS, BC);
-        launch_scalar<R, true>(gD, bD, st, c0.hC, c0.attr, F, P, S, St, acc, kf, knone, c0.dS, s, BD);
+        launch_scalar<R, true>(gD, bD, st, c0.hC, c0.attr, F, P, S, St, acc, rn, knone, c0.dS, s, BD);
+        launch_flow<R, true>(gC, bC, st, c0.hC, c0.attr, F, P, S, St, acc, rn, knone, c0.dS, s, BC);
     }
     return cudaGetLastError();
 }
@@ -253,8 +273,7 @@ cudaError_t rhs_only_impl(DevCtx& c, int t_loop) {
     for (int q = 0; q < NACC; q++) acc.p[q] = (R*)c.acc[q];
     KDbg<R> kd;
     for (int q = 0; q < NACC; q++) kd.p[q] = (R*)c.kd[q];
-    KFlow<R> kf;
-    for (int q = 0; q < 4; q++) kf.p[q] = (R*)c.kflow[q];
+    RS* rn = (RS*)c.rn;
     k_set_step<<<1, 1, 0, st>>>(c.dS, 0.0, t_loop);
     int tm = tmark_begin(c, 1);
     k_filter_props<R, RS><<<cell_grid(c, SH_FILTER), cell_block(c, SH_FILTER), 0, st>>>(c.hC, c.attr, S, F, P,
@@ -263,16 +282,16 @@ cudaError_t rhs_only_impl(DevCtx& c, int t_loop) {
     tm = tmark_begin(c, 2);
     launch_strain<R, false>(cell_grid(c, SH_STRAIN), cell_block(c, SH_STRAIN), st, c.hC, c.attr, F, P, Batch{});
     tmark_end(c, tm);
-    tm = tmark_begin(c, 3);
-    launch_flow<R, false>(cell_grid(c, SH_FLOW), cell_block(c, SH_FLOW), st, c.hC, c.attr, F, P, kf, kd, c.dS,
-                          Batch{});
-    tmark_end(c, tm);
     tm = tmark_begin(c, 5);
     if (c.scalar_tma && c.tma_ok)
-        launch_scalar_tma<R, RS>(c, st, F, P, S, St, acc, kf, kd, 0);
+        launch_scalar_tma<R, RS>(c, st, F, P, S, St, acc, rn, kd, 0);
     else
         launch_scalar<R, false>(cell_grid(c, SH_SCALAR), cell_block(c, SH_SCALAR), st, c.hC, c.attr, F, P, S, St,
-                                acc, kf, kd, c.dS, 0, Batch{});
+                                acc, rn, kd, c.dS, 0, Batch{});
+    tmark_end(c, tm);
+    tm = tmark_begin(c, 3);
+    launch_flow<R, false>(cell_grid(c, SH_FLOW), cell_block(c, SH_FLOW), st, c.hC, c.attr, F, P, S, St, acc, rn, kd,
+                          c.dS, 0, Batch{});
     tmark_end(c, tm);
     tmark_flush(c);
     return cudaGetLastError();

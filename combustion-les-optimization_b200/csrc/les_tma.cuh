@@ -131,10 +131,10 @@ __device__ __forceinline__ bool tma_wait(uint32_t bar, uint32_t phase) {
 }
 
 // The scalar pass over a (32 x 8) tile and i-planes [blockIdx.z * iseg, + iseg).
-template <typename R, typename RS>
+template <int PART, typename R, typename RS>
 __global__ void __launch_bounds__(TMA_TK* TMA_TJ, (sizeof(R) == 8) ? 2 : 3)
     k_rhs_scalar_tma(LES_KERNEL_CONSTS, const __grid_constant__ TmaMaps M, const uint8_t* __restrict__ attr, F11<R> F,
-                     PropBuf<R> P, F11<RS> S0, F11<R> St, AccBuf<R> acc, KFlow<R> kf, KDbg<R> kd,
+                     PropBuf<R> P, F11<RS> S0, F11<R> St, AccBuf<R> acc, RS* __restrict__ rn, KDbg<R> kd,
                      Scalars* __restrict__ Sc, int stage, int iseg) {
     using G = TmaGeom<R>;
     extern __shared__ __align__(128) unsigned char tma_smem[];
@@ -199,13 +199,13 @@ __global__ void __launch_bounds__(TMA_TK* TMA_TJ, (sizeof(R) == 8) ? 2 : 3)
         if (k < C.nz && j < C.ny && i + 1 < i1) {
             const size_t idn = cid(i + 1, j, k, C.ny, C.nz);
 #pragma unroll
-            for (int q = 0; q < NSTATE; q++) asm volatile("prefetch.global.L2 [%0];" ::"l"(S0.p[q] + idn));
-            if (stage > 0) {
+            for (int q = 3; q < NSTATE; q++)
+                if (q != 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(S0.p[q] + idn));
+            if (PART != RK_FIRST) {
 #pragma unroll
-                for (int q = 0; q < NACC; q++) asm volatile("prefetch.global.L2 [%0];" ::"l"(acc.p[q] + idn));
+                for (int q = 3; q < NACC; q++)
+                    if (q != 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(acc.p[q] + idn));
             }
-#pragma unroll
-            for (int q = 0; q < 4; q++) asm volatile("prefetch.global.L2 [%0];" ::"l"(kf.p[q] + idn));
 #pragma unroll
             for (int q = 0; q < NSP; q++) asm volatile("prefetch.global.L2 [%0];" ::"l"(P.D[q] + idn));
             asm volatile("prefetch.global.L2 [%0];" ::"l"(P.aT + idn));
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(TMA_TK* TMA_TJ, (sizeof(R) == 8) ? 2 : 3)
                 src.nut[d] = reinterpret_cast<const R*>(nbase + nslot * G::NSTRIDE) + (jl + 1) * G::BW +
                              (kl + G::KOFF);
             }
-            rhs_scalar_cell<R, RS>(C, attr, F, P, S0, St, acc, kf, kd, Sc, stage, i, j, k, src, (R)kc<R>(C).relax);
+            rhs_scalar_cell<PART, R, RS>(C, attr, F, P, S0, St, acc, rn, kd, Sc, stage, i, j, k, src, (R)kc<R>(C).relax);
         }
         __syncthreads();                            // the plane of step rc - 2 is free
         if (tid == 0 && rc + 3 < nsteps) {
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(TMA_TK* TMA_TJ, (sizeof(R) == 8) ? 2 : 3)
 // resident blocks (at least 4 planes per segment).
 template <typename R, typename RS>
 cudaError_t launch_scalar_tma(const DevCtx& c, cudaStream_t st, const F11<R>& F, const PropBuf<R>& P,
-                              const F11<RS>& S, const F11<R>& St, const AccBuf<R>& acc, const KFlow<R>& kf,
+                              const F11<RS>& S, const F11<R>& St, const AccBuf<R>& acc, RS* rn,
                               const KDbg<R>& kd, int stage) {
     using G = TmaGeom<R>;
     const int gx = (c.nz + TMA_TK - 1) / TMA_TK, gy = (c.ny + TMA_TJ - 1) / TMA_TJ;
@@ -259,16 +259,28 @@ cudaError_t launch_scalar_tma(const DevCtx& c, cudaStream_t st, const F11<R>& F,
     if (iseg < 4) iseg = 4;
     if (iseg > c.nx) iseg = c.nx;
     const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)((c.nx + iseg - 1) / iseg));
-    k_rhs_scalar_tma<R, RS><<<grid, dim3(TMA_TK, TMA_TJ), G::SMEM, st>>>(
-        c.hC, *reinterpret_cast<const TmaMaps*>(c.tma_maps), c.attr, F, P, S, St, acc, kf, kd, c.dS, stage, (int)iseg);
+    const dim3 block(TMA_TK, TMA_TJ);
+    const TmaMaps& maps = *reinterpret_cast<const TmaMaps*>(c.tma_maps);
+    if (stage == 0)
+        k_rhs_scalar_tma<RK_FIRST, R, RS><<<grid, block, G::SMEM, st>>>(c.hC, maps, c.attr, F, P, S, St, acc, rn, kd,
+                                                                       c.dS, stage, (int)iseg);
+    else if (stage < 3)
+        k_rhs_scalar_tma<RK_MIDDLE, R, RS><<<grid, block, G::SMEM, st>>>(c.hC, maps, c.attr, F, P, S, St, acc, rn, kd,
+                                                                        c.dS, stage, (int)iseg);
+    else
+        k_rhs_scalar_tma<RK_LAST, R, RS><<<grid, block, G::SMEM, st>>>(c.hC, maps, c.attr, F, P, S, St, acc, rn, kd,
+                                                                      c.dS, stage, (int)iseg);
     return cudaGetLastError();
 }
 
 // Once per process and instantiation: allow the staged kernel its dynamic shared memory.
 template <typename R, typename RS>
 cudaError_t prepare_scalar_tma() {
-    return cudaFuncSetAttribute(k_rhs_scalar_tma<R, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                TmaGeom<R>::SMEM);
+    const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_rhs_scalar_tma<RK_FIRST, R, RS>, at, TmaGeom<R>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rhs_scalar_tma<RK_MIDDLE, R, RS>, at, TmaGeom<R>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rhs_scalar_tma<RK_LAST, R, RS>, at, TmaGeom<R>::SMEM);
+    return e;
 }
 
 }  // namespace les
