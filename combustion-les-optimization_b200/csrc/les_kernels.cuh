@@ -3,12 +3,12 @@
 // accumulated in double.
 //
 // One RK4 stage is four passes over the grid:
-//   A  k_filter_props : 7-point box filter of the 11 stage fields (apply_box_filter,
-//                       les_combustion_solver.c:1307-1470) and the cell-local mixture
-//                       properties (update_nu_mix :1489, update_Dk :1684, update_Cp_mix
-//                       :1762, update_lambda_mix_alpha :1798); partial sums for <rho_f>.
-//   B  k_strain       : resolved strain, G-dependent Smagorinsky nu_t (calculate_nu_t
-//                       :1569), SSR-SGS flame speed (:1913) and mu_eff = mu + rho_f nu_t.
+//   A  k_filter       : 7-point box filter of the 11 stage fields (apply_box_filter,
+//                       les_combustion_solver.c:1307-1470); partial sums for <rho_f>.
+//   B  k_props        : cell-local mixture properties (update_nu_mix :1489, update_Dk :1684,
+//                       update_Cp_mix :1762, update_lambda_mix_alpha :1798), resolved strain,
+//                       G-dependent Smagorinsky nu_t (calculate_nu_t :1569), SSR-SGS flame
+//                       speed (:1913) and mu_eff = mu + rho_f nu_t.
 //   C1 k_rhs_scalar   : species and temperature right-hand sides (:2837-2962) fused with
 //                       the RK4 stage update (:4432-4455) or the final combine (:4517-4544)
 //                       of T, Y_k and rho; the new density is handed to C2.
@@ -83,16 +83,14 @@ __device__ __forceinline__ void shift_props(PropBuf<R>& P, long long d) {
     P.grad_g = nullptr;
 }
 
-// Minimum resident blocks per SM requested from the register allocator (filter / strain / flow /
-// scalar).  Swept on B200 at 256x128x128, ms per step (four launches): FP64 flow 0.95 at 5 blocks,
-// 0.91 at 4, 1.01 at 3, 1.29 at 2; scalar 1.40 at 5, 1.38 at 4, 1.51 at 3 and 2; FP32 flow
-// 0.617 at 7, 0.610 at 6 and 5 (at 96x48x48 0.0775, 0.0729, 0.0705), 0.658 at 4; scalar 1.06 at 7,
-// 1.04 at 6, 0.91 at 5, 0.88 at 4.
-#ifndef LES_MINB_FILTER
-#define LES_MINB_FILTER 5
-#endif
-#ifndef LES_MINB_STRAIN
-#define LES_MINB_STRAIN 3
+// Minimum resident blocks per SM requested from the register allocator (properties / flow /
+// scalar).  Swept on B200 at 256x128x128, ms per step (four launches): FP64 properties 1.13 at 5
+// blocks, 1.11 at 4, 1.16 at 3, 1.32 at 2; flow 0.95 at 5, 0.91 at 4, 1.01 at 3, 1.29 at 2; scalar
+// 1.40 at 5, 1.38 at 4, 1.51 at 3 and 2; FP32 properties 0.54 at 8, 0.505 at 6, 0.513 at 5, 0.536
+// at 4; flow 0.617 at 7, 0.610 at 6 and 5 (at 96x48x48 0.0775, 0.0729, 0.0705), 0.658 at 4; scalar
+// 1.06 at 7, 1.04 at 6, 0.91 at 5, 0.88 at 4.
+#ifndef LES_MINB_PROPS
+#define LES_MINB_PROPS 4
 #endif
 #ifndef LES_MINB_FLOW
 #define LES_MINB_FLOW 4
@@ -100,11 +98,8 @@ __device__ __forceinline__ void shift_props(PropBuf<R>& P, long long d) {
 #ifndef LES_MINB_SCALAR
 #define LES_MINB_SCALAR 4
 #endif
-#ifndef LES_MINB_FILTER_F32
-#define LES_MINB_FILTER_F32 8
-#endif
-#ifndef LES_MINB_STRAIN_F32
-#define LES_MINB_STRAIN_F32 8
+#ifndef LES_MINB_PROPS_F32
+#define LES_MINB_PROPS_F32 6
 #endif
 #ifndef LES_MINB_FLOW_F32
 #define LES_MINB_FLOW_F32 5
@@ -114,12 +109,12 @@ __device__ __forceinline__ void shift_props(PropBuf<R>& P, long long d) {
 #endif
 template <typename R>
 struct MinBlocks {
-    static constexpr int filter = LES_MINB_FILTER, strain = LES_MINB_STRAIN, flow = LES_MINB_FLOW,
+    static constexpr int props = LES_MINB_PROPS, flow = LES_MINB_FLOW,
                          scalar = LES_MINB_SCALAR;
 };
 template <>
 struct MinBlocks<float> {
-    static constexpr int filter = LES_MINB_FILTER_F32, strain = LES_MINB_STRAIN_F32, flow = LES_MINB_FLOW_F32,
+    static constexpr int props = LES_MINB_PROPS_F32, flow = LES_MINB_FLOW_F32,
                          scalar = LES_MINB_SCALAR_F32;
 };
 // The same register budget for a block of `ntb` threads: the resident threads per SM of the
@@ -482,83 +477,287 @@ __device__ __forceinline__ bool cell_props_fast(const Consts& C, const double* t
     return true;
 }
 
-// ------------------------------------------------------------------ pass A: filter + props
+// ------------------------------------------------------------------ pass A: filter
 
-template <typename R, typename RI = R, bool BATCH = false>
-__global__ void __launch_bounds__(NT, MinBlocks<R>::filter)
-    k_filter_props(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<RI> in, F11<R> F, PropBuf<R> P,
-                   double* __restrict__ part, Scalars* __restrict__ S, int want_max, Batch B) {
-    const auto& K = kc<R>(C);
-    __shared__ double sh[NT / 32];
+// Block partials of one or more reductions into part[q * nblk + block]; true in the last block to
+// arrive, whose threads may then reduce them.
+__device__ __forceinline__ bool last_block(double* part, unsigned nblk, unsigned bid, const double* v, int nv,
+                                           unsigned* counter, int tid) {
     __shared__ bool last;
+    if (tid == 0) {
+        for (int q = 0; q < nv; q++) part[(size_t)q * nblk + bid] = v[q];
+        __threadfence();
+        last = atomicAdd(counter, 1u) == nblk - 1;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// V consecutive values as 16-byte loads and stores.
+template <typename T, int V>
+__device__ __forceinline__ void ld_vec(const T* __restrict__ p, T (&v)[V]) {
+    if constexpr (V == 1) {
+        v[0] = __ldg(p);
+    } else if constexpr (sizeof(T) == 8) {
+        const double2 t = __ldg(reinterpret_cast<const double2*>(p));
+        v[0] = t.x; v[1] = t.y;
+    } else {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    }
+}
+template <int V>
+__device__ __forceinline__ void st_vec(double* p, const double (&v)[V]) {
+    if constexpr (V == 1) *p = v[0];
+    else *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+}
+template <int V>
+__device__ __forceinline__ void st_vec(float* p, const float (&v)[V]) {
+    if constexpr (V == 1) *p = v[0];
+    else if constexpr (V == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+    else *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+// V attribute bytes; id is a multiple of V.
+template <int V>
+__device__ __forceinline__ void ld_attr(const uint8_t* __restrict__ p, int (&a)[V]) {
+    if constexpr (V == 1) {
+        a[0] = __ldg(p);
+    } else if constexpr (V == 2) {
+        const uchar2 t = __ldg(reinterpret_cast<const uchar2*>(p));
+        a[0] = t.x; a[1] = t.y;
+    } else {
+        const uchar4 t = __ldg(reinterpret_cast<const uchar4*>(p));
+        a[0] = t.x; a[1] = t.y; a[2] = t.z; a[3] = t.w;
+    }
+}
+
+// apply_box_filter (:1307-1470) of the 11 stage fields and the stage's <rho_f> (:2536-2550).  Bound
+// by memory: 11 fields in and 11 out with nothing but sums between, so each block takes one field
+// (blockIdx.z) and needs few registers, each thread V cells of a row in 16-byte accesses and
+// marches through seg planes, keeping the planes before, at and after the current one.  One field a
+// block also gives small grids 11 times the blocks.  V > 1 needs rows that are a multiple of V
+// values; other grids take V = 1.  The mixture properties, which compute and need 7 of the 11
+// fields, are in the next pass: in one kernel the filter's loads waited for registers that the
+// properties held.  256x128x128, ms per step: filter and properties and, apart, strain took
+// 1.63 + 0.60 (FP64) and 0.92 + 0.24 (FP32); the filter alone, a cell a thread and 11 fields a block,
+// 0.76 and 0.58; in this form 0.59 and 0.36 (176 bytes a cell, 5.0 TB/s; seg = 4: 0.63, 16: 0.60,
+// 1: 0.92), with properties and strain together at 1.11 and 0.505.
+template <int V, typename R, typename RI = R, bool BATCH = false>
+__global__ void __launch_bounds__(NT)
+    k_filter(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<RI> in, F11<R> F, double* __restrict__ part,
+             Scalars* __restrict__ S, int seg, Batch B) {
+    int q = blockIdx.z;
+    if constexpr (BATCH) {
+        const int m = blockIdx.z / NSTATE;
+        q = blockIdx.z - m * NSTATE;
+        const MemberTab& e = B.mt[m];
+        shift_all(in, e.delta);
+        shift_all(F, e.delta);
+        attr = e.attr;
+        part = e.part;
+        S = e.S;
+    }
+    const RI* __restrict__ x = in.p[0];
+    R* __restrict__ y = F.p[0];
+#pragma unroll
+    for (int s = 1; s < NSTATE; s++)
+        if (q == s) { x = in.p[s]; y = F.p[s]; }
+    const int nx = C.nx, ny = C.ny, nz = C.nz, nv = nz / V;
+    const int tid = threadIdx.x, sI = ny * nz;
+    const int pv = blockIdx.x * NT + tid;
+    const int i0 = blockIdx.y * seg, i1 = min(i0 + seg, nx);
+    double mass = 0.0;
+    if (pv < ny * nv) {
+        const int j = pv / nv, k = (pv - j * nv) * V;
+        const bool row = j >= 1 && j < ny - 1;
+        int id = i0 * sI + j * nz + k;
+        RI lo[V], c[V], hi[V];
+        ld_vec<RI, V>(x + id, c);
+#pragma unroll
+        for (int v = 0; v < V; v++) lo[v] = c[v];
+        if (i0 > 0) ld_vec<RI, V>(x + id - sI, lo);
+        for (int i = i0; i < i1; i++, id += sI) {
+            int a[V];
+            ld_attr<V>(attr + id, a);
+            if (i + 1 < nx) ld_vec<RI, V>(x + id + sI, hi);
+            R f[V];
+            if (row && i >= 1 && i < nx - 1) {
+                RI dn[V], up[V];
+                ld_vec<RI, V>(x + id - nz, dn);
+                ld_vec<RI, V>(x + id + nz, up);
+                const RI left = k > 0 ? __ldg(x + id - 1) : RI(0), right = k + V < nz ? __ldg(x + id + V) : RI(0);
+#pragma unroll
+                for (int v = 0; v < V; v++) {
+                    // (50 x + six neighbours) / 56 as x + (neighbours - 6 x) / 56: fewer roundings at
+                    // the size of x, and a uniform field stays exactly what it is.  In the input's
+                    // type: the FP32 form's first stage reads the FP64 state.
+                    const RI kl = v > 0 ? c[v > 0 ? v - 1 : 0] : left, kr = v < V - 1 ? c[v < V - 1 ? v + 1 : 0] : right;
+                    const RI nb = lo[v] + dn[v] + kl + kr + up[v] + hi[v];
+                    const bool inner = a[v] == 3 && k + v >= 1 && k + v < nz - 1;
+                    f[v] = R(inner ? fma(fma(RI(-6.0), c[v], nb), RI(1.0 / 56.0), c[v]) : c[v]);
+                }
+            } else {
+#pragma unroll
+                for (int v = 0; v < V; v++) f[v] = R(c[v]);
+            }
+            st_vec<V>(y + id, f);
+            if (q == 5) {
+#pragma unroll
+                for (int v = 0; v < V; v++)
+                    if (a[v] == 1 || a[v] == 2 || a[v] == 3 || a[v] == 5) mass += (((double)f[v] * C.dx) * C.dy) * C.dz;
+            }
+#pragma unroll
+            for (int v = 0; v < V; v++) { lo[v] = c[v]; c[v] = hi[v]; }
+        }
+    }
+    if (q != 5) return;
+    // partial sums for <rho_f>; in a batched launch, over the member's own blocks
+    __shared__ double sh[NT / 32];
+    const unsigned nblk = gridDim.x * gridDim.y, bid = blockIdx.y * gridDim.x + blockIdx.x;
+    const double bm = block_sum<NT>(mass, sh, tid);
+    if (last_block(part, nblk, bid, &bm, 1, &S->counter[0], tid)) {
+        double s = 0.0;
+        // unrolled so that the partials' loads are in flight together; each thread still adds
+        // its entries in ascending order, so the sum is unchanged
+#pragma unroll 8
+        for (unsigned b = tid; b < nblk; b += NT) s += __ldcg(&part[b]);
+        s = block_sum<NT>(s, sh, tid);
+        if (tid == 0) {
+            S->rho_avg = (C.total_volume > 0) ? (s / C.total_volume) : 1.2;
+            S->counter[0] = 0u;
+        }
+    }
+}
+
+// ------------------------------------------------------------------ pass B: properties, strain, nu_t, S_T
+
+// keep: the last RHS evaluation of a step (or one on its own): mu, nu and |S| are written for
+// inspection and the probe lines, which no other pass reads, and the nu/alpha maxima that feed the
+// next dt are taken (:4401-4408).
+template <typename R, bool BATCH = false, int NTB = NT>
+__global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
+    k_props(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, double* __restrict__ part,
+            Scalars* __restrict__ S, int keep, Batch B) {
+    const auto& K = kc<R>(C);
+    __shared__ double sh[NTB / 32];
     __shared__ double tab[EXP_STEPS];
     int bz = blockIdx.z;
+    ModelK<R> M;
     if constexpr (BATCH) {
         const int m = blockIdx.z / B.gz;
         bz = blockIdx.z - m * B.gz;
         const MemberTab& e = B.mt[m];
-        shift_all(in, e.delta);
         shift_all(F, e.delta);
         shift_props(P, e.delta);
         attr = e.attr;
         part = e.part;
         S = e.S;
+        M = member_model<R>(e);
+    } else {
+        M = model_of<R>(C);
     }
     const int nx = C.nx, ny = C.ny, nz = C.nz;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = bz * blockDim.z + threadIdx.z;
     const int tid = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
-    const ptrdiff_t sI = (ptrdiff_t)ny * nz, sJ = (ptrdiff_t)nz;
-    if (std::is_same<R, double>::value && tid < EXP_STEPS) tab[tid] = C.exp_tab[tid];
-    double mass = 0.0, mnu = 0.0, mal = 0.0;
-    const bool here = k < nz && j < ny && i < C.nx;
-    const size_t id = here ? cid(i, j, k, ny, nz) : 0;
-    const int a = here ? attr[id] : 0;
-    R f[NSTATE];
-    if (here) {
-        const bool filt = (a == 3) && i >= 1 && i < nx - 1 && j >= 1 && j < ny - 1 && k >= 1 && k < nz - 1;
-        // (50 x + six neighbours) / 56 (:1307-1470) as x + (neighbours - 6 x) / 56: fewer roundings
-        // at the size of x, and a uniform field stays exactly what it is.  In the input's type:
-        // the FP32 form's first stage reads the FP64 state and converts one value instead of seven.
-#pragma unroll
-        for (int q = 0; q < NSTATE; q++) {
-            const RI* __restrict__ x = in.p[q] + id;
-            const RI x0 = x[0];
-            RI v = x0;
-            if (filt) v = fma(fma(RI(-6.0), x0, x[-sI] + x[-sJ] + x[-1] + x[1] + x[sJ] + x[sI]), RI(1.0 / 56.0), x0);
-            f[q] = R(v);
-        }
-        // stored after the last load: a store may alias the next field's loads as far as the
-        // compiler knows, and would make them wait for this field's
-#pragma unroll
-        for (int q = 0; q < NSTATE; q++) F.p[q][id] = f[q];
+    if constexpr (std::is_same<R, double>::value) {
+        if (tid < EXP_STEPS) tab[tid] = C.exp_tab[tid];
+        __syncthreads();
     }
-    if constexpr (std::is_same<R, double>::value) __syncthreads();   // exp2_fit's table
-    if (here) {
-        if (a == 1 || a == 2 || a == 3 || a == 5) mass = (((double)f[5] * C.dx) * C.dy) * C.dz;
-        if (a == 3) {
-            CellProps<R> o;
-            auto store_d = [&](const R* D) {
+    double mnu = 0.0, mal = 0.0;
+    const bool here = k < nz && j < ny && i < nx;
+    const int id = here ? (int)cid(i, j, k, ny, nz) : 0;
+    const bool interior = here && i >= 1 && i < nx - 1 && j >= 1 && j < ny - 1 && k >= 1 && k < nz - 1;
+    const int a = here ? attr[id] : 0;
+    if (a == 3) {
+        R T = F.p[3][id], rho = F.p[5][id], G = F.p[4][id], Y[NSP];
 #pragma unroll
-                for (int s = 0; s < NSP; s++) P.D[s][id] = D[s];
-            };
-            if (!cell_props_fast<R>(C, tab, f[3], &f[6], f[5], store_d, o)) {
-                CellProps<R> g;
-                R Yf[NSP];
+        for (int s = 0; s < NSP; s++) Y[s] = F.p[6 + s][id];
+        R num = R(0), div = R(0), nut = R(0), Smag = R(0);
+        if (interior) {
+            const int sI = ny * nz, sJ = nz;
+            const R* __restrict__ uf = F.p[0] + id;
+            const R* __restrict__ vf = F.p[1] + id;
+            const R* __restrict__ wf = F.p[2] + id;
+            const R du_dx = (uf[sI] - uf[-sI]) * K.d_2dx.r, dv_dy = (vf[sJ] - vf[-sJ]) * K.d_2dy.r;
+            const R dw_dz = (wf[1] - wf[-1]) * K.d_2dz.r, du_dy = (uf[sJ] - uf[-sJ]) * K.d_2dy.r;
+            const R du_dz = (uf[1] - uf[-1]) * K.d_2dz.r, dv_dx = (vf[sI] - vf[-sI]) * K.d_2dx.r;
+            const R dv_dz = (vf[1] - vf[-1]) * K.d_2dz.r, dw_dx = (wf[sI] - wf[-sI]) * K.d_2dx.r;
+            const R dw_dy = (wf[sJ] - wf[-sJ]) * K.d_2dy.r;
+            R S11 = du_dx, S22 = dv_dy, S33 = dw_dz;
+            R S12 = R(0.5) * (du_dy + dv_dx), S13 = R(0.5) * (du_dz + dw_dx), S23 = R(0.5) * (dv_dz + dw_dy);
+            const R off = fma(S23, S23, fma(S13, S13, S12 * S12));
+            const R Sij = fma(R(2.0), off, fma(S33, S33, fma(S22, S22, S11 * S11)));
+            Smag = qsqrt(R(2.0) * Sij);
+            div = du_dx + dv_dy + dw_dz;
+            R g = G;
+            if (g < R(0.0)) g = R(0.0);
+            if (g > R(1.0)) g = R(1.0);
+            R cs = fma(M.cs_b - M.cs_u, g, M.cs_u);
+            cs = fma(M.cs_boost * R(4.0) * g, R(1.0) - g, cs);
+            const R dx = (R)K.dx;
+            nut = (cs * dx) * (cs * dx) * Smag;
+            num = fma(-div * div, R(1.0 / 3.0), Sij);
+        }
+        CellProps<R> o;
+        auto store_d = [&](const R* D) {
 #pragma unroll
-                for (int s = 0; s < NSP; s++) Yf[s] = f[6 + s];
-                cell_props_any<R>(C, f[3], Yf, f[5], &g);
-                store_d(g.D);
-                o = g;
-            }
+            for (int s = 0; s < NSP; s++) P.D[s][id] = D[s];
+        };
+        if (!cell_props_fast<R>(C, tab, T, Y, rho, store_d, o)) {
+            CellProps<R> g;
+            R Yf[NSP];
+#pragma unroll
+            for (int s = 0; s < NSP; s++) Yf[s] = Y[s];
+            cell_props_any<R>(C, T, Yf, rho, &g);
+            store_d(g.D);
+            o = g;
+        }
+        mnu = (double)o.nu;
+        mal = (double)o.alpha;
+        P.aT[id] = o.aT;
+        P.nu_t[id] = nut;
+        P.mu_eff[id] = interior ? fma(rho, nut, o.mu_mix) : R(0);
+        if (keep) {
             P.mu_mix[id] = o.mu_mix;
             P.nu[id] = o.nu;
-            P.aT[id] = o.aT;
-            if (P.dbg_cp) { P.dbg_cp[id] = o.cp; P.dbg_lam[id] = o.lam; P.dbg_alpha[id] = o.alpha; }
-            mnu = (double)o.nu;
-            mal = (double)o.alpha;
-        } else if (P.dbg_cp) {
+            P.S_mag[id] = Smag;
+        }
+        if (P.dbg_cp) { P.dbg_cp[id] = o.cp; P.dbg_lam[id] = o.lam; P.dbg_alpha[id] = o.alpha; }
+        R ST = R(0);
+        if (interior) {
+            const R dx = (R)K.dx, nul = o.nu;
+            // SSR-SGS turbulent flame speed (:1926-1957)
+            const R X = (R)K.dx4 * num * frcp(nul * nul);
+            R d_eta = R(1.0);
+            if (!(X < R(SMALL))) {
+                // X^(3/4) = sqrt(X) sqrt(sqrt(X)): two square roots instead of a power
+                const R y = qsqrt(X), pX = y * qsqrt(y), arg = R(SSR_B) * pX;
+                d_eta = R(SSR_A) * pX * (arg > R(1.0) ? qlog(arg) : R(0.0));
+            }
+            const R eta = qdiv(dx, d_eta + R(SMALL));
+            R te = R(0.0);
+            if (K.tau_sl > R(SMALL)) te = dx * fmax(R(0.0), div) * K.d_tau_sl.r;
+            // The wrinkling ratio (8 exp(c / (8 eta)) eta / dx)^(2 - D3) is at most 1 where 8 eta >= dx and
+            // the exponent is negative (c >= 0); without dilatation the speed is then S_L whatever its
+            // value, and the exponential, the logarithm and the power are left out.
+            R st = (R)K.s_l;
+            if (!(te <= R(0.0) && K.ssr_exp <= R(0.0) && K.ssr_cdF >= R(0.0) && R(8.0) * eta >= dx)) {
+                const R z = qdiv((R)K.ssr_cdF, fma(R(8.0), eta, R(SMALL)));
+                const R wr = qexp((R)K.ssr_exp * (qlog(R(8.0) * eta * K.d_dx.r) + z));
+                st = (R)K.s_l * fmax(R(0.0), wr + te);
+            }
+            ST = fmax((R)K.s_l, st);
+        }
+        P.ST[id] = ST;
+    } else if (here) {
+        P.nu_t[id] = R(0);
+        P.ST[id] = interior ? (R)K.s_l : R(0);
+        P.mu_eff[id] = R(0);
+        if (keep) P.S_mag[id] = R(0);
+        if (P.dbg_cp) {
             // property values of non-fluid cells are never read by the step; they are filled
             // only for inspection, with the reference's defaults
             P.mu_mix[id] = R(1.8e-5);
@@ -569,128 +768,26 @@ __global__ void __launch_bounds__(NT, MinBlocks<R>::filter)
             P.dbg_cp[id] = R(1000.0); P.dbg_lam[id] = R(0); P.dbg_alpha[id] = R(0);
         }
     }
-    // partial sums for the stage's <rho_f> (:2536-2550) and, on the last stage, the
-    // nu/alpha maxima that feed the next dt (:4401-4408); in a batched launch, over the
-    // member's own blocks
+    if (!keep) return;
     const unsigned nblk = gridDim.x * gridDim.y * (BATCH ? (unsigned)B.gz : gridDim.z);
     const unsigned bid = ((unsigned)bz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    double bm = block_sum<NT>(mass, sh, tid);
-    double bn = 0.0, ba = 0.0;
-    if (want_max) {
-        bn = block_max<NT>(mnu, sh, tid);
-        ba = block_max<NT>(mal, sh, tid);
-    }
-    if (tid == 0) {
-        part[bid] = bm;
-        if (want_max) { part[nblk + bid] = bn; part[2 * nblk + bid] = ba; }
-        __threadfence();
-        unsigned t = atomicAdd(&S->counter[0], 1u);
-        last = (t == nblk - 1);
-    }
-    __syncthreads();
-    if (last) {
-        __threadfence();
-        double s = 0.0, mn = 0.0, ma = 0.0;
-        // unrolled so that the partials' loads are in flight together; each thread still adds
-        // its entries in ascending order, so the sum is unchanged
+    double v[2];
+    v[0] = block_max<NTB>(mnu, sh, tid);
+    v[1] = block_max<NTB>(mal, sh, tid);
+    if (last_block(part, nblk, bid, v, 2, &S->counter[2], tid)) {
+        double mn = 0.0, ma = 0.0;
 #pragma unroll 8
-        for (unsigned q = tid; q < nblk; q += NT) {
-            s += __ldcg(&part[q]);
-            if (want_max) { mn = fmax(mn, __ldcg(&part[nblk + q])); ma = fmax(ma, __ldcg(&part[2 * nblk + q])); }
+        for (unsigned q = tid; q < nblk; q += NTB) {
+            mn = fmax(mn, __ldcg(&part[q]));
+            ma = fmax(ma, __ldcg(&part[nblk + q]));
         }
-        s = block_sum<NT>(s, sh, tid);
-        if (want_max) { mn = block_max<NT>(mn, sh, tid); ma = block_max<NT>(ma, sh, tid); }
+        mn = block_max<NTB>(mn, sh, tid);
+        ma = block_max<NTB>(ma, sh, tid);
         if (tid == 0) {
-            S->rho_avg = (C.total_volume > 0) ? (s / C.total_volume) : 1.2;
-            if (want_max) { S->numax = mn; S->alphamax = ma; }
-            S->counter[0] = 0u;
+            S->numax = mn;
+            S->alphamax = ma;
+            S->counter[2] = 0u;
         }
-    }
-}
-
-// ------------------------------------------------------------------ pass B: strain + nu_t + S_T
-
-template <typename R, bool BATCH = false, int NTB = NT>
-__global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::strain, NTB))
-    k_strain(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, Batch B) {
-    const auto& K = kc<R>(C);
-    int bz = blockIdx.z;
-    ModelK<R> M;
-    if constexpr (BATCH) {
-        const int m = blockIdx.z / B.gz;
-        bz = blockIdx.z - m * B.gz;
-        const MemberTab& e = B.mt[m];
-        shift_all(F, e.delta);
-        shift_props(P, e.delta);
-        attr = e.attr;
-        M = member_model<R>(e);
-    } else {
-        M = model_of<R>(C);
-    }
-    const int nx = C.nx, ny = C.ny, nz = C.nz;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i = bz * blockDim.z + threadIdx.z;
-    if (k >= nz || j >= ny || i >= C.nx) return;
-    const ptrdiff_t sI = (ptrdiff_t)ny * nz, sJ = (ptrdiff_t)nz;
-    const size_t id = cid(i, j, k, ny, nz);
-    const bool interior = i >= 1 && i < nx - 1 && j >= 1 && j < ny - 1 && k >= 1 && k < nz - 1;
-    const int a = attr[id];
-    if (interior && a == 3) {
-        const R* __restrict__ uf = F.p[0] + id;
-        const R* __restrict__ vf = F.p[1] + id;
-        const R* __restrict__ wf = F.p[2] + id;
-        R du_dx = cdv(uf[sI] - uf[-sI], K.d_2dx);
-        R dv_dy = cdv(vf[sJ] - vf[-sJ], K.d_2dy);
-        R dw_dz = cdv(wf[1] - wf[-1], K.d_2dz);
-        R du_dy = cdv(uf[sJ] - uf[-sJ], K.d_2dy);
-        R du_dz = cdv(uf[1] - uf[-1], K.d_2dz);
-        R dv_dx = cdv(vf[sI] - vf[-sI], K.d_2dx);
-        R dv_dz = cdv(vf[1] - vf[-1], K.d_2dz);
-        R dw_dx = cdv(wf[sI] - wf[-sI], K.d_2dx);
-        R dw_dy = cdv(wf[sJ] - wf[-sJ], K.d_2dy);
-        R S11 = du_dx, S22 = dv_dy, S33 = dw_dz;
-        R S12 = R(0.5) * (du_dy + dv_dx), S13 = R(0.5) * (du_dz + dw_dx), S23 = R(0.5) * (dv_dz + dw_dy);
-        R Sij = R(2.0) * (S12 * S12 + S13 * S13 + S23 * S23) + S11 * S11 + S22 * S22 + S33 * S33;
-        R Smag = qsqrt(R(2.0) * Sij);
-        R div = du_dx + dv_dy + dw_dz;
-        R g = F.p[4][id];
-        if (g < R(0.0)) g = R(0.0);
-        if (g > R(1.0)) g = R(1.0);
-        R cs = M.cs_u + (M.cs_b - M.cs_u) * g;
-        cs += M.cs_boost * R(4.0) * g * (R(1.0) - g);
-        const R dx = (R)K.dx;
-        R nut = (cs * dx) * (cs * dx) * Smag;
-        P.nu_t[id] = nut;
-        P.S_mag[id] = Smag;
-        P.mu_eff[id] = P.mu_mix[id] + F.p[5][id] * nut;
-        // SSR-SGS turbulent flame speed (:1926-1957)
-        R nul = P.nu[id];
-        R num = Sij - (div * div) * R(1.0 / 3.0);
-        R X = qdiv((R)K.dx4, nul * nul) * num;
-        R d_eta;
-        if (X < R(SMALL)) {
-            d_eta = R(1.0);
-        } else {
-            R pX = qpow(X, R(0.75));
-            R arg = R(SSR_B) * pX;
-            d_eta = R(SSR_A) * pX * (arg > R(1.0) ? qlog(arg) : R(0.0));
-        }
-        R eta = qdiv(dx, d_eta + R(SMALL));
-        R Dce = R(8.0) * eta;
-        R asf = R(8.0) * qexp(qdiv((R)K.ssr_cdF, Dce + R(SMALL)));
-        R base = cdv(asf * eta, K.d_dx);
-        R wr = qpow(base, (R)K.ssr_exp);
-        R te = R(0.0);
-        if (K.tau_sl > R(SMALL)) te = cdv(dx * fmax(R(0.0), div), K.d_tau_sl);
-        R ratio = wr + te;
-        R st = (R)K.s_l * fmax(R(0.0), ratio);
-        P.ST[id] = fmax((R)K.s_l, st);
-    } else {
-        P.nu_t[id] = R(0);
-        P.S_mag[id] = R(0);
-        P.ST[id] = interior ? (R)K.s_l : R(0);
-        P.mu_eff[id] = R(0);
     }
 }
 

@@ -46,12 +46,45 @@ static inline dim3 cell_grid(const DevCtx& c, int cls) {
                 (unsigned)((c.nx + t.bz - 1) / t.bz));
 }
 
-// The strain, flow and scalar passes with the kernel instance of their tile's block size.
+// The filter pass: 16-byte accesses where a row is a multiple of them, and as many planes per
+// thread as leave every SM several blocks.
+constexpr int FILTER_SEG = 8;
+static inline int filter_vec(const DevCtx& c, size_t bytes) {
+    const int v = (int)(16 / bytes);
+    return c.nz % v == 0 ? v : 1;
+}
+static inline dim3 filter_grid(const DevCtx& c, size_t bytes, int& seg) {
+    const int v = filter_vec(c, bytes);
+    const unsigned gx = (unsigned)(((size_t)c.ny * (c.nz / v) + NT - 1) / NT);
+    seg = FILTER_SEG;
+    while (seg > 1 && (size_t)gx * ((c.nx + seg - 1) / seg) * NSTATE < 148 * 12) seg /= 2;
+    return dim3(gx, (unsigned)((c.nx + seg - 1) / seg), NSTATE);
+}
+template <typename R, typename RI, bool BATCH>
+static inline void launch_filter(const DevCtx& c, cudaStream_t st, const F11<RI>& in, const F11<R>& F, int members,
+                                 const Batch& B) {
+    constexpr int V = 16 / sizeof(RI);
+    int seg;
+    dim3 g = filter_grid(c, sizeof(RI), seg);
+    g.z *= (unsigned)members;
+    if (filter_vec(c, sizeof(RI)) == V)
+        k_filter<V, R, RI, BATCH><<<g, NT, 0, st>>>(c.hC, c.attr, in, F, c.part, c.dS, seg, B);
+    else
+        k_filter<1, R, RI, BATCH><<<g, NT, 0, st>>>(c.hC, c.attr, in, F, c.part, c.dS, seg, B);
+}
+static inline size_t filter_blocks(const DevCtx& c) {
+    int seg;
+    const dim3 a = filter_grid(c, c.esz, seg), b = filter_grid(c, 8, seg);
+    const size_t na = (size_t)a.x * a.y, nb = (size_t)b.x * b.y;
+    return na > nb ? na : nb;
+}
+
+// The property, flow and scalar passes with the kernel instance of their tile's block size.
 template <typename R, bool BATCH>
-static inline void launch_strain(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
-                                 const F11<R>& F, const PropBuf<R>& P, const Batch& B) {
-    if (b.x * b.y * b.z == 512) k_strain<R, BATCH, 512><<<g, b, 0, st>>>(hC, attr, F, P, B);
-    else k_strain<R, BATCH><<<g, b, 0, st>>>(hC, attr, F, P, B);
+static inline void launch_props(const DevCtx& c, dim3 g, dim3 b, cudaStream_t st, const F11<R>& F, const PropBuf<R>& P,
+                                int keep, const Batch& B) {
+    if (b.x * b.y * b.z == 512) k_props<R, BATCH, 512><<<g, b, 0, st>>>(c.hC, c.attr, F, P, c.part, c.dS, keep, B);
+    else k_props<R, BATCH><<<g, b, 0, st>>>(c.hC, c.attr, F, P, c.part, c.dS, keep, B);
 }
 template <int PART, typename R, bool BATCH>
 static inline void launch_scalar_part(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
@@ -141,10 +174,9 @@ void step_tail(DevCtx& c, cudaStream_t st, bool device_mode) {
 template <typename R>
 cudaError_t step_impl(DevCtx& c, double dt, int t_loop, bool device_mode) {
     cudaStream_t st = c.stream;
-    if (!part_fits(c, cell_blocks(c, SH_FILTER), 3) || !part_fits(c, cell_blocks(c, SH_EOS), 1) ||
+    if (!part_fits(c, filter_blocks(c), 1) || !part_fits(c, cell_blocks(c, SH_STRAIN), 2) || !part_fits(c, cell_blocks(c, SH_EOS), 1) ||
         !part_fits(c, MON_BLOCKS, 6))
         return cudaErrorInvalidValue;
-    const dim3 gA = cell_grid(c, SH_FILTER), bA = cell_block(c, SH_FILTER);
     const dim3 gB = cell_grid(c, SH_STRAIN), bB = cell_block(c, SH_STRAIN);
     const dim3 gC = cell_grid(c, SH_FLOW), bC = cell_block(c, SH_FLOW);
     const dim3 gD = cell_grid(c, SH_SCALAR), bD = cell_block(c, SH_SCALAR);
@@ -178,11 +210,11 @@ cudaError_t step_impl(DevCtx& c, double dt, int t_loop, bool device_mode) {
     // four RK4 stages (:4428-4544)
     for (int s = 0; s < 4; s++) {
         tm = tmark_begin(c, 1);
-        if (s == 0) k_filter_props<R, RS><<<gA, bA, 0, st>>>(c.hC, c.attr, S, F, P, c.part, c.dS, 0, Batch{});
-        else k_filter_props<R, R><<<gA, bA, 0, st>>>(c.hC, c.attr, St, F, P, c.part, c.dS, s == 3 ? 1 : 0, Batch{});
+        if (s == 0) launch_filter<R, RS, false>(c, st, S, F, 1, Batch{});
+        else launch_filter<R, R, false>(c, st, St, F, 1, Batch{});
         tmark_end(c, tm);
         tm = tmark_begin(c, 2);
-        launch_strain<R, false>(gB, bB, st, c.hC, c.attr, F, P, Batch{});
+        launch_props<R, false>(c, gB, bB, st, F, P, s == 3 ? 1 : 0, Batch{});
         tmark_end(c, tm);
         // the k-arrays of the first stage are kept for inspection when requested
         const KDbg<R>& kds = (s == 0) ? kd : knone;
@@ -226,7 +258,7 @@ cudaError_t batch_tail(DevCtx& c) {
 
 template <typename R>
 cudaError_t batch_stages(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t st) {
-    if (nmem < 1 || !part_fits(c0, cell_blocks(c0, SH_FILTER), 3)) return cudaErrorInvalidValue;
+    if (nmem < 1 || !part_fits(c0, filter_blocks(c0), 1) || !part_fits(c0, cell_blocks(c0, SH_STRAIN), 2)) return cudaErrorInvalidValue;
     auto grid = [&](int cls, Batch& b) {
         dim3 g = cell_grid(c0, cls);
         b.mt = mt;
@@ -234,12 +266,11 @@ cudaError_t batch_stages(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t
         g.z *= (unsigned)nmem;
         return g;
     };
-    Batch BA, BB, BC, BD;
-    const dim3 gA = grid(SH_FILTER, BA), bA = cell_block(c0, SH_FILTER);
+    Batch BB, BC, BD;
     const dim3 gB = grid(SH_STRAIN, BB), bB = cell_block(c0, SH_STRAIN);
     const dim3 gC = grid(SH_FLOW, BC), bC = cell_block(c0, SH_FLOW);
     const dim3 gD = grid(SH_SCALAR, BD), bD = cell_block(c0, SH_SCALAR);
-    if (gA.z > 65535u || gB.z > 65535u || gC.z > 65535u || gD.z > 65535u) return cudaErrorInvalidConfiguration;
+    if (gB.z > 65535u || (unsigned)nmem * NSTATE > 65535u || gC.z > 65535u || gD.z > 65535u) return cudaErrorInvalidConfiguration;
     F11<RS> S = f11<RS>(c0.S);
     F11<R> St = f11<R>(c0.St), F = f11<R>(c0.F);
     PropBuf<R> P = props<R>(c0);
@@ -249,9 +280,9 @@ cudaError_t batch_stages(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t
     for (int q = 0; q < NACC; q++) knone.p[q] = nullptr;
     RS* rn = (RS*)c0.rn;
     for (int s = 0; s < 4; s++) {
-        if (s == 0) k_filter_props<R, RS, true><<<gA, bA, 0, st>>>(c0.hC, c0.attr, S, F, P, c0.part, c0.dS, 0, BA);
-        else k_filter_props<R, R, true><<<gA, bA, 0, st>>>(c0.hC, c0.attr, St, F, P, c0.part, c0.dS, s == 3 ? 1 : 0, BA);
-        launch_strain<R, true>(gB, bB, st, c0.hC, c0.attr, F, P, BB);
+        if (s == 0) launch_filter<R, RS, true>(c0, st, S, F, nmem, Batch{mt, 0});
+        else launch_filter<R, R, true>(c0, st, St, F, nmem, Batch{mt, 0});
+        launch_props<R, true>(c0, gB, bB, st, F, P, s == 3 ? 1 : 0, BB);
         launch_scalar<R, true>(gD, bD, st, c0.hC, c0.attr, F, P, S, St, acc, rn, knone, c0.dS, s, BD);
         launch_flow<R, true>(gC, bC, st, c0.hC, c0.attr, F, P, S, St, acc, rn, knone, c0.dS, s, BC);
     }
@@ -265,7 +296,7 @@ cudaError_t batch_stages(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t
 template <typename R>
 cudaError_t rhs_only_impl(DevCtx& c, int t_loop) {
     cudaStream_t st = c.stream;
-    if (!part_fits(c, cell_blocks(c, SH_FILTER), 3)) return cudaErrorInvalidValue;
+    if (!part_fits(c, filter_blocks(c), 1) || !part_fits(c, cell_blocks(c, SH_STRAIN), 2)) return cudaErrorInvalidValue;
     F11<RS> S = f11<RS>(c.S);
     F11<R> St = f11<R>(c.St), F = f11<R>(c.F);
     PropBuf<R> P = props<R>(c);
@@ -276,11 +307,10 @@ cudaError_t rhs_only_impl(DevCtx& c, int t_loop) {
     RS* rn = (RS*)c.rn;
     k_set_step<<<1, 1, 0, st>>>(c.dS, 0.0, t_loop);
     int tm = tmark_begin(c, 1);
-    k_filter_props<R, RS><<<cell_grid(c, SH_FILTER), cell_block(c, SH_FILTER), 0, st>>>(c.hC, c.attr, S, F, P,
-                                                                                       c.part, c.dS, 1, Batch{});
+    launch_filter<R, RS, false>(c, st, S, F, 1, Batch{});
     tmark_end(c, tm);
     tm = tmark_begin(c, 2);
-    launch_strain<R, false>(cell_grid(c, SH_STRAIN), cell_block(c, SH_STRAIN), st, c.hC, c.attr, F, P, Batch{});
+    launch_props<R, false>(c, cell_grid(c, SH_STRAIN), cell_block(c, SH_STRAIN), st, F, P, 1, Batch{});
     tmark_end(c, tm);
     tm = tmark_begin(c, 5);
     if (c.scalar_tma && c.tma_ok)

@@ -256,11 +256,11 @@ int lesgpu_eval_rhs(lesgpu_ctx* ctx, int t_loop);
  * totals (ms) and launch counts per class and resets them.  Classes: */
 enum {
     LESGPU_K_SEM = 0,        /* SEM inflow plane + normalisation */
-    LESGPU_K_FILTER = 1,     /* box filter + mixture properties (4 launches per step) */
-    LESGPU_K_STRAIN = 2,     /* strain, nu_t, S_T (4 per step) */
-    LESGPU_K_RHS_FLOW = 3,   /* momentum and G right-hand sides (4 per step) */
+    LESGPU_K_FILTER = 1,     /* box filter (4 launches per step) */
+    LESGPU_K_STRAIN = 2,     /* mixture properties, strain, nu_t, S_T (4 per step) */
+    LESGPU_K_RHS_FLOW = 3,   /* momentum and G right-hand sides + their RK4 update (4 per step) */
     LESGPU_K_BC = 4,         /* boundary faces + EOS/renormalisation */
-    LESGPU_K_RHS_SCALAR = 5, /* species/T right-hand sides + RK4 stage update (4 per step) */
+    LESGPU_K_RHS_SCALAR = 5, /* species/T right-hand sides + their RK4 update (4 per step) */
     LESGPU_NK = 6
 };
 int lesgpu_kernel_timing(lesgpu_ctx* ctx, int enable);
