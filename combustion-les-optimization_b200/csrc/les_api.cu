@@ -457,6 +457,7 @@ int lesgpu_create(const lesgpu_config* cfg, const lesgpu_species* sp, lesgpu_ctx
     if (e != cudaSuccess) { int r = cuda_fail(ctx, e, "cudaStreamCreate"); delete ctx; return r; }
     e = cudaStreamCreateWithFlags(&d.side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d.ev_fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d.ev_dt, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d.ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) { int r = cuda_fail(ctx, e, "side stream"); lesgpu_destroy(ctx); return r; }
     // one arena for all per-cell fields; each field starts on a 256-byte boundary.  The
@@ -551,6 +552,7 @@ void lesgpu_destroy(lesgpu_ctx* ctx) {
     free_loop(d);
     if (d.side) { cudaStreamSynchronize(d.side); cudaStreamDestroy(d.side); }
     if (d.ev_fork) cudaEventDestroy(d.ev_fork);
+    if (d.ev_dt) cudaEventDestroy(d.ev_dt);
     if (d.ev_join) cudaEventDestroy(d.ev_join);
     if (d.stream) cudaStreamDestroy(d.stream);
     delete ctx;
@@ -1546,7 +1548,7 @@ int lesgpu_group_create_batched(lesgpu_ctx* const* ctxs, int n, int max_per_batc
         for (int q = 0; q < n && el == cudaSuccess; q++) {
             DevCtx& d = ctxs[q]->d;
             el = cudaStreamWaitEvent(d.stream, g->fork, 0);
-            if (el == cudaSuccess) el = les::loop_pre(d);
+            if (el == cudaSuccess) el = les::loop_pre(d, d.stream);
             if (el == cudaSuccess) el = cudaEventRecord(g->heads[q], d.stream);
             if (el == cudaSuccess) el = les::sem_inflow(d, d.stream);
         }

@@ -218,10 +218,10 @@ __device__ __forceinline__ T* shifted(T* p, long long d) {
 // Reduction results written by the kernels' last-block epilogues.
 struct Scalars {
     double rho_avg;                     // <rho_f> of the current stage (:2550)
-    double umax, numax, alphamax;       // dt inputs (:1472-1485, :4401-4408)
+    double umax, numax, alphamax;       // dt inputs (:1472-1485, :4401-4408); max_into
     double mon[6];                      // monitor reductions
     double sem[6];                      // SEM sums (debug)
-    unsigned int counter[4];            // last-block counters (0: filter, 1: bc, 2: aux, 3: monitor)
+    unsigned int counter[4];            // last-block counters (0: filter, 1: loop end, 2: umax, 3: monitor)
     int nonfinite;                      // bit 1: rand() jump table too short (device loop)
     double dt;                          // dt of the step being computed
     double umax_used;                   // |u|max that produced dt (after the inlet fallback)
@@ -412,6 +412,21 @@ __device__ __forceinline__ double block_max(double v, double* sh, int tid) {
 template <int NT>
 __device__ __forceinline__ double block_min(double v, double* sh, int tid) {
     return -block_max<NT>(-v, sh, tid);
+}
+
+// *to = max(*to, v) over every thread that calls it, for values >= 0 (NaN and negative count as 0):
+// doubles of one sign order like their bits, so the maximum of the converged lanes is two 32-bit warp
+// reductions, and one lane raises the global value, without an atomic where it would not.
+__device__ __forceinline__ void max_into(double* to, double v) {
+    const double w = fmax(v, 0.0);
+    const unsigned mask = __activemask();
+    const unsigned hi = (unsigned)__double2hiint(w), top = __reduce_max_sync(mask, hi);
+    const unsigned low = __reduce_max_sync(mask, hi == top ? (unsigned)__double2loint(w) : 0u);
+    const unsigned lane = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+    if ((lane & 31u) == (unsigned)(__ffs((int)mask) - 1)) {
+        const unsigned long long m = ((unsigned long long)top << 32) | low;
+        if (m > *reinterpret_cast<volatile unsigned long long*>(to)) atomicMax(reinterpret_cast<unsigned long long*>(to), m);
+    }
 }
 
 }  // namespace les

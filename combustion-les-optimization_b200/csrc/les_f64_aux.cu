@@ -58,8 +58,8 @@ int selfcheck_division(const double* divisors, int nd, size_t n, unsigned long l
     return e == cudaSuccess ? 0 : -2;
 }
 
-cudaError_t loop_pre(DevCtx& c) {
-    k_loop_pre<<<1, LOOP_THREADS, 0, c.stream>>>(c.dC, c.dS, (LoopState*)c.dL, c.J, c.jrows, c.vort, c.nv, c.noise,
+cudaError_t loop_pre(DevCtx& c, cudaStream_t st) {
+    k_loop_pre<<<1, LOOP_THREADS, 0, st>>>(c.dC, c.dS, (LoopState*)c.dL, c.J, c.jrows, c.vort, c.nv, c.noise,
                                                  c.n_inlet, c.lp_lbox, c.lp_ly, c.lp_lz, c.lp_uin, c.lp_ti, c.lp_ell,
                                                  c.lp_cfl, c.lp_cfld, c.lp_dx);
     return cudaGetLastError();

@@ -178,6 +178,24 @@ __device__ __forceinline__ double eos_rho_state(const Consts& C, double T, const
     return fallback;
 }
 
+// Mass fractions brought to the sum 1 where it is above `least` (:4447, :3152): one reciprocal, the
+// quotients sharing it corrected with one fma each.
+template <typename Form>
+__device__ __forceinline__ bool renormalise(double* Y, double least) {
+    double sy = 0.0;
+#pragma unroll
+    for (int s = 0; s < NSP; s++) sy += Y[s];
+    if (!(sy > least)) return false;
+    const double y = sdiv<Form>(1.0, sy);
+#pragma unroll
+    for (int s = 0; s < NSP; s++) Y[s] = cquot(Y[s], sy, y);
+    return true;
+}
+
+__device__ __forceinline__ bool off_faces(const Consts& C, int i, int j, int k) {
+    return i >= 1 && i < C.nx - 1 && j >= 1 && j < C.ny - 1 && k >= 1 && k < C.nz - 1;
+}
+
 // What the properties of a cell are kept in.
 template <typename R>
 struct CellProps {
@@ -637,10 +655,9 @@ __global__ void __launch_bounds__(NT)
 // next dt are taken (:4401-4408).
 template <typename R, bool BATCH = false, int NTB = NT>
 __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
-    k_props(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, double* __restrict__ part,
-            Scalars* __restrict__ S, int keep, Batch B) {
+    k_props(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, Scalars* __restrict__ S,
+            int keep, Batch B) {
     const auto& K = kc<R>(C);
-    __shared__ double sh[NTB / 32];
     __shared__ double tab[EXP_STEPS];
     int bz = blockIdx.z;
     ModelK<R> M;
@@ -651,7 +668,6 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
         shift_all(F, e.delta);
         shift_props(P, e.delta);
         attr = e.attr;
-        part = e.part;
         S = e.S;
         M = member_model<R>(e);
     } else {
@@ -666,7 +682,6 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
         if (tid < EXP_STEPS) tab[tid] = C.exp_tab[tid];
         __syncthreads();
     }
-    double mnu = 0.0, mal = 0.0;
     const bool here = k < nz && j < ny && i < nx;
     const int id = here ? (int)cid(i, j, k, ny, nz) : 0;
     const bool interior = here && i >= 1 && i < nx - 1 && j >= 1 && j < ny - 1 && k >= 1 && k < nz - 1;
@@ -715,8 +730,6 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
             store_d(g.D);
             o = g;
         }
-        mnu = (double)o.nu;
-        mal = (double)o.alpha;
         P.aT[id] = o.aT;
         P.nu_t[id] = nut;
         P.mu_eff[id] = interior ? fma(rho, nut, o.mu_mix) : R(0);
@@ -724,6 +737,8 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
             P.mu_mix[id] = o.mu_mix;
             P.nu[id] = o.nu;
             P.S_mag[id] = Smag;
+            max_into(&S->numax, (double)o.nu);
+            max_into(&S->alphamax, (double)o.alpha);
         }
         if (P.dbg_cp) { P.dbg_cp[id] = o.cp; P.dbg_lam[id] = o.lam; P.dbg_alpha[id] = o.alpha; }
         R ST = R(0);
@@ -766,27 +781,6 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
             for (int s = 0; s < NSP; s++) P.D[s][id] = R(0);
             P.aT[id] = R(0);
             P.dbg_cp[id] = R(1000.0); P.dbg_lam[id] = R(0); P.dbg_alpha[id] = R(0);
-        }
-    }
-    if (!keep) return;
-    const unsigned nblk = gridDim.x * gridDim.y * (BATCH ? (unsigned)B.gz : gridDim.z);
-    const unsigned bid = ((unsigned)bz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    double v[2];
-    v[0] = block_max<NTB>(mnu, sh, tid);
-    v[1] = block_max<NTB>(mal, sh, tid);
-    if (last_block(part, nblk, bid, v, 2, &S->counter[2], tid)) {
-        double mn = 0.0, ma = 0.0;
-#pragma unroll 8
-        for (unsigned q = tid; q < nblk; q += NTB) {
-            mn = fmax(mn, __ldcg(&part[q]));
-            ma = fmax(ma, __ldcg(&part[nblk + q]));
-        }
-        mn = block_max<NTB>(mn, sh, tid);
-        ma = block_max<NTB>(ma, sh, tid);
-        if (tid == 0) {
-            S->numax = mn;
-            S->alphamax = ma;
-            S->counter[2] = 0u;
         }
     }
 }
@@ -946,12 +940,16 @@ struct GSrc {
 // The RK stages as the scalar pass sees them: the first starts the running sum, the last ends it.
 enum { RK_FIRST = 0, RK_MIDDLE = 1, RK_LAST = 2 };
 
+// The dt inputs of the step have been read by now (the first stage's update has used dt), and the
+// last stage's property and flow passes take them anew.
+__device__ __forceinline__ void reset_maxima(Scalars* Sc) { Sc->umax = Sc->numax = Sc->alphamax = 0.0; }
+
 // One cell of the scalar pass (the body shared by both read paths).
 template <int PART, typename R, typename RS, typename Src>
 __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* __restrict__ attr, const F11<R>& F,
                                                 const PropBuf<R>& P, const F11<RS>& S0, const F11<R>& St,
                                                 const AccBuf<R>& acc, RS* __restrict__ rn, const KDbg<R>& kd,
-                                                const Scalars* __restrict__ Sc, int stage, int i, int j, int k,
+                                                Scalars* __restrict__ Sc, int stage, int i, int j, int k,
                                                 Src& src, const R relax) {
     const auto& K = kc<R>(C);
     const int nx = C.nx, ny = C.ny, nz = C.nz;
@@ -961,6 +959,8 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
         // non-fluid cells: the temp state is Phi_n (:4444, :4454); rho_temp is only ever written on
         // outlet/fluid cells (:1893), so it stays 0 on inlet/wall/symmetry cells.  These values
         // are the same for all stages of a step.
+        // Cells of the boundary faces get their final values in k_bc; the last stage brings any
+        // other cell that is not fluid to what the reference's EOS sweep (:3130-3160) leaves there.
         RS Y0[NSP];
         const RS T0 = S0.p[3][id], r0 = S0.p[5][id];
 #pragma unroll
@@ -971,8 +971,12 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
 #pragma unroll
             for (int s = 0; s < NSP; s++) St.p[6 + s][id] = R(Y0[s]);
             if (a == 2) St.p[5][id] = R(r);
-        } else if (PART == RK_LAST && a == 2) {
-            rn[id] = eos_rho_state<R>(C, T0, Y0, r0);
+        } else if (PART == RK_LAST && off_faces(C, i, j, k)) {
+            rn[id] = eos_rho_state<R>(C, T0, Y0, RS(1.2));
+            if ((a == 2 || a == 5) && renormalise<R>(Y0, RS(1e-6))) {
+#pragma unroll
+                for (int s = 0; s < NSP; s++) S0.p[6 + s][id] = Y0[s];
+            }
         }
         if (kd.p[0]) {
 #pragma unroll
@@ -1042,22 +1046,22 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
     // FP32 and Phi_n, the stage update and the final combine FP64, so increments far below
     // the state's FP32 ulp are not rounded away step after step.
     const RS cdt = PART == RK_LAST ? (RS)(dt / 6.0) : (RS)((PART == RK_MIDDLE && stage == 2 ? 1.0 : 0.5) * dt);
-    RS up[1 + NSP], sy = RS(0);
+    RS up[1 + NSP];
 #pragma unroll
     for (int q = 0; q < 1 + NSP; q++) {
         const R incr = PART == RK_LAST ? ac[q] + kv[q] : kv[q];
         ac[q] = PART == RK_FIRST ? kv[q] : fma(R(2.0), kv[q], ac[q]);
         up[q] = fma(cdt, (RS)incr, sn[q]);
         up[q] = q == 0 ? fmax(RS(200.0), fmin(RS(3000.0), up[q])) : fmax(RS(0.0), fmin(RS(1.0), up[q]));
-        if (q > 0) sy += up[q];
     }
-    // one reciprocal, the quotients sharing it corrected with one fma each
-    if (sy > RS(SMALL)) {
-        const RS y = sdiv<R>(RS(1.0), sy);
-#pragma unroll
-        for (int s = 1; s < 1 + NSP; s++) up[s] = cquot(up[s], sy, y);
+    renormalise<R>(up + 1, RS(SMALL));
+    RS rho = eos_rho_state<R>(C, up[0], up + 1, PART == RK_LAST ? RS(0.0) : rho_n);
+    if (PART == RK_LAST) {
+        // the EOS sweep after the boundary conditions (:3130-3160) finds this density again (and 1.2
+        // where there is none, which a negative sign tells the flow pass) and renormalises once more
+        if (rho == RS(0.0)) rho = -fabs(rho_n);
+        renormalise<R>(up + 1, RS(1e-6));
     }
-    const RS rho = eos_rho_state<R>(C, up[0], up + 1, rho_n);
     if (kd.p[0]) {
 #pragma unroll
         for (int q = 0; q < 1 + NSP; q++) kd.p[q == 0 ? 3 : 4 + q][id] = kv[q];
@@ -1078,7 +1082,7 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
 template <int PART, typename R, typename RS = R, bool BATCH = false, int NTB = NT>
 __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
     k_rhs_scalar(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, F11<RS> S0, F11<R> St,
-                 AccBuf<R> acc, RS* __restrict__ rn, KDbg<R> kd, const Scalars* __restrict__ Sc, int stage, Batch B) {
+                 AccBuf<R> acc, RS* __restrict__ rn, KDbg<R> kd, Scalars* __restrict__ Sc, int stage, Batch B) {
     int bz = blockIdx.z;
     R relax;
     if constexpr (BATCH) {
@@ -1105,6 +1109,7 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
     const int i = bz * blockDim.z + threadIdx.z;
     if (k >= nz || j >= ny || i >= C.nx) return;
     const size_t id = cid(i, j, k, ny, nz);
+    if (PART == RK_MIDDLE && id == 0) reset_maxima(Sc);
     GSrc<R> src;
     src.id = (int)id;
     src.s[0] = ny * nz;
@@ -1129,7 +1134,7 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
 template <int PART, typename R, typename RS = R, bool BATCH = false, int NTB = NT>
 __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
     k_rhs_flow(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, F11<RS> S0, F11<R> St,
-               AccBuf<R> acc, RS* __restrict__ rn, KDbg<R> kd, const Scalars* __restrict__ Sc, int stage, Batch B) {
+               AccBuf<R> acc, RS* __restrict__ rn, KDbg<R> kd, Scalars* __restrict__ Sc, int stage, Batch B) {
     const auto& K = kc<R>(C);
     int bz = blockIdx.z;
     ModelK<R> M;
@@ -1159,14 +1164,16 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
     const int id = (int)cid(i, j, k, ny, nz);
     const int a = attr[id];
     if (a != 3) {
-        // as in the scalar pass: the stage state of other cells is Phi_n, and only outlet cells
-        // get a new density
+        // as in the scalar pass: the stage state of other cells is Phi_n, and the last stage leaves
+        // cells off the faces as the EOS sweep does
         if (PART == RK_FIRST) {
 #pragma unroll
             for (int q = 0; q < 5; q++)
                 if (q != 3) St.p[q][id] = R(S0.p[q][id]);
-        } else if (PART == RK_LAST && a == 2) {
+        } else if (PART == RK_LAST && off_faces(C, i, j, k)) {
             S0.p[5][id] = rn[id];
+            const RS u = S0.p[0][id], v = S0.p[1][id], w = S0.p[2][id];
+            if (a == 1) max_into(&Sc->umax, sqrt(u * u + v * v + w * w));
         }
         return;
     }
@@ -1277,7 +1284,8 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
         sn[q] = ld_stream(S0.p[qa[q]] + id);
         ac[q] = PART != RK_FIRST ? ld_stream(acc.p[qa[q]] + id) : R(0);
     }
-    const RS rho_n = ld_stream(S0.p[5] + id), rho = ld_stream(rn + id);
+    const RS rho_n = ld_stream(S0.p[5] + id), left = ld_stream(rn + id);
+    const RS rho = PART == RK_LAST ? fabs(left) : left;
     const double dt = Sc->dt;
     const RS cdt = PART == RK_LAST ? (RS)(dt / 6.0) : (RS)((PART == RK_MIDDLE && stage == 2 ? 1.0 : 0.5) * dt);
     const RS irho = sdiv<R>(RS(1.0), rho);
@@ -1306,19 +1314,29 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
             S0.p[qa[q]][id] = out[q];
         }
     }
-    if (PART == RK_LAST) S0.p[5][id] = rho;
+    if (PART == RK_LAST) {
+        S0.p[5][id] = left < RS(0.0) ? RS(1.2) : left;
+        // |u| of the next dt (:1472-1485)
+        max_into(&Sc->umax, sqrt(out[0] * out[0] + out[1] * out[1] + out[2] * out[2]));
+    }
 }
 
 // ------------------------------------------------------------------ boundary conditions
-// apply_boundary_conditions (:2967-3161) in its face order: i-faces (with the SEM +
-// white-noise inflow), then for every interior i the j-faces, then the k-faces, then the
-// equation of state and mass-fraction renormalisation everywhere.
+// apply_boundary_conditions (:2967-3161): the i-faces (with the SEM + white-noise inflow), then for
+// every interior i the j-faces, then the k-faces, then the equation of state and mass-fraction
+// renormalisation.  Only the cells of the six faces change: the last stage's scalar and flow passes
+// leave every other cell as the reference's EOS sweep over the grid does, and take the maximum
+// of |u| over fluid cells, so no pass over the whole grid is needed here.
 
 template <typename R>
 __device__ __forceinline__ void copy_cell(F11<R>& S, size_t dst, size_t src) {
+    R v[NSTATE];
 #pragma unroll
     for (int q = 0; q < NSTATE; q++)
-        if (q != 5) S.p[q][dst] = S.p[q][src];
+        if (q != 5) v[q] = S.p[q][src];
+#pragma unroll
+    for (int q = 0; q < NSTATE; q++)
+        if (q != 5) S.p[q][dst] = v[q];
 }
 template <typename R>
 __device__ __forceinline__ void ambient_cell(const Consts& C, F11<R>& S, size_t dst) {
@@ -1329,15 +1347,13 @@ __device__ __forceinline__ void ambient_cell(const Consts& C, F11<R>& S, size_t 
     for (int s = 0; s < NSP; s++) S.p[6 + s][dst] = (R)K.ambientYk[s];
 }
 
-template <typename R, typename Form = R>
-__global__ void k_bc_iface(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> S,
-                           const double* __restrict__ plane, const double* __restrict__ noise,
-                           const int* __restrict__ inlet_pos) {
+// The cell (0, j, k): inflow, open face or rim; the cell (nx-1, j, k): outlet.
+template <typename R>
+__device__ __forceinline__ void bc_first_plane(const Consts& C, const uint8_t* __restrict__ attr, F11<R>& S,
+                                               const double* __restrict__ plane, const double* __restrict__ noise,
+                                               const int* __restrict__ inlet_pos, int j, int k) {
     const auto& K = kc<R>(C);
-    const int nx = C.nx, ny = C.ny, nz = C.nz;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y;
-    if (k >= nz) return;
+    const int ny = C.ny, nz = C.nz;
     const size_t i0 = cid(0, j, k, ny, nz), i1 = cid(1, j, k, ny, nz);
     const int a0 = attr[i0];
     if (a0 == 1) {
@@ -1357,112 +1373,109 @@ __global__ void k_bc_iface(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, 
         if (S.p[0][i1] < R(0)) ambient_cell<R>(C, S, i0);
         else copy_cell<R>(S, i0, i1);
     } else if (a0 == 6) {
+        copy_cell<R>(S, i0, i1);
         S.p[0][i0] = R(0); S.p[1][i0] = R(0); S.p[2][i0] = R(0);
-        S.p[3][i0] = S.p[3][i1];
-        S.p[4][i0] = S.p[4][i1];
-#pragma unroll
-        for (int s = 0; s < NSP; s++) S.p[6 + s][i0] = S.p[6 + s][i1];
     }
-    const size_t in = cid(nx - 1, j, k, ny, nz), im = cid(nx - 2, j, k, ny, nz);
+}
+template <typename R>
+__device__ __forceinline__ void bc_last_plane(const Consts& C, const uint8_t* __restrict__ attr, F11<R>& S, int j, int k) {
+    const size_t in = cid(C.nx - 1, j, k, C.ny, C.nz), im = cid(C.nx - 2, j, k, C.ny, C.nz);
     if (attr[in] == 2) copy_cell<R>(S, in, im);
 }
 
-template <typename R, typename Form = R>
-__global__ void k_bc_jface(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> S) {
-    const int ny = C.ny, nz = C.nz;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y + 1;
-    if (k >= nz) return;
-    const size_t b = cid(i, 0, k, ny, nz), n1 = cid(i, 1, k, ny, nz);
-    if (attr[b] == 5) {
-        S.p[3][b] = S.p[3][n1];
-        S.p[4][b] = S.p[4][n1];
+// EOS + renormalisation (:3130-3160) of one cell, and |u| of an inlet or fluid cell for the next
+// dt (:1472-1485).
+template <typename R, typename Form>
+__device__ __forceinline__ void bc_eos_cell(const Consts& C, const uint8_t* __restrict__ attr, F11<R>& S, size_t id,
+                                            Scalars* __restrict__ Sc) {
+    const int a = attr[id];
+    R Y[NSP];
 #pragma unroll
-        for (int s = 0; s < NSP; s++) S.p[6 + s][b] = S.p[6 + s][n1];
-        S.p[0][b] = S.p[0][n1];
-        S.p[1][b] = R(0.0);
-        S.p[2][b] = S.p[2][n1];
+    for (int s = 0; s < NSP; s++) Y[s] = S.p[6 + s][id];
+    const R T = S.p[3][id], u = S.p[0][id], v = S.p[1][id], w = S.p[2][id];
+    S.p[5][id] = eos_rho_state<Form>(C, T, Y, R(1.2));
+    if ((a == 3 || a == 2 || a == 5) && renormalise<Form>(Y, R(1e-6))) {
+#pragma unroll
+        for (int s = 0; s < NSP; s++) S.p[6 + s][id] = Y[s];
     }
-    const size_t t = cid(i, ny - 1, k, ny, nz), tm = cid(i, ny - 2, k, ny, nz);
-    if (attr[t] == 4) {
-        if (S.p[1][tm] < R(0)) ambient_cell<R>(C, S, t);
-        else copy_cell<R>(S, t, tm);
+    if (a == 1 || a == 3) max_into(&Sc->umax, sqrt(u * u + v * v + w * w));
+}
+
+// The q-th of the 2 (ny + nz) - 4 cells around a plane.
+__device__ __forceinline__ void ring_cell(int q, int ny, int nz, int& j, int& k) {
+    if (q < 2 * nz) {
+        j = q < nz ? 0 : ny - 1;
+        k = q < nz ? q : q - nz;
+    } else {
+        q -= 2 * nz;
+        j = 1 + (q >> 1);
+        k = (q & 1) ? nz - 1 : 0;
     }
 }
 
+// One launch for all of it.  Block b < nx - 2 takes the faces around plane i = b + 1 in the
+// reference's order, its own barriers between the steps; the blocks of the second and the last
+// but one plane also take the cells around planes 0 and nx - 1 first, which copy cells that the
+// j- and k-faces then overwrite.  The remaining blocks take the inner cells of planes 0 and
+// nx - 1, which copy cells that nothing here writes.
 template <typename R, typename Form = R>
-__global__ void k_bc_kface(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> S) {
-    const int ny = C.ny, nz = C.nz;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y + 1;
-    if (j >= ny) return;
-    const size_t b = cid(i, j, 0, ny, nz), n1 = cid(i, j, 1, ny, nz);
-    if (attr[b] == 4) {
-        if (S.p[2][n1] > R(0)) ambient_cell<R>(C, S, b);
-        else copy_cell<R>(S, b, n1);
+__global__ void __launch_bounds__(NT) k_bc(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> S,
+                                           const double* __restrict__ plane, const double* __restrict__ noise,
+                                           const int* __restrict__ inlet_pos, Scalars* __restrict__ Sc) {
+    const int nx = C.nx, ny = C.ny, nz = C.nz, tid = threadIdx.x;
+    const int ring = 2 * (ny + nz) - 4;
+    int j, k;
+    if ((int)blockIdx.x >= nx - 2) {
+        const int q = ((int)blockIdx.x - (nx - 2)) * NT + tid;
+        if (q >= (ny - 2) * (nz - 2)) return;
+        j = 1 + q / (nz - 2);
+        k = 1 + q % (nz - 2);
+        bc_first_plane<R>(C, attr, S, plane, noise, inlet_pos, j, k);
+        bc_last_plane<R>(C, attr, S, j, k);
+        bc_eos_cell<R, Form>(C, attr, S, cid(0, j, k, ny, nz), Sc);
+        bc_eos_cell<R, Form>(C, attr, S, cid(nx - 1, j, k, ny, nz), Sc);
+        return;
     }
-    const size_t t = cid(i, j, nz - 1, ny, nz), tm = cid(i, j, nz - 2, ny, nz);
-    if (attr[t] == 4) {
-        if (S.p[2][tm] < R(0)) ambient_cell<R>(C, S, t);
-        else copy_cell<R>(S, t, tm);
-    }
-}
-
-// EOS + renormalisation everywhere (:3130-3160) fused with the max-velocity reduction
-// over inlet/fluid cells for the next dt (:1472-1485).
-template <typename R, typename Form = R>
-__global__ void __launch_bounds__(NT) k_bc_eos(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> S,
-                                               double* __restrict__ part, Scalars* __restrict__ Sc) {
-    const auto& K = kc<R>(C);
-    __shared__ double sh[NT / 32];
-    __shared__ bool last;
-    const int ny = C.ny, nz = C.nz;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i = blockIdx.z * blockDim.z + threadIdx.z;
-    const int tid = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
-    double vmax = 0.0;
-    if (k < nz && j < ny && i < C.nx) {
-        const size_t id = cid(i, j, k, ny, nz);
-        const int a = attr[id];
-        R Y[NSP];
-#pragma unroll
-        for (int s = 0; s < NSP; s++) Y[s] = S.p[6 + s][id];
-        const R T = S.p[3][id];
-        const R u = S.p[0][id], v = S.p[1][id], w = S.p[2][id];
-        S.p[5][id] = eos_rho_state<Form>(C, T, Y, R(1.2));
-        if (a == 3 || a == 2 || a == 5) {
-            R sy = R(0);
-#pragma unroll
-            for (int s = 0; s < NSP; s++) sy += Y[s];
-            if (sy > R(1e-6)) {
-                const R y = sdiv<Form>(R(1.0), sy);
-#pragma unroll
-                for (int s = 0; s < NSP; s++) S.p[6 + s][id] = cquot(Y[s], sy, y);
-            }
+    const int i = (int)blockIdx.x + 1;
+    if (i == 1 || i == nx - 2) {
+        for (int q = tid; q < ring; q += NT) {
+            ring_cell(q, ny, nz, j, k);
+            if (i == 1) bc_first_plane<R>(C, attr, S, plane, noise, inlet_pos, j, k);
+            else bc_last_plane<R>(C, attr, S, j, k);
         }
-        if (a == 1 || a == 3) vmax = (double)sqrt(u * u + v * v + w * w);
+        __syncthreads();
     }
-    const unsigned nblk = gridDim.x * gridDim.y * gridDim.z;
-    const unsigned bid = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    double bm = block_max<NT>(vmax, sh, tid);
-    if (tid == 0) {
-        part[bid] = bm;
-        __threadfence();
-        unsigned t = atomicAdd(&Sc->counter[1], 1u);
-        last = (t == nblk - 1);
+    for (k = tid; k < nz; k += NT) {
+        const size_t b = cid(i, 0, k, ny, nz), n1 = cid(i, 1, k, ny, nz);
+        if (attr[b] == 5) {
+            copy_cell<R>(S, b, n1);
+            S.p[1][b] = R(0.0);
+        }
+        const size_t t = cid(i, ny - 1, k, ny, nz), tm = cid(i, ny - 2, k, ny, nz);
+        if (attr[t] == 4) {
+            if (S.p[1][tm] < R(0)) ambient_cell<R>(C, S, t);
+            else copy_cell<R>(S, t, tm);
+        }
     }
     __syncthreads();
-    if (last) {
-        __threadfence();
-        double m = 0.0;
-#pragma unroll 8
-        for (unsigned q = tid; q < nblk; q += NT) m = fmax(m, __ldcg(&part[q]));
-        m = block_max<NT>(m, sh, tid);
-        if (tid == 0) {
-            Sc->umax = m;
-            Sc->counter[1] = 0u;
+    for (j = tid; j < ny; j += NT) {
+        const size_t b = cid(i, j, 0, ny, nz), n1 = cid(i, j, 1, ny, nz);
+        if (attr[b] == 4) {
+            if (S.p[2][n1] > R(0)) ambient_cell<R>(C, S, b);
+            else copy_cell<R>(S, b, n1);
         }
+        const size_t t = cid(i, j, nz - 1, ny, nz), tm = cid(i, j, nz - 2, ny, nz);
+        if (attr[t] == 4) {
+            if (S.p[2][tm] < R(0)) ambient_cell<R>(C, S, t);
+            else copy_cell<R>(S, t, tm);
+        }
+    }
+    __syncthreads();
+    for (int q = tid; q < ring; q += NT) {
+        ring_cell(q, ny, nz, j, k);
+        bc_eos_cell<R, Form>(C, attr, S, cid(i, j, k, ny, nz), Sc);
+        if (i == 1) bc_eos_cell<R, Form>(C, attr, S, cid(0, j, k, ny, nz), Sc);
+        if (i == nx - 2) bc_eos_cell<R, Form>(C, attr, S, cid(nx - 1, j, k, ny, nz), Sc);
     }
 }
 
@@ -1589,69 +1602,53 @@ static __global__ void k_set_step(Scalars* __restrict__ Sc, double dt, int t_loo
     Sc->t_loop = t_loop;
 }
 
-// Device loop, after the boundary conditions: the probe lines of record_flame_region_data
-// (:3403-3471) and dt/|u|max of this step go to history slot run_step.
+// Device loop, last launch of a step: the probe lines of record_flame_region_data (:3403-3471)
+// and dt/|u|max of this step go to history slot run_step, on steps with t_loop % 10 == 0 the
+// monitor reductions (:3874-3918) too (other slots are left untouched), and the last block to
+// finish advances the step counters.
 template <typename RS, typename R = RS>
-__global__ void k_loop_post(LES_KERNEL_CONSTS, F11<RS> S, PropBuf<R> P, const Scalars* __restrict__ Sc,
-                            const int* __restrict__ st, int n, int kline, int cap, double* __restrict__ hprobe,
-                            double* __restrict__ hdt, double* __restrict__ humax) {
-    const int ny = C.ny, nz = C.nz;
-    const int slot = Sc->run_step;
-    if (slot < 0 || slot >= cap) return;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int q = blockIdx.y;
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
-        hdt[slot] = Sc->dt;
-        humax[slot] = Sc->umax_used;
-    }
-    if (j >= ny || q >= n) return;
-    const size_t id = cid(st[q], j, kline, ny, nz);
-    double* o = hprobe + (((size_t)slot * n + q) * ny + j) * 6;
-    o[0] = (double)S.p[0][id];
-    o[1] = (double)S.p[1][id];
-    o[2] = (double)S.p[2][id];
-    o[3] = (double)S.p[4][id];
-    o[4] = (double)P.nu_t[id];
-    o[5] = (double)P.S_mag[id];
-}
-
-// Device loop: the monitor reductions (:3874-3918) on steps with t_loop % 10 == 0, written
-// to history slot run_step (other slots are left untouched).
-template <typename R, typename Form = R>
-__global__ void __launch_bounds__(NT) k_loop_monitor(LES_KERNEL_CONSTS, F11<R> S, double* __restrict__ part,
-                                                     Scalars* __restrict__ Sc, size_t n, int cap,
-                                                     double* __restrict__ hmon) {
+__global__ void __launch_bounds__(NT)
+    k_loop_end(LES_KERNEL_CONSTS, F11<RS> S, PropBuf<R> P, double* __restrict__ part, Scalars* __restrict__ Sc,
+               const int* __restrict__ st, int nst, int kline, size_t n, int cap, double* __restrict__ hprobe,
+               double* __restrict__ hdt, double* __restrict__ humax, double* __restrict__ hmon) {
     __shared__ double sh[NT / 32];
-    __shared__ bool last;
-    if (Sc->t_loop % 10 != 0) return;          // uniform across the grid
+    const int ny = C.ny, nz = C.nz, tid = threadIdx.x;
     const int slot = Sc->run_step;
-    if (slot < 0 || slot >= cap) return;
-    const int tid = threadIdx.x;
-    double mass = 0.0, tmin = 1.0e9, tmax = -1.0e9, gmin = 1.0e9, gmax = -1.0e9, ymin = 1.0e9;
-    for (size_t id = (size_t)blockIdx.x * NT + tid; id < n; id += (size_t)gridDim.x * NT) {
-        double r = (double)S.p[5][id], T = (double)S.p[3][id], G = (double)S.p[4][id], Y = (double)S.p[6][id];
-        mass += ((r * C.dx) * C.dy) * C.dz;
-        tmin = fmin(tmin, T); tmax = fmax(tmax, T);
-        gmin = fmin(gmin, G); gmax = fmax(gmax, G);
-        ymin = fmin(ymin, Y);
-    }
+    const bool monitor = Sc->t_loop % 10 == 0;          // uniform across the grid
     const unsigned nblk = gridDim.x;
     double v[6];
-    v[0] = block_sum<NT>(mass, sh, tid);
-    v[1] = block_min<NT>(tmin, sh, tid);
-    v[2] = block_max<NT>(tmax, sh, tid);
-    v[3] = block_min<NT>(gmin, sh, tid);
-    v[4] = block_max<NT>(gmax, sh, tid);
-    v[5] = block_min<NT>(ymin, sh, tid);
-    if (tid == 0) {
-        for (int q = 0; q < 6; q++) part[q * nblk + blockIdx.x] = v[q];
-        __threadfence();
-        unsigned t = atomicAdd(&Sc->counter[3], 1u);
-        last = (t == nblk - 1);
+    if (slot >= 0 && slot < cap) {
+        if (blockIdx.x == 0 && tid == 0) {
+            hdt[slot] = Sc->dt;
+            humax[slot] = Sc->umax_used;
+        }
+        for (int r = (int)blockIdx.x * NT + tid; r < nst * ny; r += (int)nblk * NT) {
+            const int q = r / ny, j = r - q * ny;
+            const size_t id = cid(st[q], j, kline, ny, nz);
+            double* o = hprobe + (((size_t)slot * nst + q) * ny + j) * 6;
+            const double a0 = (double)S.p[0][id], a1 = (double)S.p[1][id], a2 = (double)S.p[2][id],
+                         a3 = (double)S.p[4][id], a4 = (double)P.nu_t[id], a5 = (double)P.S_mag[id];
+            o[0] = a0; o[1] = a1; o[2] = a2; o[3] = a3; o[4] = a4; o[5] = a5;
+        }
+        if (monitor) {
+            double mass = 0.0, tmin = 1.0e9, tmax = -1.0e9, gmin = 1.0e9, gmax = -1.0e9, ymin = 1.0e9;
+            for (size_t id = (size_t)blockIdx.x * NT + tid; id < n; id += (size_t)nblk * NT) {
+                double r = (double)S.p[5][id], T = (double)S.p[3][id], G = (double)S.p[4][id], Y = (double)S.p[6][id];
+                mass += ((r * C.dx) * C.dy) * C.dz;
+                tmin = fmin(tmin, T); tmax = fmax(tmax, T);
+                gmin = fmin(gmin, G); gmax = fmax(gmax, G);
+                ymin = fmin(ymin, Y);
+            }
+            v[0] = block_sum<NT>(mass, sh, tid);
+            v[1] = block_min<NT>(tmin, sh, tid);
+            v[2] = block_max<NT>(tmax, sh, tid);
+            v[3] = block_min<NT>(gmin, sh, tid);
+            v[4] = block_max<NT>(gmax, sh, tid);
+            v[5] = block_min<NT>(ymin, sh, tid);
+        }
     }
-    __syncthreads();
-    if (last) {
-        __threadfence();
+    if (!last_block(part, nblk, blockIdx.x, v, monitor && slot >= 0 && slot < cap ? 6 : 0, &Sc->counter[1], tid)) return;
+    if (monitor && slot >= 0 && slot < cap) {
         double acc[6] = {0.0, 1.0e9, -1.0e9, 1.0e9, -1.0e9, 1.0e9};
 #pragma unroll 4
         for (unsigned q = tid; q < nblk; q += NT) {
@@ -1668,10 +1665,13 @@ __global__ void __launch_bounds__(NT) k_loop_monitor(LES_KERNEL_CONSTS, F11<R> S
         acc[3] = block_min<NT>(acc[3], sh, tid);
         acc[4] = block_max<NT>(acc[4], sh, tid);
         acc[5] = block_min<NT>(acc[5], sh, tid);
-        if (tid == 0) {
+        if (tid == 0)
             for (int q = 0; q < 6; q++) hmon[(size_t)slot * 6 + q] = acc[q];
-            Sc->counter[3] = 0u;
-        }
+    }
+    if (tid == 0) {
+        Sc->counter[1] = 0u;
+        Sc->t_loop += 1;
+        Sc->run_step += 1;
     }
 }
 
@@ -1695,12 +1695,6 @@ __global__ void __launch_bounds__(NT) k_time_avg(F11<RS> S, AvgBuf A, Scalars* _
         A.p[8][id] += v * w;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) Sc->avg_steps += 1;
-}
-
-// Device loop, last launch of a step: advance the step counters.
-static __global__ void k_loop_tick(Scalars* __restrict__ Sc) {
-    Sc->t_loop += 1;
-    Sc->run_step += 1;
 }
 
 template <typename R, typename Form = R>

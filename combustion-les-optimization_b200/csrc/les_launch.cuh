@@ -83,8 +83,8 @@ static inline size_t filter_blocks(const DevCtx& c) {
 template <typename R, bool BATCH>
 static inline void launch_props(const DevCtx& c, dim3 g, dim3 b, cudaStream_t st, const F11<R>& F, const PropBuf<R>& P,
                                 int keep, const Batch& B) {
-    if (b.x * b.y * b.z == 512) k_props<R, BATCH, 512><<<g, b, 0, st>>>(c.hC, c.attr, F, P, c.part, c.dS, keep, B);
-    else k_props<R, BATCH><<<g, b, 0, st>>>(c.hC, c.attr, F, P, c.part, c.dS, keep, B);
+    if (b.x * b.y * b.z == 512) k_props<R, BATCH, 512><<<g, b, 0, st>>>(c.hC, c.attr, F, P, c.dS, keep, B);
+    else k_props<R, BATCH><<<g, b, 0, st>>>(c.hC, c.attr, F, P, c.dS, keep, B);
 }
 template <int PART, typename R, bool BATCH>
 static inline void launch_scalar_part(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
@@ -142,29 +142,16 @@ template <typename R>
 void step_tail(DevCtx& c, cudaStream_t st, bool device_mode) {
     F11<RS> S = f11<RS>(c.S);
     PropBuf<R> P = props<R>(c);
-    const dim3 gE = cell_grid(c, SH_EOS), bE = cell_block(c, SH_EOS);
-    {
-        const int tpb = 128;
-        k_bc_iface<RS, R><<<dim3((c.nz + tpb - 1) / tpb, c.ny), tpb, 0, st>>>(c.hC, c.attr, S, c.plane, c.noise,
-                                                                                c.inlet_pos);
-        if (c.nx > 2) {
-            k_bc_jface<RS, R><<<dim3((c.nz + tpb - 1) / tpb, c.nx - 2), tpb, 0, st>>>(c.hC, c.attr, S);
-            k_bc_kface<RS, R><<<dim3((c.ny + tpb - 1) / tpb, c.nx - 2), tpb, 0, st>>>(c.hC, c.attr, S);
-        }
-        k_bc_eos<RS, R><<<gE, bE, 0, st>>>(c.hC, c.attr, S, c.part, c.dS);
-    }
+    const unsigned inner = (unsigned)(((size_t)(c.ny - 2) * (c.nz - 2) + NT - 1) / NT);
+    k_bc<RS, R><<<(unsigned)(c.nx - 2) + inner, NT, 0, st>>>(c.hC, c.attr, S, c.plane, c.noise, c.inlet_pos, c.dS);
     if (c.avg) {
         AvgBuf A;
         for (int q = 0; q < NAVG; q++) A.p[q] = c.avg + (size_t)q * c.n;
         k_time_avg<RS, R><<<MON_BLOCKS, NT, 0, st>>>(S, A, c.dS, c.n, c.avg_start);
     }
-    if (device_mode) {
-        const int tpb = 64;
-        k_loop_post<RS, R><<<dim3((c.ny + tpb - 1) / tpb, c.loop_nst > 0 ? c.loop_nst : 1), tpb, 0, st>>>(
-            c.hC, S, P, c.dS, c.loop_st, c.loop_nst, c.loop_kline, c.loop_cap, c.hist_probe, c.hist_dt, c.hist_umax);
-        k_loop_monitor<RS, R><<<MON_BLOCKS, NT, 0, st>>>(c.hC, S, c.part, c.dS, c.n, c.loop_cap, c.hist_mon);
-        k_loop_tick<<<1, 1, 0, st>>>(c.dS);
-    }
+    if (device_mode)
+        k_loop_end<RS, R><<<MON_BLOCKS, NT, 0, st>>>(c.hC, S, P, c.part, c.dS, c.loop_st, c.loop_nst, c.loop_kline, c.n,
+                                                     c.loop_cap, c.hist_probe, c.hist_dt, c.hist_umax, c.hist_mon);
 }
 
 // One time step.  Host-driven (device_mode false): dt and t_loop come from the caller and
@@ -174,8 +161,7 @@ void step_tail(DevCtx& c, cudaStream_t st, bool device_mode) {
 template <typename R>
 cudaError_t step_impl(DevCtx& c, double dt, int t_loop, bool device_mode) {
     cudaStream_t st = c.stream;
-    if (!part_fits(c, filter_blocks(c), 1) || !part_fits(c, cell_blocks(c, SH_STRAIN), 2) || !part_fits(c, cell_blocks(c, SH_EOS), 1) ||
-        !part_fits(c, MON_BLOCKS, 6))
+    if (!part_fits(c, filter_blocks(c), 1) || !part_fits(c, MON_BLOCKS, 6))
         return cudaErrorInvalidValue;
     const dim3 gB = cell_grid(c, SH_STRAIN), bB = cell_block(c, SH_STRAIN);
     const dim3 gC = cell_grid(c, SH_FLOW), bC = cell_block(c, SH_FLOW);
@@ -192,20 +178,23 @@ cudaError_t step_impl(DevCtx& c, double dt, int t_loop, bool device_mode) {
     RS* rn = (RS*)c.rn;
 
     int tm = tmark_begin(c, 0);
-    if (device_mode) loop_pre(c);
-    else k_set_step<<<1, 1, 0, st>>>(c.dS, dt, t_loop);
-    // SEM inflow plane (:943-1075).  Only the boundary conditions read it, so it runs on a
-    // side stream beside the four RK stages (joined before the BC); with kernel timing on
-    // it runs in line so that its events bracket it alone.
-    const bool overlap = !c.timing && c.side && c.n_inlet > 0;
+    // The head of a step runs on a side stream: dt and the draws of the device loop beside the
+    // first stage's filter and properties, which need neither, the SEM inflow plane (:943-1075)
+    // beside the four RK stages, as only the boundary conditions read it.  With kernel timing
+    // on it runs in line so that its events bracket it alone.
+    const bool overlap = !c.timing && c.side;
+    cudaStream_t hs = overlap ? c.side : st;
+    if (!device_mode) k_set_step<<<1, 1, 0, st>>>(c.dS, dt, t_loop);
     if (overlap) {
         cudaEventRecord(c.ev_fork, st);
-        cudaStreamWaitEvent(c.side, c.ev_fork, 0);
-        sem_inflow(c, c.side);
-        cudaEventRecord(c.ev_join, c.side);
-    } else {
-        sem_inflow(c, st);
+        cudaStreamWaitEvent(hs, c.ev_fork, 0);
     }
+    if (device_mode) {
+        loop_pre(c, hs);
+        if (overlap) cudaEventRecord(c.ev_dt, hs);
+    }
+    sem_inflow(c, hs);
+    if (overlap) cudaEventRecord(c.ev_join, hs);
     tmark_end(c, tm);
     // four RK4 stages (:4428-4544)
     for (int s = 0; s < 4; s++) {
@@ -216,6 +205,7 @@ cudaError_t step_impl(DevCtx& c, double dt, int t_loop, bool device_mode) {
         tm = tmark_begin(c, 2);
         launch_props<R, false>(c, gB, bB, st, F, P, s == 3 ? 1 : 0, Batch{});
         tmark_end(c, tm);
+        if (s == 0 && device_mode && overlap) cudaStreamWaitEvent(st, c.ev_dt, 0);
         // the k-arrays of the first stage are kept for inspection when requested
         const KDbg<R>& kds = (s == 0) ? kd : knone;
         tm = tmark_begin(c, 5);
@@ -245,7 +235,7 @@ cudaError_t step_impl(DevCtx& c, double dt, int t_loop, bool device_mode) {
 
 template <typename R>
 cudaError_t batch_head(DevCtx& c) {
-    loop_pre(c);
+    loop_pre(c, c.stream);
     sem_inflow(c, c.stream);
     return cudaGetLastError();
 }
@@ -258,7 +248,7 @@ cudaError_t batch_tail(DevCtx& c) {
 
 template <typename R>
 cudaError_t batch_stages(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t st) {
-    if (nmem < 1 || !part_fits(c0, filter_blocks(c0), 1) || !part_fits(c0, cell_blocks(c0, SH_STRAIN), 2)) return cudaErrorInvalidValue;
+    if (nmem < 1 || !part_fits(c0, filter_blocks(c0), 1)) return cudaErrorInvalidValue;
     auto grid = [&](int cls, Batch& b) {
         dim3 g = cell_grid(c0, cls);
         b.mt = mt;
@@ -296,7 +286,7 @@ cudaError_t batch_stages(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t
 template <typename R>
 cudaError_t rhs_only_impl(DevCtx& c, int t_loop) {
     cudaStream_t st = c.stream;
-    if (!part_fits(c, filter_blocks(c), 1) || !part_fits(c, cell_blocks(c, SH_STRAIN), 2)) return cudaErrorInvalidValue;
+    if (!part_fits(c, filter_blocks(c), 1)) return cudaErrorInvalidValue;
     F11<RS> S = f11<RS>(c.S);
     F11<R> St = f11<R>(c.St), F = f11<R>(c.F);
     PropBuf<R> P = props<R>(c);

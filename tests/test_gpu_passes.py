@@ -1,0 +1,82 @@
+"""The stage passes and the boundary kernel where they can go wrong: grids whose rows are no
+multiple of a 16-byte access, grids as small as a solver takes, and cells on either side of the
+line between the property pass's ordinary and general paths.
+
+Tolerances: the parity tolerances of tests/test_gpu_parity.py (intermediates 1e-12, state 1e-10
+after one step, 1e-8 after three).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+STATE = ["u", "v", "w", "T", "G", "rho", "Y0", "Y1", "Y2", "Y3", "Y4"]
+PROPS = ["nu", "mu_mix", "Cp", "lambda", "alpha"] + [f"D{k}" for k in range(5)]
+
+
+def rel(a, b):
+    nb = np.linalg.norm(b)
+    return float(np.linalg.norm(a - b) / (nb if nb > 0 else 1.0))
+
+
+@pytest.fixture(scope="module")
+def N(lesgpu_native, cuda_device):
+    return lesgpu_native
+
+
+def _grid(nx, ny, nz):
+    from lesgpu.config import preset
+    return preset("tiny").replace(nx=nx, ny=ny, nz=nz, lx=0.002 * nx, ly=0.002 * ny, lz=0.002 * nz,
+                                  num_vortices=20, initial_flame_front_i=nx // 3, inlet_radius=0.5 * 0.002 * ny,
+                                  seed=11)
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(4, 4, 4), (5, 6, 7), (9, 8, 10), (12, 5, 33), (7, 9, 64), (16, 11, 130), (33, 7, 6)])
+def test_steps_on_small_and_odd_grids(N, oracle_mod, nx, ny, nz):
+    cfg = _grid(nx, ny, nz)
+    orc = oracle_mod.Oracle(cfg.as_dict())
+    sol = N.Solver(cfg)
+    for n in (1, 2, 3):
+        orc.step()
+        sol.step()
+        assert abs(sol.last_dt - orc.dt) <= 1e-13 * orc.dt, f"dt differs at step {n}"
+        st, ref = sol.state(), orc.state()
+        errs = {f: rel(st[f], ref[f]) for f in STATE}
+        k = max(errs, key=errs.get)
+        assert errs[k] <= (1e-10 if n == 1 else 1e-8), f"step {n}: {k} {errs[k]:.2e}"
+    sol.close()
+    orc.close()
+
+
+@pytest.mark.parametrize("T", [140.0, 149.0, 151.0, 300.0, 999.0, 1001.0, 2200.0, 3990.0, 4100.0])
+def test_properties_on_both_sides_of_the_ordinary_range(N, oracle_mod, T):
+    """A temperature ramp of 3 per cent around T with every kind of composition: all species,
+    several absent, one pure species, next to no mass."""
+    cfg = _grid(17, 8, 12)
+    orc = oracle_mod.Oracle(cfg.as_dict())
+    shape = (cfg.nx, cfg.ny, cfg.nz)
+    st = orc.state()
+    i = np.arange(cfg.nx)[:, None, None] + np.zeros(shape)
+    st["T"] = T * (0.985 + 0.03 * np.linspace(0.0, 1.0, cfg.nz)[None, None, :]) + np.zeros(shape)
+    mixes = [[0.1, 0.2, 0.5, 0.12, 0.08], [0.0, 0.232, 0.768, 0.0, 0.0], [0.0, 0.0, 1.0, 0.0, 0.0],
+             [0.06, 0.22, 0.72, 0.0, 0.0], [1e-14, 1e-14, 1e-14, 0.0, 0.0]]
+    which = (i // 3).astype(int) % len(mixes)
+    for k in range(5):
+        st[f"Y{k}"] = np.array([m[k] for m in mixes])[which]
+    st["rho"] = np.full(shape, 0.7)
+    for f in STATE:
+        orc.set_field(f, st[f])
+    ctx = N.Context(cfg)
+    ctx.upload_attribute(orc.attribute())
+    ctx.upload_state(st)
+    ctx.eval_rhs(0)
+    orc.rhs_only(0)
+    fluid = orc.attribute() == 3
+    bad = {}
+    for f in PROPS:
+        e = rel(ctx.field(f)[fluid], orc.field(f)[fluid])
+        if not e <= 1e-12:
+            bad[f] = e
+    ctx.close()
+    orc.close()
+    assert not bad, bad
