@@ -585,6 +585,7 @@ __global__ void __launch_bounds__(NT)
     const int tid = threadIdx.x, sI = ny * nz;
     const int pv = blockIdx.x * NT + tid;
     const int i0 = blockIdx.y * seg, i1 = min(i0 + seg, nx);
+    pdl_wait();
     double mass = 0.0;
     if (pv < ny * nv) {
         const int j = pv / nv, k = (pv - j * nv) * V;
@@ -682,6 +683,7 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
         if (tid < EXP_STEPS) tab[tid] = C.exp_tab[tid];
         __syncthreads();
     }
+    pdl_wait();
     const bool here = k < nz && j < ny && i < nx;
     const int id = here ? (int)cid(i, j, k, ny, nz) : 0;
     const bool interior = here && i >= 1 && i < nx - 1 && j >= 1 && j < ny - 1 && k >= 1 && k < nz - 1;
@@ -1107,6 +1109,7 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = bz * blockDim.z + threadIdx.z;
+    pdl_wait();
     if (k >= nz || j >= ny || i >= C.nx) return;
     const size_t id = cid(i, j, k, ny, nz);
     if (PART == RK_MIDDLE && id == 0) reset_maxima(Sc);
@@ -1160,6 +1163,7 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = bz * blockDim.z + threadIdx.z;
+    pdl_wait();
     if (k >= nz || j >= ny || i >= C.nx) return;
     const int id = (int)cid(i, j, k, ny, nz);
     const int a = attr[id];
@@ -1425,6 +1429,7 @@ __global__ void __launch_bounds__(NT) k_bc(LES_KERNEL_CONSTS, const uint8_t* __r
     const int nx = C.nx, ny = C.ny, nz = C.nz, tid = threadIdx.x;
     const int ring = 2 * (ny + nz) - 4;
     int j, k;
+    pdl_wait();
     if ((int)blockIdx.x >= nx - 2) {
         const int q = ((int)blockIdx.x - (nx - 2)) * NT + tid;
         if (q >= (ny - 2) * (nz - 2)) return;
@@ -1613,6 +1618,7 @@ __global__ void __launch_bounds__(NT)
                double* __restrict__ hdt, double* __restrict__ humax, double* __restrict__ hmon) {
     __shared__ double sh[NT / 32];
     const int ny = C.ny, nz = C.nz, tid = threadIdx.x;
+    pdl_wait();
     const int slot = Sc->run_step;
     const bool monitor = Sc->t_loop % 10 == 0;          // uniform across the grid
     const unsigned nblk = gridDim.x;

@@ -46,6 +46,23 @@ static inline dim3 cell_grid(const DevCtx& c, int cls) {
                 (unsigned)((c.nx + t.bz - 1) / t.bz));
 }
 
+// A launch in a step's chain.  With `pdl` it may start while the launch before it in the stream
+// drains (pdl_wait); without, it starts when everything before it is complete, as a launch does
+// that follows an event of another stream.
+template <typename... P, typename... A>
+static inline void chain(bool pdl, void (*kernel)(P...), dim3 g, dim3 b, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = g;
+    cfg.blockDim = b;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // The filter pass: 16-byte accesses where a row is a multiple of them, and as many planes per
 // thread as leave every SM several blocks.
 constexpr int FILTER_SEG = 8;
@@ -61,16 +78,16 @@ static inline dim3 filter_grid(const DevCtx& c, size_t bytes, int& seg) {
     return dim3(gx, (unsigned)((c.nx + seg - 1) / seg), NSTATE);
 }
 template <typename R, typename RI, bool BATCH>
-static inline void launch_filter(const DevCtx& c, cudaStream_t st, const F11<RI>& in, const F11<R>& F, int members,
+static inline void launch_filter(bool pdl, const DevCtx& c, cudaStream_t st, const F11<RI>& in, const F11<R>& F, int members,
                                  const Batch& B) {
     constexpr int V = 16 / sizeof(RI);
     int seg;
     dim3 g = filter_grid(c, sizeof(RI), seg);
     g.z *= (unsigned)members;
     if (filter_vec(c, sizeof(RI)) == V)
-        k_filter<V, R, RI, BATCH><<<g, NT, 0, st>>>(c.hC, c.attr, in, F, c.part, c.dS, seg, B);
+        chain(pdl, k_filter<V, R, RI, BATCH>, g, NT, st, c.hC, c.attr, in, F, c.part, c.dS, seg, B);
     else
-        k_filter<1, R, RI, BATCH><<<g, NT, 0, st>>>(c.hC, c.attr, in, F, c.part, c.dS, seg, B);
+        chain(pdl, k_filter<1, R, RI, BATCH>, g, NT, st, c.hC, c.attr, in, F, c.part, c.dS, seg, B);
 }
 static inline size_t filter_blocks(const DevCtx& c) {
     int seg;
@@ -81,49 +98,49 @@ static inline size_t filter_blocks(const DevCtx& c) {
 
 // The property, flow and scalar passes with the kernel instance of their tile's block size.
 template <typename R, bool BATCH>
-static inline void launch_props(const DevCtx& c, dim3 g, dim3 b, cudaStream_t st, const F11<R>& F, const PropBuf<R>& P,
+static inline void launch_props(bool pdl, const DevCtx& c, dim3 g, dim3 b, cudaStream_t st, const F11<R>& F, const PropBuf<R>& P,
                                 int keep, const Batch& B) {
-    if (b.x * b.y * b.z == 512) k_props<R, BATCH, 512><<<g, b, 0, st>>>(c.hC, c.attr, F, P, c.dS, keep, B);
-    else k_props<R, BATCH><<<g, b, 0, st>>>(c.hC, c.attr, F, P, c.dS, keep, B);
+    if (b.x * b.y * b.z == 512) chain(pdl, k_props<R, BATCH, 512>, g, b, st, c.hC, c.attr, F, P, c.dS, keep, B);
+    else chain(pdl, k_props<R, BATCH>, g, b, st, c.hC, c.attr, F, P, c.dS, keep, B);
 }
 template <int PART, typename R, bool BATCH>
-static inline void launch_scalar_part(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
+static inline void launch_scalar_part(bool pdl, dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
                                       const F11<R>& F, const PropBuf<R>& P, const F11<RS>& S, const F11<R>& St,
                                       const AccBuf<R>& acc, RS* rn, const KDbg<R>& kd, Scalars* dS,
                                       int stage, const Batch& B) {
     if (b.x * b.y * b.z == 512)
-        k_rhs_scalar<PART, R, RS, BATCH, 512><<<g, b, 0, st>>>(hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+        chain(pdl, k_rhs_scalar<PART, R, RS, BATCH, 512>, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
     else
-        k_rhs_scalar<PART, R, RS, BATCH><<<g, b, 0, st>>>(hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+        chain(pdl, k_rhs_scalar<PART, R, RS, BATCH>, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
 }
 template <typename R, bool BATCH>
-static inline void launch_scalar(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
+static inline void launch_scalar(bool pdl, dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
                                  const F11<R>& F, const PropBuf<R>& P, const F11<RS>& S, const F11<R>& St,
                                  const AccBuf<R>& acc, RS* rn, const KDbg<R>& kd, Scalars* dS,
                                  int stage, const Batch& B) {
-    if (stage == 0) launch_scalar_part<RK_FIRST, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
-    else if (stage < 3) launch_scalar_part<RK_MIDDLE, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
-    else launch_scalar_part<RK_LAST, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    if (stage == 0) launch_scalar_part<RK_FIRST, R, BATCH>(pdl, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    else if (stage < 3) launch_scalar_part<RK_MIDDLE, R, BATCH>(pdl, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    else launch_scalar_part<RK_LAST, R, BATCH>(pdl, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
 }
 
 template <int PART, typename R, bool BATCH>
-static inline void launch_flow_part(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
+static inline void launch_flow_part(bool pdl, dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
                                       const F11<R>& F, const PropBuf<R>& P, const F11<RS>& S, const F11<R>& St,
                                       const AccBuf<R>& acc, RS* rn, const KDbg<R>& kd, Scalars* dS,
                                       int stage, const Batch& B) {
     if (b.x * b.y * b.z == 512)
-        k_rhs_flow<PART, R, RS, BATCH, 512><<<g, b, 0, st>>>(hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+        chain(pdl, k_rhs_flow<PART, R, RS, BATCH, 512>, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
     else
-        k_rhs_flow<PART, R, RS, BATCH><<<g, b, 0, st>>>(hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+        chain(pdl, k_rhs_flow<PART, R, RS, BATCH>, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
 }
 template <typename R, bool BATCH>
-static inline void launch_flow(dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
+static inline void launch_flow(bool pdl, dim3 g, dim3 b, cudaStream_t st, const Consts& hC, const uint8_t* attr,
                                  const F11<R>& F, const PropBuf<R>& P, const F11<RS>& S, const F11<R>& St,
                                  const AccBuf<R>& acc, RS* rn, const KDbg<R>& kd, Scalars* dS,
                                  int stage, const Batch& B) {
-    if (stage == 0) launch_flow_part<RK_FIRST, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
-    else if (stage < 3) launch_flow_part<RK_MIDDLE, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
-    else launch_flow_part<RK_LAST, R, BATCH>(g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    if (stage == 0) launch_flow_part<RK_FIRST, R, BATCH>(pdl, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    else if (stage < 3) launch_flow_part<RK_MIDDLE, R, BATCH>(pdl, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
+    else launch_flow_part<RK_LAST, R, BATCH>(pdl, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
 }
 
 // Every launch that writes per-block partials checks the buffer first: `per_block` values
@@ -139,19 +156,19 @@ static inline size_t cell_blocks(const DevCtx& c, int cls) {
 // The end of a step after the four RK stages: boundary conditions, EOS, time averages and,
 // in the device loop, the step's history and counters.
 template <typename R>
-void step_tail(DevCtx& c, cudaStream_t st, bool device_mode) {
+void step_tail(DevCtx& c, cudaStream_t st, bool device_mode, bool pdl) {
     F11<RS> S = f11<RS>(c.S);
     PropBuf<R> P = props<R>(c);
     const unsigned inner = (unsigned)(((size_t)(c.ny - 2) * (c.nz - 2) + NT - 1) / NT);
-    k_bc<RS, R><<<(unsigned)(c.nx - 2) + inner, NT, 0, st>>>(c.hC, c.attr, S, c.plane, c.noise, c.inlet_pos, c.dS);
+    chain(pdl, k_bc<RS, R>, (unsigned)(c.nx - 2) + inner, NT, st, c.hC, c.attr, S, c.plane, c.noise, c.inlet_pos, c.dS);
     if (c.avg) {
         AvgBuf A;
         for (int q = 0; q < NAVG; q++) A.p[q] = c.avg + (size_t)q * c.n;
         k_time_avg<RS, R><<<MON_BLOCKS, NT, 0, st>>>(S, A, c.dS, c.n, c.avg_start);
     }
     if (device_mode)
-        k_loop_end<RS, R><<<MON_BLOCKS, NT, 0, st>>>(c.hC, S, P, c.part, c.dS, c.loop_st, c.loop_nst, c.loop_kline, c.n,
-                                                     c.loop_cap, c.hist_probe, c.hist_dt, c.hist_umax, c.hist_mon);
+        chain(!c.timing && !c.avg, k_loop_end<RS, R>, MON_BLOCKS, NT, st, c.hC, S, P, c.part, c.dS, c.loop_st,
+              c.loop_nst, c.loop_kline, c.n, c.loop_cap, c.hist_probe, c.hist_dt, c.hist_umax, c.hist_mon);
 }
 
 // One time step.  Host-driven (device_mode false): dt and t_loop come from the caller and
@@ -196,30 +213,31 @@ cudaError_t step_impl(DevCtx& c, double dt, int t_loop, bool device_mode) {
     sem_inflow(c, hs);
     if (overlap) cudaEventRecord(c.ev_join, hs);
     tmark_end(c, tm);
+    const bool pdl = !c.timing;
     // four RK4 stages (:4428-4544)
     for (int s = 0; s < 4; s++) {
         tm = tmark_begin(c, 1);
-        if (s == 0) launch_filter<R, RS, false>(c, st, S, F, 1, Batch{});
-        else launch_filter<R, R, false>(c, st, St, F, 1, Batch{});
+        if (s == 0) launch_filter<R, RS, false>(false, c, st, S, F, 1, Batch{});
+        else launch_filter<R, R, false>(pdl, c, st, St, F, 1, Batch{});
         tmark_end(c, tm);
         tm = tmark_begin(c, 2);
-        launch_props<R, false>(c, gB, bB, st, F, P, s == 3 ? 1 : 0, Batch{});
+        launch_props<R, false>(pdl, c, gB, bB, st, F, P, s == 3 ? 1 : 0, Batch{});
         tmark_end(c, tm);
         if (s == 0 && device_mode && overlap) cudaStreamWaitEvent(st, c.ev_dt, 0);
         // the k-arrays of the first stage are kept for inspection when requested
         const KDbg<R>& kds = (s == 0) ? kd : knone;
         tm = tmark_begin(c, 5);
         if (c.scalar_tma && c.tma_ok) launch_scalar_tma<R, RS>(c, st, F, P, S, St, acc, rn, kds, s);
-        else launch_scalar<R, false>(gD, bD, st, c.hC, c.attr, F, P, S, St, acc, rn, kds, c.dS, s, Batch{});
+        else launch_scalar<R, false>(pdl && !(s == 0 && device_mode && overlap), gD, bD, st, c.hC, c.attr, F, P, S, St, acc, rn, kds, c.dS, s, Batch{});
         tmark_end(c, tm);
         tm = tmark_begin(c, 3);
-        launch_flow<R, false>(gC, bC, st, c.hC, c.attr, F, P, S, St, acc, rn, kds, c.dS, s, Batch{});
+        launch_flow<R, false>(pdl, gC, bC, st, c.hC, c.attr, F, P, S, St, acc, rn, kds, c.dS, s, Batch{});
         tmark_end(c, tm);
     }
     // apply_boundary_conditions (:2967-3161)
     if (overlap) cudaStreamWaitEvent(st, c.ev_join, 0);
     tm = tmark_begin(c, 4);
-    step_tail<R>(c, st, device_mode);
+    step_tail<R>(c, st, device_mode, pdl && !overlap);
     tmark_end(c, tm);
     tmark_flush(c);
     return cudaGetLastError();
@@ -242,7 +260,7 @@ cudaError_t batch_head(DevCtx& c) {
 
 template <typename R>
 cudaError_t batch_tail(DevCtx& c) {
-    step_tail<R>(c, c.stream, true);
+    step_tail<R>(c, c.stream, true, false);
     return cudaGetLastError();
 }
 
@@ -270,11 +288,11 @@ cudaError_t batch_stages(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t
     for (int q = 0; q < NACC; q++) knone.p[q] = nullptr;
     RS* rn = (RS*)c0.rn;
     for (int s = 0; s < 4; s++) {
-        if (s == 0) launch_filter<R, RS, true>(c0, st, S, F, nmem, Batch{mt, 0});
-        else launch_filter<R, R, true>(c0, st, St, F, nmem, Batch{mt, 0});
-        launch_props<R, true>(c0, gB, bB, st, F, P, s == 3 ? 1 : 0, BB);
-        launch_scalar<R, true>(gD, bD, st, c0.hC, c0.attr, F, P, S, St, acc, rn, knone, c0.dS, s, BD);
-        launch_flow<R, true>(gC, bC, st, c0.hC, c0.attr, F, P, S, St, acc, rn, knone, c0.dS, s, BC);
+        if (s == 0) launch_filter<R, RS, true>(false, c0, st, S, F, nmem, Batch{mt, 0});
+        else launch_filter<R, R, true>(true, c0, st, St, F, nmem, Batch{mt, 0});
+        launch_props<R, true>(true, c0, gB, bB, st, F, P, s == 3 ? 1 : 0, BB);
+        launch_scalar<R, true>(true, gD, bD, st, c0.hC, c0.attr, F, P, S, St, acc, rn, knone, c0.dS, s, BD);
+        launch_flow<R, true>(true, gC, bC, st, c0.hC, c0.attr, F, P, S, St, acc, rn, knone, c0.dS, s, BC);
     }
     return cudaGetLastError();
 }
@@ -297,20 +315,20 @@ cudaError_t rhs_only_impl(DevCtx& c, int t_loop) {
     RS* rn = (RS*)c.rn;
     k_set_step<<<1, 1, 0, st>>>(c.dS, 0.0, t_loop);
     int tm = tmark_begin(c, 1);
-    launch_filter<R, RS, false>(c, st, S, F, 1, Batch{});
+    launch_filter<R, RS, false>(false, c, st, S, F, 1, Batch{});
     tmark_end(c, tm);
     tm = tmark_begin(c, 2);
-    launch_props<R, false>(c, cell_grid(c, SH_STRAIN), cell_block(c, SH_STRAIN), st, F, P, 1, Batch{});
+    launch_props<R, false>(false, c, cell_grid(c, SH_STRAIN), cell_block(c, SH_STRAIN), st, F, P, 1, Batch{});
     tmark_end(c, tm);
     tm = tmark_begin(c, 5);
     if (c.scalar_tma && c.tma_ok)
         launch_scalar_tma<R, RS>(c, st, F, P, S, St, acc, rn, kd, 0);
     else
-        launch_scalar<R, false>(cell_grid(c, SH_SCALAR), cell_block(c, SH_SCALAR), st, c.hC, c.attr, F, P, S, St,
+        launch_scalar<R, false>(false, cell_grid(c, SH_SCALAR), cell_block(c, SH_SCALAR), st, c.hC, c.attr, F, P, S, St,
                                 acc, rn, kd, c.dS, 0, Batch{});
     tmark_end(c, tm);
     tm = tmark_begin(c, 3);
-    launch_flow<R, false>(cell_grid(c, SH_FLOW), cell_block(c, SH_FLOW), st, c.hC, c.attr, F, P, S, St, acc, rn, kd,
+    launch_flow<R, false>(false, cell_grid(c, SH_FLOW), cell_block(c, SH_FLOW), st, c.hC, c.attr, F, P, S, St, acc, rn, kd,
                           c.dS, 0, Batch{});
     tmark_end(c, tm);
     tmark_flush(c);

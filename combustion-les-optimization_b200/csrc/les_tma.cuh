@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(TMA_TK* TMA_TJ, (sizeof(R) == 8) ? 2 : 3)
     int& abort_flag = *reinterpret_cast<int*>(bars + 8);
 
     const int tid = threadIdx.y * TMA_TK + threadIdx.x;
+    pdl_wait();
     if (PART == RK_MIDDLE && tid == 0 && blockIdx.x + blockIdx.y + blockIdx.z == 0) reset_maxima(Sc);
     const int k0 = blockIdx.x * TMA_TK, j0 = blockIdx.y * TMA_TJ;
     const int i0 = blockIdx.z * iseg;
