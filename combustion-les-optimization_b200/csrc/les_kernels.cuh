@@ -688,10 +688,12 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
     const int id = here ? (int)cid(i, j, k, ny, nz) : 0;
     const bool interior = here && i >= 1 && i < nx - 1 && j >= 1 && j < ny - 1 && k >= 1 && k < nz - 1;
     const int a = here ? attr[id] : 0;
-    if (a == 3) {
-        R T = F.p[3][id], rho = F.p[5][id], G = F.p[4][id], Y[NSP];
+    // loaded beside the attribute, not after it: one trip to memory less
+    const R T = F.p[3][id], rho = F.p[5][id], G = F.p[4][id];
+    R Y[NSP];
 #pragma unroll
-        for (int s = 0; s < NSP; s++) Y[s] = F.p[6 + s][id];
+    for (int s = 0; s < NSP; s++) Y[s] = F.p[6 + s][id];
+    if (a == 3) {
         R num = R(0), div = R(0), nut = R(0), Smag = R(0);
         if (interior) {
             const int sI = ny * nz, sJ = nz;
@@ -972,6 +974,10 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
     const int nx = C.nx, ny = C.ny, nz = C.nz;
     const size_t id = cid(i, j, k, ny, nz);
     const int a = attr[id];
+    // loaded beside the attribute, not after it: one trip to memory less
+    const R vel[3] = {F.p[0][id], F.p[1][id], F.p[2][id]};
+    R g = F.p[4][id];
+
     if (a != 3) {
         // non-fluid cells: the temp state is Phi_n (:4444, :4454); rho_temp is only ever written on
         // outlet/fluid cells (:1893), so it stays 0 on inlet/wall/symmetry cells.  These values
@@ -1002,8 +1008,6 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
         return;
     }
 
-    const R vel[3] = {F.p[0][id], F.p[1][id], F.p[2][id]};
-    R g = F.p[4][id];
     // the right-hand sides and running sums of T, Y0..Y4 in this order, fields 3 and 5..9 of acc
     R kv[1 + NSP];
     const bool band2 = (i < 2 || i >= nx - 2 || j < 2 || j >= ny - 2 || k < 2 || k >= nz - 2);
@@ -1182,6 +1186,9 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
     if (k >= nz || j >= ny || i >= C.nx) return;
     const int id = (int)cid(i, j, k, ny, nz);
     const int a = attr[id];
+    // loaded beside the attribute, not after it: one trip to memory less
+    const R p0[3] = {F.p[0][id], F.p[1][id], F.p[2][id]};
+    const R r0 = F.p[5][id], G0 = F.p[4][id], n0 = P.nu_t[id], mu = P.mu_eff[id];
     if (a != 3) {
         // as in the scalar pass: the stage state of other cells is Phi_n, and the last stage leaves
         // cells off the faces as the EOS sweep does
@@ -1200,8 +1207,6 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
     const R ih[3] = {K.d_dx.r, K.d_dy.r, K.d_dz.r}, ih2[3] = {K.d_dxx.r, K.d_dyy.r, K.d_dzz.r};
     const bool band2 = (i < 2 || i >= nx - 2 || j < 2 || j >= ny - 2 || k < 2 || k >= nz - 2);
     const bool band3 = (i < 3 || i >= nx - 3 || j < 3 || j >= ny - 3 || k < 3 || k >= nz - 3);
-    const R p0[3] = {F.p[0][id], F.p[1][id], F.p[2][id]};
-    const R r0 = F.p[5][id], G0 = F.p[4][id], n0 = P.nu_t[id], mu = P.mu_eff[id];
     R km[3];
     {
         R out = R(0);
