@@ -1455,8 +1455,10 @@ int lesgpu_group_create(lesgpu_ctx* const* ctxs, int n, lesgpu_group** out) {
         for (int q = 0; q < n && el == cudaSuccess; q++) {
             DevCtx& d = ctxs[q]->d;
             el = cudaStreamWaitEvent(d.stream, g->fork, 0);
+            d.in_group = true;
             if (el == cudaSuccess)
                 el = (d.precision == LESGPU_FP64) ? les::step_f64(d, 0.0, 0, true) : les::step_f32(d, 0.0, 0, true);
+            d.in_group = false;
             if (el == cudaSuccess) el = cudaEventRecord(g->joins[q], d.stream);
             if (el == cudaSuccess) el = cudaStreamWaitEvent(g->root, g->joins[q], 0);
         }

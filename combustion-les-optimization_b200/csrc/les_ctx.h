@@ -77,6 +77,7 @@ struct DevCtx {
     void* kd[NACC] = {};
     void* grad_g = nullptr;             // optional |grad G| field (lesgpu_keep_grad_g)
     bool debug = false;
+    bool in_group = false;              // a group's step is being captured
     double* part = nullptr;             // per-block partials of the reductions
     size_t part_len = 0;
     double* plane = nullptr;            // SEM fluctuation planes, 3 x NY x NZ

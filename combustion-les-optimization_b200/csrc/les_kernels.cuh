@@ -956,6 +956,20 @@ struct GSrc {
     }
 };
 
+template <typename R>
+__device__ __forceinline__ GSrc<R> global_source(const F11<R>& F, const PropBuf<R>& P, int id, int ny, int nz) {
+    GSrc<R> src;
+    src.id = id;
+    src.s[0] = ny * nz;
+    src.s[1] = nz;
+    src.s[2] = 1;
+    src.T = F.p[3];
+#pragma unroll
+    for (int s = 0; s < NSP; s++) src.Y[s] = F.p[6 + s];
+    src.nut = P.nu_t;
+    return src;
+}
+
 // The RK stages as the scalar pass sees them: the first starts the running sum, the last ends it.
 enum { RK_FIRST = 0, RK_MIDDLE = 1, RK_LAST = 2 };
 
@@ -964,10 +978,10 @@ enum { RK_FIRST = 0, RK_MIDDLE = 1, RK_LAST = 2 };
 __device__ __forceinline__ void reset_maxima(Scalars* Sc) { Sc->umax = Sc->numax = Sc->alphamax = 0.0; }
 
 // One cell of the scalar pass (the body shared by both read paths).
-template <int PART, typename R, typename RS, typename Src>
+template <int PART, typename R, typename RS, typename Src, typename Hand>
 __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* __restrict__ attr, const F11<R>& F,
                                                 const PropBuf<R>& P, const F11<RS>& S0, const F11<R>& St,
-                                                const AccBuf<R>& acc, RS* __restrict__ rn, const KDbg<R>& kd,
+                                                const AccBuf<R>& acc, const Hand& hand, const KDbg<R>& kd,
                                                 Scalars* __restrict__ Sc, int stage, int i, int j, int k,
                                                 Src& src, const R relax) {
     const auto& K = kc<R>(C);
@@ -995,7 +1009,7 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
             for (int s = 0; s < NSP; s++) St.p[6 + s][id] = R(Y0[s]);
             if (a == 2) St.p[5][id] = R(r);
         } else if (PART == RK_LAST && off_faces(C, i, j, k)) {
-            rn[id] = eos_rho_state<R>(C, T0, Y0, RS(1.2));
+            hand(eos_rho_state<R>(C, T0, Y0, RS(1.2)));
             if ((a == 2 || a == 5) && renormalise<R>(Y0, RS(1e-6))) {
 #pragma unroll
                 for (int s = 0; s < NSP; s++) S0.p[6 + s][id] = Y0[s];
@@ -1087,7 +1101,7 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
 #pragma unroll
         for (int q = 0; q < 1 + NSP; q++) kd.p[q == 0 ? 3 : 4 + q][id] = kv[q];
     }
-    st_stream(rn + id, rho);
+    hand(rho);
     if (PART != RK_LAST) St.p[5][id] = R(rho);
 #pragma unroll
     for (int q = 0; q < 1 + NSP; q++) {
@@ -1132,16 +1146,9 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
     if (k >= nz || j >= ny || i >= C.nx) return;
     const size_t id = cid(i, j, k, ny, nz);
     if (PART == RK_MIDDLE && id == 0) reset_maxima(Sc);
-    GSrc<R> src;
-    src.id = (int)id;
-    src.s[0] = ny * nz;
-    src.s[1] = nz;
-    src.s[2] = 1;
-    src.T = F.p[3];
-#pragma unroll
-    for (int s = 0; s < NSP; s++) src.Y[s] = F.p[6 + s];
-    src.nut = P.nu_t;
-    rhs_scalar_cell<PART, R, RS>(C, attr, F, P, S0, St, acc, rn, kd, Sc, stage, i, j, k, src, relax);
+    GSrc<R> src = global_source<R>(F, P, (int)id, ny, nz);
+    auto hand = [&](RS rho) { st_stream(rn + id, rho); };
+    rhs_scalar_cell<PART, R, RS>(C, attr, F, P, S0, St, acc, hand, kd, Sc, stage, i, j, k, src, relax);
 }
 
 // C2: momentum (:2552-2697) with calculate_convection_conservative (:683-727) and the G
@@ -1153,56 +1160,25 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
 // Everything is in differences across the six faces: a conservative flux m p with the face
 // value p = p0 + d/2 (first-order upwind next to the boundary: p0 or p0 + d by the sign of m),
 // so convection and diffusion of all three components are two coefficients a face.
-template <int PART, typename R, typename RS = R, bool BATCH = false, int NTB = NT>
-__global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
-    k_rhs_flow(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, F11<RS> S0, F11<R> St,
-               AccBuf<R> acc, RS* __restrict__ rn, KDbg<R> kd, Scalars* __restrict__ Sc, int stage, Batch B) {
+// What the flow pass loads of a cell before it knows its attribute.
+template <typename R>
+struct FlowCell {
+    R p0[3], r0, G0, n0, mu;
+    __device__ __forceinline__ void load(const F11<R>& F, const PropBuf<R>& P, int id) {
+        p0[0] = F.p[0][id]; p0[1] = F.p[1][id]; p0[2] = F.p[2][id];
+        r0 = F.p[5][id]; G0 = F.p[4][id]; n0 = P.nu_t[id]; mu = P.mu_eff[id];
+    }
+};
+
+// The right-hand sides of rho u, rho v, rho w and G of one fluid cell.
+template <typename R>
+__device__ __forceinline__ void flow_rhs(const Consts& C, const ModelK<R>& M, const F11<R>& F, const PropBuf<R>& P,
+                                         const Scalars* __restrict__ Sc, int i, int j, int k, int id,
+                                         const FlowCell<R>& c, R (&kv)[4]) {
     const auto& K = kc<R>(C);
-    int bz = blockIdx.z;
-    ModelK<R> M;
-    if constexpr (BATCH) {
-        const int m = blockIdx.z / B.gz;
-        bz = blockIdx.z - m * B.gz;
-        const MemberTab& e = B.mt[m];
-        shift_all(F, e.delta);
-        shift_props(P, e.delta);
-        shift_all(S0, e.delta);
-        shift_all(St, e.delta);
-        shift_all(acc, e.delta);
-        rn = shifted(rn, e.delta);
-#pragma unroll
-        for (int q = 0; q < NACC; q++) kd.p[q] = nullptr;
-        attr = e.attr;
-        Sc = e.S;
-        M = member_model<R>(e);
-    } else {
-        M = model_of<R>(C);
-    }
     const int nx = C.nx, ny = C.ny, nz = C.nz;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i = bz * blockDim.z + threadIdx.z;
-    pdl_wait();
-    if (k >= nz || j >= ny || i >= C.nx) return;
-    const int id = (int)cid(i, j, k, ny, nz);
-    const int a = attr[id];
-    // loaded beside the attribute, not after it: one trip to memory less
-    const R p0[3] = {F.p[0][id], F.p[1][id], F.p[2][id]};
-    const R r0 = F.p[5][id], G0 = F.p[4][id], n0 = P.nu_t[id], mu = P.mu_eff[id];
-    if (a != 3) {
-        // as in the scalar pass: the stage state of other cells is Phi_n, and the last stage leaves
-        // cells off the faces as the EOS sweep does
-        if (PART == RK_FIRST) {
-#pragma unroll
-            for (int q = 0; q < 5; q++)
-                if (q != 3) St.p[q][id] = R(S0.p[q][id]);
-        } else if (PART == RK_LAST && off_faces(C, i, j, k)) {
-            S0.p[5][id] = rn[id];
-            const RS u = S0.p[0][id], v = S0.p[1][id], w = S0.p[2][id];
-            if (a == 1) max_into(&Sc->umax, sqrt(u * u + v * v + w * w));
-        }
-        return;
-    }
+    const R (&p0)[3] = c.p0;
+    const R r0 = c.r0, G0 = c.G0, n0 = c.n0, mu = c.mu;
     const int st[3] = {ny * nz, nz, 1};
     const R ih[3] = {K.d_dx.r, K.d_dy.r, K.d_dz.r}, ih2[3] = {K.d_dxx.r, K.d_dyy.r, K.d_dzz.r};
     const bool band2 = (i < 2 || i >= nx - 2 || j < 2 || j >= ny - 2 || k < 2 || k >= nz - 2);
@@ -1297,9 +1273,30 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
     const R gmag = qsqrt(fma(grad[2], grad[2], fma(grad[1], grad[1], grad[0] * grad[0])));
     if (P.grad_g) P.grad_g[id] = gmag;   // grad_G_magnitude_for_debug (:2783)
     kG = fma(P.ST[id], gmag, kG) + art;
+    kv[0] = km[0]; kv[1] = km[1]; kv[2] = km[2]; kv[3] = kG;
+}
 
-    // ---- RK4 bookkeeping (see rhs_scalar_cell); every load ahead of the first store
-    const R kv[4] = {km[0], km[1], km[2], kG};
+// A cell that is not fluid, as in the scalar pass: its stage state is Phi_n, and the last stage
+// leaves cells off the faces as the EOS sweep does.
+template <int PART, typename R, typename RS>
+__device__ __forceinline__ void flow_other(const Consts& C, int a, const F11<RS>& S0, const F11<R>& St,
+                                           Scalars* __restrict__ Sc, int i, int j, int k, int id, const RS* left) {
+    if (PART == RK_FIRST) {
+#pragma unroll
+        for (int q = 0; q < 5; q++)
+            if (q != 3) St.p[q][id] = R(S0.p[q][id]);
+    } else if (PART == RK_LAST && off_faces(C, i, j, k)) {
+        S0.p[5][id] = *left;
+        const RS u = S0.p[0][id], v = S0.p[1][id], w = S0.p[2][id];
+        if (a == 1) max_into(&Sc->umax, sqrt(u * u + v * v + w * w));
+    }
+}
+
+// The RK4 bookkeeping of a fluid cell (see rhs_scalar_cell) with the density that the scalar pass
+// left; every load ahead of the first store.
+template <int PART, typename R, typename RS>
+__device__ __forceinline__ void flow_update(const F11<RS>& S0, const F11<R>& St, const AccBuf<R>& acc, const KDbg<R>& kd,
+                                            Scalars* __restrict__ Sc, int stage, int id, const R (&kv)[4], RS left) {
     constexpr int qa[4] = {0, 1, 2, 4};
     RS sn[4];
     R ac[4];
@@ -1308,7 +1305,7 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
         sn[q] = ld_stream(S0.p[qa[q]] + id);
         ac[q] = PART != RK_FIRST ? ld_stream(acc.p[qa[q]] + id) : R(0);
     }
-    const RS rho_n = ld_stream(S0.p[5] + id), left = ld_stream(rn + id);
+    const RS rho_n = ld_stream(S0.p[5] + id);
     const RS rho = PART == RK_LAST ? fabs(left) : left;
     const double dt = Sc->dt;
     const RS cdt = PART == RK_LAST ? (RS)(dt / 6.0) : (RS)((PART == RK_MIDDLE && stage == 2 ? 1.0 : 0.5) * dt);
@@ -1342,6 +1339,90 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
         S0.p[5][id] = left < RS(0.0) ? RS(1.2) : left;
         // |u| of the next dt (:1472-1485)
         max_into(&Sc->umax, sqrt(out[0] * out[0] + out[1] * out[1] + out[2] * out[2]));
+    }
+}
+
+template <int PART, typename R, typename RS = R, bool BATCH = false, int NTB = NT>
+__global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
+    k_rhs_flow(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, F11<RS> S0, F11<R> St,
+               AccBuf<R> acc, RS* __restrict__ rn, KDbg<R> kd, Scalars* __restrict__ Sc, int stage, Batch B) {
+    const auto& K = kc<R>(C);
+    int bz = blockIdx.z;
+    ModelK<R> M;
+    if constexpr (BATCH) {
+        const int m = blockIdx.z / B.gz;
+        bz = blockIdx.z - m * B.gz;
+        const MemberTab& e = B.mt[m];
+        shift_all(F, e.delta);
+        shift_props(P, e.delta);
+        shift_all(S0, e.delta);
+        shift_all(St, e.delta);
+        shift_all(acc, e.delta);
+        rn = shifted(rn, e.delta);
+#pragma unroll
+        for (int q = 0; q < NACC; q++) kd.p[q] = nullptr;
+        attr = e.attr;
+        Sc = e.S;
+        M = member_model<R>(e);
+    } else {
+        M = model_of<R>(C);
+    }
+    const int nx = C.nx, ny = C.ny, nz = C.nz;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = bz * blockDim.z + threadIdx.z;
+    pdl_wait();
+    if (k >= nz || j >= ny || i >= nx) return;
+    const int id = (int)cid(i, j, k, ny, nz);
+    const int a = attr[id];
+    // loaded beside the attribute, not after it: one trip to memory less
+    FlowCell<R> c;
+    c.load(F, P, id);
+    if (a != 3) {
+        flow_other<PART, R, RS>(C, a, S0, St, Sc, i, j, k, id, rn + id);
+        return;
+    }
+    R kv[4];
+    flow_rhs<R>(C, M, F, P, Sc, i, j, k, id, c, kv);
+    flow_update<PART, R, RS>(S0, St, acc, kd, Sc, stage, id, kv, ld_stream(rn + id));
+}
+
+// Both passes in one launch, for grids that do not fill the GPU several times over: the first half
+// of a block's threads takes the scalar pass of its cells, the second half the flow pass, which
+// needs the other's density only for its update; it is handed over through shared memory at a
+// named barrier at which the scalar half arrives without waiting (2 blocks an SM; 1 and 3 were
+// slower).  When it is used: both_passes, les_launch.cuh.
+template <int PART, typename R, typename RS = R>
+__global__ void __launch_bounds__(2 * NT, 2)
+    k_rhs_both(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, F11<RS> S0, F11<R> St,
+               AccBuf<R> acc, KDbg<R> kd, Scalars* __restrict__ Sc, int stage, int3 tile) {
+    __shared__ RS rn[NT];
+    const int t = threadIdx.x & (NT - 1);
+    const int tk = t % tile.x, tj = (t / tile.x) % tile.y, ti = t / (tile.x * tile.y);
+    const int nx = C.nx, ny = C.ny, nz = C.nz;
+    const int k = blockIdx.x * tile.x + tk, j = blockIdx.y * tile.y + tj, i = blockIdx.z * tile.z + ti;
+    const bool here = k < nz && j < ny && i < nx;
+    const int id = here ? (int)cid(i, j, k, ny, nz) : 0;
+    pdl_wait();
+    if (threadIdx.x < NT) {
+        if (here) {
+            if (PART == RK_MIDDLE && id == 0) reset_maxima(Sc);
+            GSrc<R> src = global_source<R>(F, P, id, ny, nz);
+            auto hand = [&](RS rho) { rn[t] = rho; };
+            rhs_scalar_cell<PART, R, RS>(C, attr, F, P, S0, St, acc, hand, kd, Sc, stage, i, j, k, src, (R)kc<R>(C).relax);
+        }
+        __syncwarp();
+        asm volatile("barrier.cta.arrive 1, 512;" ::: "memory");
+    } else {
+        const int a = here ? attr[id] : 0;
+        FlowCell<R> c;
+        c.load(F, P, id);
+        R kv[4];
+        if (a == 3) flow_rhs<R>(C, model_of<R>(C), F, P, Sc, i, j, k, id, c, kv);
+        __syncwarp();
+        asm volatile("barrier.cta.sync 1, 512;" ::: "memory");
+        if (a == 3) flow_update<PART, R, RS>(S0, St, acc, kd, Sc, stage, id, kv, rn[t]);
+        else if (here) flow_other<PART, R, RS>(C, a, S0, St, Sc, i, j, k, id, &rn[t]);
     }
 }
 

@@ -143,6 +143,30 @@ static inline void launch_flow(bool pdl, dim3 g, dim3 b, cudaStream_t st, const 
     else launch_flow_part<RK_LAST, R, BATCH>(pdl, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
 }
 
+// Scalar and flow pass in one launch (k_rhs_both).  On a small grid both passes are short latency
+// chains on a GPU they do not fill, and one launch runs them side by side; on a larger one the flow
+// half's wait for the scalar half costs more than a launch and a tail.  64 steps (32 of
+// 128x64x64), apart -> together: 64x32x32 FP64 9.16 -> 8.24 ms, FP32 7.73 -> 7.22; 80x40x40 FP64 15.1 -> 13.9,
+// FP32 12.7 -> 12.3; 96x48x48 (221k cells) FP64 20.0 -> 19.2, FP32 13.5 -> 13.3; 110x56x54 (333k) FP32 22.4 ->
+// 22.5; 128x64x64 (524k) FP64 21.0 -> 22.0; 191x95x97 66.3 -> 71.4.  The line is at 2^18 cells.  Members of
+// a group keep them apart whatever their size, as together they fill the GPU (six 64x32x32 members:
+// 20.9 -> 25.9).
+constexpr size_t BOTH_CELLS = (size_t)1 << 18;
+static inline bool both_passes(const DevCtx& c) {
+    return !c.timing && !c.scalar_tma && !c.in_group && c.n <= BOTH_CELLS;
+}
+template <typename R>
+static inline void launch_both(bool pdl, const DevCtx& c, cudaStream_t st, const F11<R>& F, const PropBuf<R>& P,
+                               const F11<RS>& S, const F11<R>& St, const AccBuf<R>& acc, const KDbg<R>& kd, int stage) {
+    const int sh = c.shape[SH_FLOW] < NSHAPES_256 ? c.shape[SH_FLOW] : c.shape[SH_SCALAR] < NSHAPES_256 ? c.shape[SH_SCALAR] : 0;
+    const Shape t = kShapes[sh];
+    const int3 tile = make_int3(t.bx, t.by, t.bz);
+    const dim3 g((unsigned)((c.nz + t.bx - 1) / t.bx), (unsigned)((c.ny + t.by - 1) / t.by), (unsigned)((c.nx + t.bz - 1) / t.bz));
+    if (stage == 0) chain(pdl, k_rhs_both<RK_FIRST, R, RS>, g, 2 * NT, st, c.hC, c.attr, F, P, S, St, acc, kd, c.dS, stage, tile);
+    else if (stage < 3) chain(pdl, k_rhs_both<RK_MIDDLE, R, RS>, g, 2 * NT, st, c.hC, c.attr, F, P, S, St, acc, kd, c.dS, stage, tile);
+    else chain(pdl, k_rhs_both<RK_LAST, R, RS>, g, 2 * NT, st, c.hC, c.attr, F, P, S, St, acc, kd, c.dS, stage, tile);
+}
+
 // Every launch that writes per-block partials checks the buffer first: `per_block` values
 // per block for `blocks` blocks must fit in c.part.
 static inline bool part_fits(const DevCtx& c, size_t blocks, size_t per_block) {
@@ -226,6 +250,10 @@ cudaError_t step_impl(DevCtx& c, double dt, int t_loop, bool device_mode) {
         if (s == 0 && device_mode && overlap) cudaStreamWaitEvent(st, c.ev_dt, 0);
         // the k-arrays of the first stage are kept for inspection when requested
         const KDbg<R>& kds = (s == 0) ? kd : knone;
+        if (both_passes(c)) {   // (kernel timing brackets the two apart)
+            launch_both<R>(pdl && !(s == 0 && device_mode && overlap), c, st, F, P, S, St, acc, kds, s);
+            continue;
+        }
         tm = tmark_begin(c, 5);
         if (c.scalar_tma && c.tma_ok) launch_scalar_tma<R, RS>(c, st, F, P, S, St, acc, rn, kds, s);
         else launch_scalar<R, false>(pdl && !(s == 0 && device_mode && overlap), gD, bD, st, c.hC, c.attr, F, P, S, St, acc, rn, kds, c.dS, s, Batch{});

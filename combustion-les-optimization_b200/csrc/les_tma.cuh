@@ -231,7 +231,9 @@ __global__ void __launch_bounds__(TMA_TK* TMA_TJ, (sizeof(R) == 8) ? 2 : 3)
                 src.nut[d] = reinterpret_cast<const R*>(nbase + nslot * G::NSTRIDE) + (jl + 1) * G::BW +
                              (kl + G::KOFF);
             }
-            rhs_scalar_cell<PART, R, RS>(C, attr, F, P, S0, St, acc, rn, kd, Sc, stage, i, j, k, src, (R)kc<R>(C).relax);
+            RS* __restrict__ to = rn + cid(i, j, k, C.ny, C.nz);
+            auto hand = [&](RS rho) { st_stream(to, rho); };
+            rhs_scalar_cell<PART, R, RS>(C, attr, F, P, S0, St, acc, hand, kd, Sc, stage, i, j, k, src, (R)kc<R>(C).relax);
         }
         __syncthreads();                            // the plane of step rc - 2 is free
         if (tid == 0 && rc + 3 < nsteps) {

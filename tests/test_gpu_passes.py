@@ -80,3 +80,25 @@ def test_properties_on_both_sides_of_the_ordinary_range(N, oracle_mod, T):
     ctx.close()
     orc.close()
     assert not bad, bad
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny,nz,tile", [(4, 4, 4, 0), (9, 8, 10, 7), (33, 7, 6, 6), (12, 5, 33, 3), (64, 32, 32, 0), (64, 32, 32, 2)])
+def test_scalar_and_flow_in_one_launch(N, nx, ny, nz, tile, prec):
+    """Small grids run the scalar and flow passes as halves of one block; with kernel timing on
+    they run apart.  The arithmetic is the same: identical states in FP64, in FP32 up to how the
+    compiler contracts it (2^-24 a term, 1e-6 over three steps)."""
+    cfg = _grid(nx, ny, nz).replace(weno_transition_step=2)
+    out = []
+    for apart in (False, True):
+        s = N.Solver(cfg, precision=N.FP64 if prec == "fp64" else N.FP32)
+        s.ctx.set_tiles([0, tile, tile, tile, 0])
+        s.ctx.kernel_timing(apart)
+        s.step(3)
+        out.append(s.state())
+        s.close()
+    for f in STATE:
+        if prec == "fp64":
+            np.testing.assert_array_equal(out[0][f], out[1][f], err_msg=f)
+        else:
+            assert rel(out[0][f], out[1][f]) <= 1e-6, f
