@@ -115,8 +115,8 @@ struct DevCtx {
     double* hist_umax = nullptr;        // cap
     double* hist_mon = nullptr;         // cap x 6
     double lp_lbox = 0, lp_ly = 0, lp_lz = 0, lp_uin = 0, lp_ti = 0, lp_ell = 0, lp_cfl = 0, lp_cfld = 0, lp_dx = 0;
-    cudaGraphExec_t graph = nullptr;    // one captured device-loop step
-    bool graph_ok = false;
+    cudaGraphExec_t graph[2] = {};      // captured device-loop steps: one, and several of them
+    long long steps_run = 0;            // steps of the session so far
     int shape[NSH_CLASSES] = {0, 0, 0, 0, 0};   // tile (index into kShapes) per kernel class
     // scalar pass with TMA-staged stencil fields (les_tma.cuh): tensor maps of the six
     // filtered scalars and nu_t (7 CUtensorMap, 128 bytes each), built at create time
