@@ -100,8 +100,14 @@ struct DevCtx {
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;        // dt, draws and SEM plane, overlapped with the RK stages
     cudaEvent_t ev_fork = nullptr, ev_dt = nullptr, ev_join = nullptr;
-    double* h_pinned = nullptr;         // pinned staging for small transfers
+    double* h_pinned = nullptr;         // pinned staging of the host-driven inflow: noise, then vortices
     size_t h_pinned_len = 0;
+    Scalars* h_scal = nullptr;          // pinned copy of the scalar block
+    // host-driven steps replayed as a graph (lesgpu_step): its first node sets dt and t_loop
+    cudaGraph_t step_gr = nullptr;
+    cudaGraphExec_t step_graph = nullptr;
+    cudaGraphNode_t step_head = nullptr;
+    int step_count = 0;                 // host-driven steps since something the graph holds changed
     bool have_attr = false, have_state = false, have_inflow = false;
     // device-resident time loop (les_devloop.cuh)
     bool loop_ready = false;
