@@ -469,6 +469,7 @@ int lesgpu_create(const lesgpu_config* cfg, const lesgpu_species* sp, lesgpu_ctx
     d.n = (size_t)cfg->nx * cfg->ny * cfg->nz;
     d.precision = cfg->precision;
     d.esz = (cfg->precision == LESGPU_FP32) ? 4 : 8;
+    for (int q : {les::SH_STRAIN, les::SH_FLOW, les::SH_SCALAR}) d.shape[q] = les::default_shape(d.nx, d.ny, d.nz);
     build_consts(*cfg, *sp, d.hC);
     cudaError_t e = cudaSetDevice(cfg->device);
     if (e != cudaSuccess) { int r = cuda_fail(ctx, e, "cudaSetDevice"); delete ctx; return r; }

@@ -50,6 +50,18 @@ inline size_t max_cell_blocks(int nx, int ny, int nz) {
     return m;
 }
 
+// The tile of a context that sets none: 32x8x1, or the 256-thread shape that covers the grid with the
+// fewest blocks where that is at least 5 % fewer, since a block of mostly padding costs as much as
+// a full one.  Per step, 32x8x1 -> this choice: 60x20x40 FP64 208 -> 171 us (16x4x4), 70x35x38 FP64 220 -> 185,
+// 138x66x69 FP32 597 -> 538, 152x77x79 FP64 1236 -> 1146; 63x33x31 FP32 177 -> 183; ties (all powers of two)
+// keep 32x8x1, which is as good there or better.
+inline int default_shape(int nx, int ny, int nz) {
+    int best = 0;
+    for (int s = 1; s < NSHAPES_256; s++)
+        if (blocks_for_shape(nx, ny, nz, s) < blocks_for_shape(nx, ny, nz, best)) best = s;
+    return blocks_for_shape(nx, ny, nz, best) * 20 <= blocks_for_shape(nx, ny, nz, 0) * 19 ? best : 0;
+}
+
 struct DevCtx {
     int nx = 0, ny = 0, nz = 0, precision = 0;
     size_t n = 0;                       // cells
