@@ -560,7 +560,9 @@ __device__ __forceinline__ void ld_attr(const uint8_t* __restrict__ p, int (&a)[
 // properties held.  256x128x128, ms per step: filter and properties and, apart, strain took
 // 1.63 + 0.60 (FP64) and 0.92 + 0.24 (FP32); the filter alone, a cell a thread and 11 fields a block,
 // 0.76 and 0.58; in this form 0.59 and 0.36 (176 bytes a cell, 5.0 TB/s; seg = 4: 0.63, 16: 0.60,
-// 1: 0.92), with properties and strain together at 1.11 and 0.505.
+// 1: 0.92), with properties and strain together at 1.11 and 0.505.  With V = 1 a thread has few bytes
+// in flight, so it loads the plane after the next one ahead: 191x95x97 FP64 0.380 -> 0.336; with
+// V > 1 the registers cost more than that gives (256x128x128 0.592 -> 0.607, FP32 0.365 -> 0.379).
 template <int V, typename R, typename RI = R, bool BATCH = false>
 __global__ void __launch_bounds__(NT)
     k_filter(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<RI> in, F11<R> F, double* __restrict__ part,
@@ -585,21 +587,27 @@ __global__ void __launch_bounds__(NT)
     const int tid = threadIdx.x, sI = ny * nz;
     const int pv = blockIdx.x * NT + tid;
     const int i0 = blockIdx.y * seg, i1 = min(i0 + seg, nx);
+    constexpr bool AHEAD = V == 1;
     pdl_wait();
     double mass = 0.0;
     if (pv < ny * nv) {
         const int j = pv / nv, k = (pv - j * nv) * V;
         const bool row = j >= 1 && j < ny - 1;
         int id = i0 * sI + j * nz + k;
-        RI lo[V], c[V], hi[V];
+        RI lo[V], c[V], hi[V], ahead[V];
         ld_vec<RI, V>(x + id, c);
 #pragma unroll
         for (int v = 0; v < V; v++) lo[v] = c[v];
         if (i0 > 0) ld_vec<RI, V>(x + id - sI, lo);
+        if (AHEAD && i0 + 1 < nx) ld_vec<RI, V>(x + id + sI, hi);
         for (int i = i0; i < i1; i++, id += sI) {
             int a[V];
             ld_attr<V>(attr + id, a);
-            if (i + 1 < nx) ld_vec<RI, V>(x + id + sI, hi);
+            if constexpr (AHEAD) {
+                if (i + 1 < i1 && i + 2 < nx) ld_vec<RI, V>(x + id + 2 * sI, ahead);
+            } else {
+                if (i + 1 < nx) ld_vec<RI, V>(x + id + sI, hi);
+            }
             R f[V];
             if (row && i >= 1 && i < nx - 1) {
                 RI dn[V], up[V];
@@ -627,7 +635,11 @@ __global__ void __launch_bounds__(NT)
                     if (a[v] == 1 || a[v] == 2 || a[v] == 3 || a[v] == 5) mass += (((double)f[v] * C.dx) * C.dy) * C.dz;
             }
 #pragma unroll
-            for (int v = 0; v < V; v++) { lo[v] = c[v]; c[v] = hi[v]; }
+            for (int v = 0; v < V; v++) {
+                lo[v] = c[v];
+                c[v] = hi[v];
+                if (AHEAD) hi[v] = ahead[v];
+            }
         }
     }
     if (q != 5) return;
