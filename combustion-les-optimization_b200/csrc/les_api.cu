@@ -121,7 +121,6 @@ void build_consts(const lesgpu_config& g, const lesgpu_species& sp, les::Consts&
     C.dx4 = pow(C.dx, 4.0);
     C.inlet_center_z = g.lz / 2.0;       // INLET_CENTER_Z (:110)
     for (int s = 0; s < les::NSP; s++) {
-        C.mw[s] = sp.mw[s];
         C.mwk[s] = sp.mw[s] / 1000.0;
         C.t_mid[s] = sp.t_mid[s];
         for (int q = 0; q < 7; q++) { C.nasa_high[s][q] = sp.nasa_high[s][q]; C.nasa_low[s][q] = sp.nasa_low[s][q]; }
@@ -176,8 +175,6 @@ void build_consts(const lesgpu_config& g, const lesgpu_species& sp, les::Consts&
     C.d_dx = dc(C.dx); C.d_dy = dc(C.dy); C.d_dz = dc(C.dz);
     C.d_2dx = dc(C.two_dx); C.d_2dy = dc(C.two_dy); C.d_2dz = dc(C.two_dz);
     C.d_dxx = dc(C.dxx); C.d_dyy = dc(C.dyy); C.d_dzz = dc(C.dzz);
-    C.d_six = dc(6.0);
-    C.d_filter = dc(6.0 + 50.0);
     C.d_sct2 = dc(C.sc_t2); C.d_prt2 = dc(C.pr_t2);
     C.d_ramp = dc(0.03);
     C.d_w2 = dc(C.two_w2);
@@ -185,14 +182,6 @@ void build_consts(const lesgpu_config& g, const lesgpu_species& sp, les::Consts&
     for (int a = 0; a < les::NSP; a++) {
         C.d_mwk[a] = dc(C.mwk[a]);
         for (int b = 0; b < les::NSP; b++) C.d_wden[a][b] = dc(C.wden[a][b]);
-    }
-    // TENO weight sums w0 + w1 + w2 (w = d * {0.1, 0.6, 0.3}) for each cut-off pattern, with
-    // the kernel's operation order (teno5_reconstruct, :2224-2231)
-    for (int q = 0; q < 8; q++) {
-        const int d0 = q & 1, d1 = (q >> 1) & 1, d2 = (q >> 2) & 1;
-        const double w0 = (double)d0 * 0.1, w1 = (double)d1 * 0.6, w2 = (double)d2 * 0.3;
-        const double ws = w0 + w1 + w2;
-        C.d_tenows[q] = dc(q == 0 ? 1.0 : ws);
     }
     C.ssr_exp = 2.0 - C.d3;                                             // :1946
     build_fits(sp, C);
@@ -784,7 +773,7 @@ int lesgpu_set_inflow(lesgpu_ctx* ctx, const double* vortices, int nv, const dou
         dfree(d, d.vort);
         d.vort = nb;
         d.nv_cap = nv;
-        drop_step_graph(d);
+        drop_graph(d);      // every graph holds the old buffer's address
     }
     if (nv != d.nv) drop_step_graph(d);
     d.nv = nv;
@@ -1178,8 +1167,8 @@ int lesgpu_autotune(lesgpu_ctx* ctx, int reps, int tiles_out[5], double* ms_out)
     double ms[4][les::NSHAPES];
     cudaError_t e = cudaSuccess;
     for (int t = 0; t < les::NSHAPES && e == cudaSuccess; t++) {
-        // a 512-thread tile is timed for the strain, flow and scalar classes; the filter and
-        // EOS kernels keep the first tile meanwhile
+        // a 512-thread tile is timed for the strain, flow and scalar classes; the EOS class (the
+        // |u| reduction) keeps the first tile meanwhile, and the filter pass has no tile
         for (int q = 0; q < les::NSH_CLASSES; q++) d.shape[q] = les::shape_allowed(q, t) ? t : 0;
         d.timing = false;
         e = (d.precision == LESGPU_FP64) ? les::rhs_only_f64(d, 0) : les::rhs_only_f32(d, 0);   // warm-up
@@ -1209,7 +1198,7 @@ int lesgpu_autotune(lesgpu_ctx* ctx, int reps, int tiles_out[5], double* ms_out)
     best[les::SH_EOS] = best[les::SH_FILTER];
     for (int q = 0; q < les::NSH_CLASSES; q++) d.shape[q] = best[q];
     // The TMA-staged scalar pass (les_tma.cuh) is not timed here: on B200 it is slower than the
-    // plain pass at every grid measured (256x128x128 FP64: 4.03 against 3.07 ms per step), so
+    // plain pass (256x128x128 FP64: 1.43 against 1.19 ms per step), so
     // tuning it would only cost time on every new grid shape.  It stays selectable with
     // lesgpu_set_scalar_staging, which the autotuner leaves as it is.
     drop_graph(d);

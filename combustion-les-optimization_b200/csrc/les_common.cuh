@@ -67,8 +67,8 @@ struct ModelK {
     X(inletYk, [NSP]) X(ambientYk, [NSP]) X(cons_o2, ) X(prod_co2, ) X(prod_h2o, )               \
     X(u_in, ) X(noise_amp, )                                                                     \
     XD(d_dx, ) XD(d_dy, ) XD(d_dz, ) XD(d_2dx, ) XD(d_2dy, ) XD(d_2dz, ) XD(d_dxx, ) XD(d_dyy, ) \
-    XD(d_dzz, ) XD(d_six, ) XD(d_filter, ) XD(d_sct2, ) XD(d_prt2, ) XD(d_ramp, ) XD(d_w2, )      \
-    XD(d_tau_sl, ) XD(d_mwk, [NSP]) XD(d_wden, [NSP][NSP]) XD(d_tenows, [8])                     \
+    XD(d_dzz, ) XD(d_sct2, ) XD(d_prt2, ) XD(d_ramp, ) XD(d_w2, )      \
+    XD(d_tau_sl, ) XD(d_mwk, [NSP]) XD(d_wden, [NSP][NSP])                     \
     X(t_split, ) X(cp_high, [NSP][5]) X(cp_low, [NSP][5]) X(w0, [NSP][NSP]) X(w1, [NSP][NSP])                  \
     X(f_smu, [NSP][4]) X(f_lam, [NSP][4]) X(f_idif, [NPAIR][4])
 
@@ -93,7 +93,7 @@ struct Consts {
     double inlet_center_z;              // LZ/2.0
     double total_volume;                // serial sum of DX*DY*DZ over attr {1,2,3,5} (:2545)
     // species (:292-305)
-    double mw[NSP], mwk[NSP];           // g/mol and mw/1000.0
+    double mwk[NSP];                    // kg/mol
     double t_mid[NSP];
     double nasa_high[NSP][7], nasa_low[NSP][7];
     double eta[NSP][4], lam[NSP][4], dco[NSP][NSP][4];
@@ -102,10 +102,9 @@ struct Consts {
     double wden[NSP][NSP];              // sqrt(8.0)*sqrt(1.0 + M_i/M_j) [i][j]
     // divisors of the reference's divisions by constants, with reciprocals
     DC d_dx, d_dy, d_dz, d_2dx, d_2dy, d_2dz, d_dxx, d_dyy, d_dzz;
-    DC d_six, d_filter, d_sct2, d_prt2, d_ramp, d_w2, d_tau_sl;
+    DC d_sct2, d_prt2, d_ramp, d_w2, d_tau_sl;
     DC d_mwk[NSP];
     DC d_wden[NSP][NSP];
-    DC d_tenows[8];                     // TENO weight sums by cut-off pattern d0 + 2 d1 + 4 d2
     // model (:257-262, :2834, :2700-2704)
     double cs_u, cs_b, cs_boost;
     double accel_strength, accel_center, two_w2;   // two_w2 = 2.0*W*W
@@ -257,8 +256,8 @@ __device__ __forceinline__ double cdv(double x, const DC& d) {
 }
 __device__ __forceinline__ float cdv(float x, const DCT<float>& d) { return x * d.r; }
 
-// Arithmetic of the per-cell formulas.  The FP64 form uses IEEE double operations, as the
-// reference does; the FP32 form uses the hardware approximations (MUFU ex2/lg2/rcp/sqrt,
+// Arithmetic of the per-cell formulas.  The FP64 form uses IEEE double operations or, in the
+// property pass, the routines below with their stated errors; the FP32 form uses the hardware approximations (MUFU ex2/lg2/rcp/sqrt,
 // ~2 ulp), which its stated error budget covers.
 __device__ __forceinline__ double qdiv(double a, double b) { return a / b; }
 #ifdef LES_FP32_IEEE_MATH

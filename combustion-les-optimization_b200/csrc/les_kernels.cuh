@@ -14,13 +14,13 @@
 //                       of T, Y_k and rho; the new density is handed to C2.
 //   C2 k_rhs_flow     : momentum and G right-hand sides (calculate_RHS :2552-2825) fused with
 //                       the same update of u, v, w and G.
-// After the fourth stage the boundary kernels replay apply_boundary_conditions
+// After the fourth stage one kernel over the faces replays apply_boundary_conditions
 // (:2967-3161) in the reference's face order.
 //
 // Every kernel takes the constant table by value (__grid_constant__): divisors, their
-// reciprocals and the species data are read from the constant bank.  Divisions by
-// constants use cdv() (correctly rounded, see les_common.cuh); divisions by per-cell
-// values are IEEE divisions.
+// reciprocals and the species data are read from the constant bank.  FP64 arithmetic is explicit
+// about contraction (the unit is built without it; fma() where it is wanted), so that every
+// instance of a kernel gives the same bits.
 #pragma once
 
 #include <type_traits>
@@ -152,23 +152,9 @@ __device__ __forceinline__ R fit_prop(const R co[4], int zero, R L, R L2, R L3) 
     return qexp(lp);
 }
 
-template <typename R>
-__device__ __forceinline__ R eos_rho(const Consts& C, R T, const R Y[NSP], R fallback) {
-    const auto& K = kc<R>(C);
-    // update_rho_from_EOS (:1894-1905)
-    R syw = R(0);
-#pragma unroll
-    for (int s = 0; s < NSP; s++) syw += cdv(Y[s], K.d_mwk[s]);
-    if (syw > R(1e-9) && T > R(1.0)) {
-        R W = qdiv(R(1.0), syw);
-        R Rm = qdiv((R)R_UNIV, W);
-        return qdiv((R)P_CONST, Rm * T);
-    }
-    return fallback;
-}
-// The same on the FP64 state, with the state division of the precision form Form.  The gas
-// constant of the mixture is multiplied out (rho = p / ((R sum Y_k / M_k) T): one division
-// instead of three).
+// update_rho_from_EOS (:1894-1905) on the FP64 state, with the state division of the precision form
+// Form.  The gas constant of the mixture is multiplied out (rho = p / ((R sum Y_k / M_k) T): one
+// division instead of three).
 template <typename Form>
 __device__ __forceinline__ double eos_rho_state(const Consts& C, double T, const double Y[NSP], double fallback) {
     double syw = Y[0] * C.d_mwk[0].r;
@@ -616,13 +602,19 @@ __global__ void __launch_bounds__(NT)
                 const RI left = k > 0 ? __ldg(x + id - 1) : RI(0), right = k + V < nz ? __ldg(x + id + V) : RI(0);
 #pragma unroll
                 for (int v = 0; v < V; v++) {
-                    // (50 x + six neighbours) / 56 as x + (neighbours - 6 x) / 56: fewer roundings at
-                    // the size of x, and a uniform field stays exactly what it is.  In the input's
-                    // type: the FP32 form's first stage reads the FP64 state.
+                    // FP64: (50 x + six neighbours) / 56 as x + (neighbours - 6 x) / 56: fewer roundings at
+                    // the size of x, and a uniform field stays exactly what it is.  FP32: the sum
+                    // itself, in the reference's order, as the picks of the G equation (teno_picks)
+                    // hang on its last bits.
                     const RI kl = v > 0 ? c[v > 0 ? v - 1 : 0] : left, kr = v < V - 1 ? c[v < V - 1 ? v + 1 : 0] : right;
-                    const RI nb = lo[v] + dn[v] + kl + kr + up[v] + hi[v];
                     const bool inner = a[v] == 3 && k + v >= 1 && k + v < nz - 1;
-                    f[v] = R(inner ? fma(fma(RI(-6.0), c[v], nb), RI(1.0 / 56.0), c[v]) : c[v]);
+                    if constexpr (std::is_same<R, float>::value) {
+                        const R sum = fma(R(FILTER_W), R(c[v]), R(lo[v]) + R(dn[v]) + R(kl));
+                        f[v] = inner ? (sum + R(kr) + R(up[v]) + R(hi[v])) * R(1.0 / (FILTER_W + 6.0)) : R(c[v]);
+                    } else {
+                        const RI nb = lo[v] + dn[v] + kl + kr + up[v] + hi[v];
+                        f[v] = R(inner ? fma(fma(RI(-6.0), c[v], nb), RI(1.0 / 56.0), c[v]) : c[v]);
+                    }
                 }
             } else {
 #pragma unroll
@@ -835,6 +827,31 @@ __device__ __forceinline__ R teno_faces(R f1, R f2, R f3, R f4, R f5) {
     const R p = teno_pick<R>(smooth(t2, fma(R(3.0), f3, -f2)), smooth(t3, f3 + f4), smooth(t4, fma(R(-3.0), f4, f5)),
                              fma(R(5.0), f3, R(-2.0) * f2), fma(R(2.0), f4, f3), fma(R(4.0), f4, -f5));
     return fma(p - m, R(1.0 / 6.0), f3);
+}
+
+// The same from the six values v0..v5 for FP32.  Which candidates count is decided by comparing
+// smoothness with a fixed number, and a candidate more or less moves a cell at a front by 1e-3 of G in a few
+// steps.  The smoothness is therefore taken from the values in the reference's order, so that runs of the
+// FP32 form that differ only in how they round elsewhere decide alike (six 128x64x64 members, 32 steps:
+// two forms of the other passes apart by up to 1.3e-3 of G with the smoothness in differences, by 1e-4 so);
+// the candidates themselves are in differences.  FP32 flow pass 0.725 -> 0.743 ms per 256x128x128 step.
+__device__ __forceinline__ void teno_picks(float v0, float v1, float v2, float v3, float v4, float& is0, float& is1,
+                                           float& is2) {
+    const float a0 = v0 - 2.0f * v1 + v2, b0 = v0 - 4.0f * v1 + 3.0f * v2;
+    const float a1 = v1 - 2.0f * v2 + v3, b1 = v1 - v3;
+    const float a2 = v2 - 2.0f * v3 + v4, b2 = 3.0f * v2 - 4.0f * v3 + v4;
+    is0 = float(13.0 / 12.0) * (a0 * a0) + 0.25f * (b0 * b0);
+    is1 = float(13.0 / 12.0) * (a1 * a1) + 0.25f * (b1 * b1);
+    is2 = float(13.0 / 12.0) * (a2 * a2) + 0.25f * (b2 * b2);
+}
+__device__ __forceinline__ float teno_faces(float v0, float v1, float v2, float v3, float v4, float v5) {
+    const float f1 = v1 - v0, f2 = v2 - v1, f3 = v3 - v2, f4 = v4 - v3, f5 = v5 - v4;
+    float i0, i1, i2;
+    teno_picks(v0, v1, v2, v3, v4, i0, i1, i2);
+    const float m = teno_pick<float>(i0, i1, i2, fmaf(5.0f, f2, -2.0f * f1), fmaf(2.0f, f3, f2), fmaf(4.0f, f3, -f4));
+    teno_picks(v1, v2, v3, v4, v5, i0, i1, i2);
+    const float p = teno_pick<float>(i0, i1, i2, fmaf(5.0f, f3, -2.0f * f2), fmaf(2.0f, f4, f3), fmaf(4.0f, f4, -f5));
+    return fmaf(p - m, float(1.0 / 6.0), f3);
 }
 
 // The WENO5 gradient (:735-827, on the cells -2..+3 whatever the velocity) times the spacing, e1..e5 the
@@ -1260,7 +1277,8 @@ __device__ __forceinline__ void flow_rhs(const Consts& C, const ModelK<R>& M, co
             R d = f3;                                   // first-order upwind (:642-651)
             if (!band3) {
                 const R UU = G[id + 2 * o], U3 = G[id + 3 * o], DD = G[id - 2 * o];
-                d = teno_faces<R>(UU - U3, U - UU, f3, f4, DD - Dn);
+                if constexpr (std::is_same<R, float>::value) d = teno_faces(U3, UU, U, G0, Dn, DD);
+                else d = teno_faces<R>(UU - U3, U - UU, f3, f4, DD - Dn);
             } else if (!band2) {
                 // central faces (:652-677): the zero UW2 coefficient makes both upwind branches identical
                 d = R(0.5) * (f3 + f4);

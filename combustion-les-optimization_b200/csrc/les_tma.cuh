@@ -3,8 +3,7 @@
 //
 // The scalar pass reads six fields with a +-2 stencil in all three directions (filtered T and
 // Y_k: MUSCL, Laplacian, SGS flux) and nu_t with +-1.  From global memory each cell issues
-// ~13 loads per field, mostly L1/L2 hits whose latency the kernel cannot hide at its
-// occupancy.  Here a block owns a 32 x 8 (k, j) tile and marches through a segment of
+// 10 loads per field (its star follows the velocity), mostly L1/L2 hits.  Here a block owns a 32 x 8 (k, j) tile and marches through a segment of
 // i-planes: the (k, j) tile plus a 2-cell halo of each field, one i-plane at a time, is
 // copied by cp.async.bulk.tensor into a ring of five shared-memory planes (three for nu_t),
 // and the plane four ahead is in flight while the current one is computed.  Every value is

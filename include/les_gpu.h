@@ -305,8 +305,9 @@ int lesgpu_avg_upload(lesgpu_ctx* ctx, const double* const* sums, int count);
  * filter), installs it and optionally returns it and the times (ms_out: 4 classes x
  * LESGPU_NTILES, ms per launch; 1e30 where a shape does not serve the class).  It leaves the
  * state, the dt inputs and the step counters as they were.  The tile changes only the launch
- * geometry; results change only through the summation order of the block partials of
- * <rho_f> (rounding level). */
+ * geometry, never the results.  The filter pass chooses its own split: its tile is kept and
+ * reported but has no effect.  A context that sets none starts with 32x8x1, or with the 256-thread
+ * shape that covers its grid with the fewest blocks where that is at least 5 % fewer. */
 #define LESGPU_NTILES 13
 int lesgpu_set_tiles(lesgpu_ctx* ctx, const int tiles[5]);
 int lesgpu_get_tiles(const lesgpu_ctx* ctx, int tiles[5]);
@@ -315,7 +316,8 @@ int lesgpu_autotune(lesgpu_ctx* ctx, int reps, int tiles_out[5], double* ms_out)
  * (cp.async.bulk.tensor, a (32 x 8) tile marching through i-planes; the same arithmetic, so
  * the same bits).  Available when a grid row (NZ values) is a multiple of 16 bytes.  Off
  * by default and left alone by lesgpu_autotune: on B200 it is slower than the plain pass
- * (two resident blocks of 112.5 KB shared memory per SM instead of four). */
+ * (two resident blocks of 112.5 KB shared memory per SM instead of four; FP64 256x128x128 1.43
+ * against 1.19 ms per step). */
 int lesgpu_set_scalar_staging(lesgpu_ctx* ctx, int enable);
 int lesgpu_get_scalar_staging(const lesgpu_ctx* ctx);
 
