@@ -292,8 +292,8 @@ def run_ours(args):
         ctx.autotune(3)
     tiles = {k: "x".join(map(str, ctx.TILES[t])) for k, t in
              zip(["filter_props", "strain", "rhs_flow", "rhs_scalar", "eos"], ctx.get_tiles())}
-    # per step: loop_pre, 2 SEM, 4 x 4 stage kernels, 4 BC, loop_post, loop_monitor, loop_tick
-    per_step_launches = 1 + 2 + 16 + 4 + 3
+    # per step: loop_pre, 2 SEM, 4 x 4 stage kernels, the faces, loop_end
+    per_step_launches = 1 + 2 + 16 + 1 + 1
 
     # ---- warm-up (device-resident loop session; graph capture happens here)
     sol.loop_begin(chunk=max(args.warmup, args.steps))
