@@ -484,10 +484,12 @@ __device__ __forceinline__ bool cell_props_fast(const Consts& C, const double* t
 // ------------------------------------------------------------------ pass A: filter
 
 // Block partials of one or more reductions into part[q * nblk + block]; true in the last block to
-// arrive, whose threads may then reduce them.
+// arrive, whose threads may then reduce them and change what the blocks have read.  The block
+// arrives only when all its threads have come here, so what they read before is read.
 __device__ __forceinline__ bool last_block(double* part, unsigned nblk, unsigned bid, const double* v, int nv,
                                            unsigned* counter, int tid) {
     __shared__ bool last;
+    __syncthreads();
     if (tid == 0) {
         for (int q = 0; q < nv; q++) part[(size_t)q * nblk + bid] = v[q];
         __threadfence();
@@ -1773,10 +1775,18 @@ __global__ void __launch_bounds__(NT)
                const int* __restrict__ st, int nst, int kline, size_t n, int cap, double* __restrict__ hprobe,
                double* __restrict__ hdt, double* __restrict__ humax, double* __restrict__ hmon) {
     __shared__ double sh[NT / 32];
+    __shared__ int now[2];
     const int ny = C.ny, nz = C.nz, tid = threadIdx.x;
     pdl_wait();
-    const int slot = Sc->run_step;
-    const bool monitor = Sc->t_loop % 10 == 0;          // uniform across the grid
+    // The grid's last block advances these two: one thread reads them for its block, before the
+    // block can be counted as arrived.
+    if (tid == 0) {
+        now[0] = Sc->run_step;
+        now[1] = Sc->t_loop;
+    }
+    __syncthreads();
+    const int slot = now[0];
+    const bool monitor = now[1] % 10 == 0;              // uniform across the grid
     const unsigned nblk = gridDim.x;
     double v[6];
     if (slot >= 0 && slot < cap) {
