@@ -342,6 +342,9 @@ cudaError_t rhs_only_impl(DevCtx& c, int t_loop) {
     for (int q = 0; q < NACC; q++) kd.p[q] = (R*)c.kd[q];
     RS* rn = (RS*)c.rn;
     k_set_step<<<1, 1, 0, st>>>(c.dS, 0.0, t_loop);
+    // the nu and alpha maxima become this state's (the property pass raises them)
+    static_assert(offsetof(Scalars, alphamax) == offsetof(Scalars, numax) + sizeof(double), "cleared together");
+    cudaMemsetAsync(&c.dS->numax, 0, 2 * sizeof(double), st);
     int tm = tmark_begin(c, 1);
     launch_filter<R, RS, false>(false, c, st, S, F, 1, Batch{});
     tmark_end(c, tm);

@@ -102,3 +102,24 @@ def test_scalar_and_flow_in_one_launch(N, nx, ny, nz, tile, prec):
             np.testing.assert_array_equal(out[0][f], out[1][f], err_msg=f)
         else:
             assert rel(out[0][f], out[1][f]) <= 1e-6, f
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_dt_inputs_after_an_evaluation_are_that_states(N, prec):
+    """An evaluation of the right-hand sides leaves the nu and alpha maxima of the state it evaluated,
+    whatever larger ones the steps before it left."""
+    cfg = _grid(16, 11, 20)
+    s = N.Solver(cfg, precision=N.FP64 if prec == "fp64" else N.FP32)
+    s.step(2)
+    umax, nu0, al0 = s.ctx.dt_inputs()
+    st = s.state()
+    st["T"] = 0.5 * (st["T"] + st["T"].min())       # colder, so less viscous
+    st["rho"] = st["rho"] * 1.5
+    s.ctx.upload_state(st)
+    assert N.lib().lesgpu_set_dt_inputs(s.ctx._h, nu0, al0) == 0
+    s.ctx.eval_rhs(0)
+    _, nu, al = s.ctx.dt_inputs()
+    fluid = s.attribute() == 3
+    assert nu == s.field("nu")[fluid].max() < nu0
+    assert al == s.field("alpha")[fluid].max() < al0
+    s.close()
