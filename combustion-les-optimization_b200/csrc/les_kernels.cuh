@@ -1126,7 +1126,8 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
     RS rho = eos_rho_state<R>(C, up[0], up + 1, PART == RK_LAST ? RS(0.0) : rho_n);
     if (PART == RK_LAST) {
         // the EOS sweep after the boundary conditions (:3130-3160) finds this density again (and 1.2
-        // where there is none, which a negative sign tells the flow pass) and renormalises once more
+        // where there is none, which the sign bit tells the flow pass, of zero and NaN too) and
+        // renormalises once more
         if (rho == RS(0.0)) rho = -fabs(rho_n);
         renormalise<R>(up + 1, RS(1e-6));
     }
@@ -1395,7 +1396,7 @@ __device__ __forceinline__ void flow_update(const F11<RS>& S0, const F11<R>& St,
         }
     }
     if (PART == RK_LAST) {
-        S0.p[5][id] = left < RS(0.0) ? RS(1.2) : left;
+        S0.p[5][id] = signbit(left) ? RS(1.2) : left;
         // |u| of the next dt (:1472-1485)
         max_into(&Sc->umax, sqrt(out[0] * out[0] + out[1] * out[1] + out[2] * out[2]));
     }

@@ -123,3 +123,25 @@ def test_dt_inputs_after_an_evaluation_are_that_states(N, prec):
     assert nu == s.field("nu")[fluid].max() < nu0
     assert al == s.field("alpha")[fluid].max() < al0
     s.close()
+
+
+@pytest.mark.parametrize("rho", [0.0, 0.7])
+def test_density_of_cells_without_mass_fractions(N, oracle_mod, rho):
+    """Where the mass fractions are all zero the step keeps the density through its stages and the
+    sweep after the boundary conditions sets 1.2, whatever the density was, zero included."""
+    cfg = _grid(17, 12, 14).replace(relax=0.0)
+    orc = oracle_mod.Oracle(cfg.as_dict())
+    sol = N.Solver(cfg)
+    shape = (cfg.nx, cfg.ny, cfg.nz)
+    st = orc.state()
+    for f in STATE:
+        st[f] = np.full(shape, {"T": 300.0, "rho": rho}.get(f, 0.0))
+        orc.set_field(f, st[f])
+    sol.ctx.upload_state(st)
+    orc.step()
+    sol.step()
+    got, want = sol.state()["rho"], orc.state()["rho"]
+    assert (want[5:-3, 3:-3, 3:-3] == 1.2).all()
+    np.testing.assert_allclose(got, want, rtol=1e-10)
+    sol.close()
+    orc.close()
