@@ -69,8 +69,7 @@ struct ModelK {
     XD(d_dx, ) XD(d_dy, ) XD(d_dz, ) XD(d_2dx, ) XD(d_2dy, ) XD(d_2dz, ) XD(d_dxx, ) XD(d_dyy, ) \
     XD(d_dzz, ) XD(d_sct2, ) XD(d_prt2, ) XD(d_ramp, ) XD(d_w2, )      \
     XD(d_tau_sl, ) XD(d_mwk, [NSP]) XD(d_wden, [NSP][NSP])                     \
-    X(t_split, ) X(cp_high, [NSP][5]) X(cp_low, [NSP][5]) X(w0, [NSP][NSP]) X(w1, [NSP][NSP])                  \
-    X(f_smu, [NSP][4]) X(f_lam, [NSP][4]) X(f_idif, [NPAIR][4])
+    X(t_split, )
 
 struct ConstsF {
 #define LES_DECL_F(name, dims) float name dims;
@@ -174,14 +173,6 @@ inline void fill_float_consts(Consts& C) {
 #define LES_CONV(name, dims) to_float(C.f.name, C.name);
     LES_FCONSTS(LES_CONV, LES_CONV)
 #undef LES_CONV
-    // the FP32 form's fits are plain base-2 exponents (ex2.approx)
-    for (int q = 0; q < 4; q++) {
-        for (int s = 0; s < NSP; s++) {
-            C.f.f_smu[s][q] = (float)(C.f_smu[s][q] / EXP_STEPS);
-            C.f.f_lam[s][q] = (float)(C.f_lam[s][q] / EXP_STEPS);
-        }
-        for (int p = 0; p < NPAIR; p++) C.f.f_idif[p][q] = (float)(C.f_idif[p][q] / EXP_STEPS);
-    }
 }
 
 // A batched launch (les_launch.cuh, batch_stages) steps several members of one grid shape in
@@ -307,17 +298,22 @@ __device__ __forceinline__ double cquot(double a, double b, double y) {
 // in IEEE double, as the reference does.  The FP32 form keeps its state in FP64 only so that
 // small increments survive; there a float reciprocal refined by one Newton step and one
 // quotient correction in double (relative error ~1e-15) replaces the division sequence.
+// srecip is the reciprocal that quotients by one denominator share (cquot).
+template <typename Form>
+__device__ __forceinline__ double srecip(double b);
+template <>
+__device__ __forceinline__ double srecip<double>(double b) { return 1.0 / b; }
+template <>
+__device__ __forceinline__ double srecip<float>(double b) {
+    const double y = (double)__frcp_rn((float)b);
+    return fma(y, fma(-b, y, 1.0), y);
+}
 template <typename Form>
 __device__ __forceinline__ double sdiv(double a, double b);
 template <>
 __device__ __forceinline__ double sdiv<double>(double a, double b) { return a / b; }
 template <>
-__device__ __forceinline__ double sdiv<float>(double a, double b) {
-    double y = (double)__frcp_rn((float)b);
-    y = fma(y, fma(-b, y, 1.0), y);
-    const double q = a * y;
-    return fma(fma(-q, b, a), y, q);
-}
+__device__ __forceinline__ double sdiv<float>(double a, double b) { return cquot(a, b, srecip<float>(b)); }
 
 // 1 / x for a positive x far from the ends of the range: the hardware's approximation (about 20
 // bits) and one third-order Newton (Householder) step, y (1 + e + e^2) with e = 1 - x y: 2^-60 and
@@ -328,8 +324,6 @@ __device__ __forceinline__ double frcp(double x) {
     const double e = fma(-x, y, 1.0);
     return fma(y, fma(e, e, e), y);
 }
-__device__ __forceinline__ float frcp(float x) { return __fdividef(1.0f, x); }
-__device__ __forceinline__ float cquot(float a, float b, float y) { return a * y; }
 
 // 2^(t / EXP_STEPS) for |t| < 16000, t a fit's value: Tang's table-driven method (ACM TOMS 15,
 // 1989) in base 2.  t = k + r with an integer k and |r| <= 1/2, both exact, so no constant has to
@@ -351,12 +345,6 @@ __device__ __forceinline__ double exp2_fit(double t, const double* tab) {
     const double y = fma(v, p * r, v);
     return __hiloint2double(__double2hiint(y) + ((k >> 4) << 20), __double2loint(y));
 }
-__device__ __forceinline__ float exp2_fit(float t, const double*) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(t));
-    return y;
-}
-
 // x^3 and x^4 rounded once: glibc pow() returns the correctly rounded power for these
 // arguments, while a plain product rounds twice.  The exact square is split with fma,
 // the rest is carried as a double-double and rounded once at the end.

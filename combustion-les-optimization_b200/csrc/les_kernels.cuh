@@ -57,6 +57,28 @@ struct KDbg {                // optional (nullptr): the stage's k-arrays for ins
     R* p[NACC];
 };
 
+// What the properties of a cell are kept in.
+template <typename R>
+struct CellProps {
+    R D[NSP], mu_mix, nu, aT, cp, lam, alpha;
+};
+
+// What the flow pass loads of a cell before it knows its attribute.
+template <typename R>
+struct FlowCell {
+    R p0[3], r0, G0, n0, mu;
+    __device__ __forceinline__ void load(const F11<R>& F, const PropBuf<R>& P, int id) {
+        p0[0] = F.p[0][id]; p0[1] = F.p[1][id]; p0[2] = F.p[2][id];
+        r0 = F.p[5][id]; G0 = F.p[4][id]; n0 = P.nu_t[id]; mu = P.mu_eff[id];
+    }
+};
+
+}  // namespace les
+
+#include "les_f32_form.cuh"
+
+namespace les {
+
 #define LES_KERNEL_CONSTS const __grid_constant__ Consts C
 
 // A member's fields in a batched launch: every per-cell field lives in the member's arena at
@@ -153,14 +175,22 @@ __device__ __forceinline__ R fit_prop(const R co[4], int zero, R L, R L2, R L3) 
 }
 
 // update_rho_from_EOS (:1894-1905) on the FP64 state, with the state division of the precision form
-// Form.  The gas constant of the mixture is multiplied out (rho = p / ((R sum Y_k / M_k) T): one
-// division instead of three).
+// Form.  In the FP64 form the gas constant of the mixture is multiplied out (rho = p / ((R sum Y_k / M_k) T):
+// one division instead of three); the FP32 form keeps its three (les_f32_form.cuh says why).
 template <typename Form>
 __device__ __forceinline__ double eos_rho_state(const Consts& C, double T, const double Y[NSP], double fallback) {
-    double syw = Y[0] * C.d_mwk[0].r;
+    if constexpr (std::is_same<Form, float>::value) {
+        double syw = cdv(Y[0], C.d_mwk[0]);
 #pragma unroll
-    for (int s = 1; s < NSP; s++) syw = fma(Y[s], C.d_mwk[s].r, syw);
-    if (syw > 1e-9 && T > 1.0) return sdiv<Form>(P_CONST, (R_UNIV * syw) * T);
+        for (int s = 1; s < NSP; s++) syw += cdv(Y[s], C.d_mwk[s]);
+        if (syw > 1e-9 && T > 1.0)
+            return sdiv<Form>(P_CONST, __dmul_rn(sdiv<Form>(R_UNIV, sdiv<Form>(1.0, syw)), T));
+    } else {
+        double syw = Y[0] * C.d_mwk[0].r;
+#pragma unroll
+        for (int s = 1; s < NSP; s++) syw = fma(Y[s], C.d_mwk[s].r, syw);
+        if (syw > 1e-9 && T > 1.0) return sdiv<Form>(P_CONST, (R_UNIV * syw) * T);
+    }
     return fallback;
 }
 
@@ -172,7 +202,7 @@ __device__ __forceinline__ bool renormalise(double* Y, double least) {
 #pragma unroll
     for (int s = 0; s < NSP; s++) sy += Y[s];
     if (!(sy > least)) return false;
-    const double y = sdiv<Form>(1.0, sy);
+    const double y = srecip<Form>(sy);
 #pragma unroll
     for (int s = 0; s < NSP; s++) Y[s] = cquot(Y[s], sy, y);
     return true;
@@ -181,12 +211,6 @@ __device__ __forceinline__ bool renormalise(double* Y, double least) {
 __device__ __forceinline__ bool off_faces(const Consts& C, int i, int j, int k) {
     return i >= 1 && i < C.nx - 1 && j >= 1 && j < C.ny - 1 && k >= 1 && k < C.nz - 1;
 }
-
-// What the properties of a cell are kept in.
-template <typename R>
-struct CellProps {
-    R D[NSP], mu_mix, nu, aT, cp, lam, alpha;
-};
 
 // Cell-local mixture properties of one fluid cell (attr == 3), general path: any temperature, any
 // composition, any fits, by the reference's own rules term by term.  Called, not inlined: ordinary
@@ -606,7 +630,7 @@ __global__ void __launch_bounds__(NT)
                 for (int v = 0; v < V; v++) {
                     // FP64: (50 x + six neighbours) / 56 as x + (neighbours - 6 x) / 56: fewer roundings at
                     // the size of x, and a uniform field stays exactly what it is.  FP32: the sum
-                    // itself, in the reference's order, as the picks of the G equation (teno_picks)
+                    // itself, in the reference's order, as the picks of the G equation
                     // hang on its last bits.
                     const RI kl = v > 0 ? c[v > 0 ? v - 1 : 0] : left, kr = v < V - 1 ? c[v < V - 1 ? v + 1 : 0] : right;
                     const bool inner = a[v] == 3 && k + v >= 1 && k + v < nz - 1;
@@ -703,35 +727,42 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
         R num = R(0), div = R(0), nut = R(0), Smag = R(0);
         if (interior) {
             const int sI = ny * nz, sJ = nz;
-            const R* __restrict__ uf = F.p[0] + id;
-            const R* __restrict__ vf = F.p[1] + id;
-            const R* __restrict__ wf = F.p[2] + id;
-            const R du_dx = (uf[sI] - uf[-sI]) * K.d_2dx.r, dv_dy = (vf[sJ] - vf[-sJ]) * K.d_2dy.r;
-            const R dw_dz = (wf[1] - wf[-1]) * K.d_2dz.r, du_dy = (uf[sJ] - uf[-sJ]) * K.d_2dy.r;
-            const R du_dz = (uf[1] - uf[-1]) * K.d_2dz.r, dv_dx = (vf[sI] - vf[-sI]) * K.d_2dx.r;
-            const R dv_dz = (vf[1] - vf[-1]) * K.d_2dz.r, dw_dx = (wf[sI] - wf[-sI]) * K.d_2dx.r;
-            const R dw_dy = (wf[sJ] - wf[-sJ]) * K.d_2dy.r;
-            R S11 = du_dx, S22 = dv_dy, S33 = dw_dz;
-            R S12 = R(0.5) * (du_dy + dv_dx), S13 = R(0.5) * (du_dz + dw_dx), S23 = R(0.5) * (dv_dz + dw_dy);
-            const R off = fma(S23, S23, fma(S13, S13, S12 * S12));
-            const R Sij = fma(R(2.0), off, fma(S33, S33, fma(S22, S22, S11 * S11)));
-            Smag = qsqrt(R(2.0) * Sij);
-            div = du_dx + dv_dy + dw_dz;
-            R g = G;
-            if (g < R(0.0)) g = R(0.0);
-            if (g > R(1.0)) g = R(1.0);
-            R cs = fma(M.cs_b - M.cs_u, g, M.cs_u);
-            cs = fma(M.cs_boost * R(4.0) * g, R(1.0) - g, cs);
-            const R dx = (R)K.dx;
-            nut = (cs * dx) * (cs * dx) * Smag;
-            num = fma(-div * div, R(1.0 / 3.0), Sij);
+            if constexpr (std::is_same<R, float>::value) {
+                f32_strain(K, M, F, id, sI, sJ, G, Smag, nut, div, num);
+            } else {
+                const R* __restrict__ uf = F.p[0] + id;
+                const R* __restrict__ vf = F.p[1] + id;
+                const R* __restrict__ wf = F.p[2] + id;
+                const R du_dx = (uf[sI] - uf[-sI]) * K.d_2dx.r, dv_dy = (vf[sJ] - vf[-sJ]) * K.d_2dy.r;
+                const R dw_dz = (wf[1] - wf[-1]) * K.d_2dz.r, du_dy = (uf[sJ] - uf[-sJ]) * K.d_2dy.r;
+                const R du_dz = (uf[1] - uf[-1]) * K.d_2dz.r, dv_dx = (vf[sI] - vf[-sI]) * K.d_2dx.r;
+                const R dv_dz = (vf[1] - vf[-1]) * K.d_2dz.r, dw_dx = (wf[sI] - wf[-sI]) * K.d_2dx.r;
+                const R dw_dy = (wf[sJ] - wf[-sJ]) * K.d_2dy.r;
+                R S11 = du_dx, S22 = dv_dy, S33 = dw_dz;
+                R S12 = R(0.5) * (du_dy + dv_dx), S13 = R(0.5) * (du_dz + dw_dx), S23 = R(0.5) * (dv_dz + dw_dy);
+                const R off = fma(S23, S23, fma(S13, S13, S12 * S12));
+                const R Sij = fma(R(2.0), off, fma(S33, S33, fma(S22, S22, S11 * S11)));
+                Smag = qsqrt(R(2.0) * Sij);
+                div = du_dx + dv_dy + dw_dz;
+                R g = G;
+                if (g < R(0.0)) g = R(0.0);
+                if (g > R(1.0)) g = R(1.0);
+                R cs = fma(M.cs_b - M.cs_u, g, M.cs_u);
+                cs = fma(M.cs_boost * R(4.0) * g, R(1.0) - g, cs);
+                const R dx = (R)K.dx;
+                nut = (cs * dx) * (cs * dx) * Smag;
+                num = fma(-div * div, R(1.0 / 3.0), Sij);
+            }
         }
         CellProps<R> o;
         auto store_d = [&](const R* D) {
 #pragma unroll
             for (int s = 0; s < NSP; s++) P.D[s][id] = D[s];
         };
-        if (!cell_props_fast<R>(C, tab, T, Y, rho, store_d, o)) {
+        bool ordinary;
+        if constexpr (std::is_same<R, float>::value) ordinary = f32_cell_props(C, T, Y, rho, store_d, o);
+        else ordinary = cell_props_fast(C, tab, T, Y, rho, store_d, o);
+        if (!ordinary) {
             CellProps<R> g;
             R Yf[NSP];
 #pragma unroll
@@ -752,7 +783,9 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::props, NTB))
         }
         if (P.dbg_cp) { P.dbg_cp[id] = o.cp; P.dbg_lam[id] = o.lam; P.dbg_alpha[id] = o.alpha; }
         R ST = R(0);
-        if (interior) {
+        if constexpr (std::is_same<R, float>::value) {
+            if (interior) ST = f32_flame_speed(K, num, div, o.nu);
+        } else if (interior) {
             const R dx = (R)K.dx, nul = o.nu;
             // SSR-SGS turbulent flame speed (:1926-1957)
             const R X = (R)K.dx4 * num * frcp(nul * nul);
@@ -831,31 +864,6 @@ __device__ __forceinline__ R teno_faces(R f1, R f2, R f3, R f4, R f5) {
     return fma(p - m, R(1.0 / 6.0), f3);
 }
 
-// The same from the six values v0..v5 for FP32.  Which candidates count is decided by comparing
-// smoothness with a fixed number, and a candidate more or less moves a cell at a front by 1e-3 of G in a few
-// steps.  The smoothness is therefore taken from the values in the reference's order, so that runs of the
-// FP32 form that differ only in how they round elsewhere decide alike (six 128x64x64 members, 32 steps:
-// two forms of the other passes apart by up to 1.3e-3 of G with the smoothness in differences, by 1e-4 so);
-// the candidates themselves are in differences.  FP32 flow pass 0.725 -> 0.743 ms per 256x128x128 step.
-__device__ __forceinline__ void teno_picks(float v0, float v1, float v2, float v3, float v4, float& is0, float& is1,
-                                           float& is2) {
-    const float a0 = v0 - 2.0f * v1 + v2, b0 = v0 - 4.0f * v1 + 3.0f * v2;
-    const float a1 = v1 - 2.0f * v2 + v3, b1 = v1 - v3;
-    const float a2 = v2 - 2.0f * v3 + v4, b2 = 3.0f * v2 - 4.0f * v3 + v4;
-    is0 = float(13.0 / 12.0) * (a0 * a0) + 0.25f * (b0 * b0);
-    is1 = float(13.0 / 12.0) * (a1 * a1) + 0.25f * (b1 * b1);
-    is2 = float(13.0 / 12.0) * (a2 * a2) + 0.25f * (b2 * b2);
-}
-__device__ __forceinline__ float teno_faces(float v0, float v1, float v2, float v3, float v4, float v5) {
-    const float f1 = v1 - v0, f2 = v2 - v1, f3 = v3 - v2, f4 = v4 - v3, f5 = v5 - v4;
-    float i0, i1, i2;
-    teno_picks(v0, v1, v2, v3, v4, i0, i1, i2);
-    const float m = teno_pick<float>(i0, i1, i2, fmaf(5.0f, f2, -2.0f * f1), fmaf(2.0f, f3, f2), fmaf(4.0f, f3, -f4));
-    teno_picks(v1, v2, v3, v4, v5, i0, i1, i2);
-    const float p = teno_pick<float>(i0, i1, i2, fmaf(5.0f, f3, -2.0f * f2), fmaf(2.0f, f4, f3), fmaf(4.0f, f4, -f5));
-    return fmaf(p - m, float(1.0 / 6.0), f3);
-}
-
 // The WENO5 gradient (:735-827, on the cells -2..+3 whatever the velocity) times the spacing, e1..e5 the
 // differences of its six values.  The weights gamma_k / (eps + IS_k)^2 are brought to one
 // denominator: one reciprocal per half instead of three quotients and three shares of their sum.
@@ -893,14 +901,6 @@ __device__ __forceinline__ double half_slope(double a, double b) {
     double x = fabs(lo) >= fabs(hh) ? hh : lo;
     x = (a * b <= 0.0) ? 0.0 : x;
     return fabs(b) < SMALL ? b : x;
-}
-// FP32 has minima and maxima as instructions: with a' = a sign(b), the same value is
-// sign(b) max(0, min(a', max(|b|/2, min(a'/2, |b|)))).
-__device__ __forceinline__ float half_slope(float a, float b) {
-    const unsigned sb = __float_as_uint(b) & 0x80000000u;
-    const float m = __uint_as_float(__float_as_uint(a) ^ sb), n = fabsf(b);
-    const float x = fmaxf(0.0f, fminf(m, fmaxf(0.5f * n, fminf(0.5f * m, n))));
-    return n < (float)SMALL ? b : __uint_as_float(__float_as_uint(x) ^ sb);
 }
 
 // One field around a cell, along each axis in the direction of the velocity there: the cell, its
@@ -1062,39 +1062,73 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
     if (g > R(1.0)) g = R(1.0);
     const bool pos[3] = {vel[0] >= R(0.0), vel[1] >= R(0.0), vel[2] >= R(0.0)};
     src.orient(pos, !band2);
-    const R ih2[3] = {K.d_dxx.r, K.d_dyy.r, K.d_dzz.r};
-    StarCoef<R> co;
-    co.lim = band2 ? R(0.0) : R(1.0);
-    co.av[0] = fabs(vel[0]) * K.d_dx.r;
-    co.av[1] = fabs(vel[1]) * K.d_dy.r;
-    co.av[2] = fabs(vel[2]) * K.d_dz.r;
-    {
-        R n0, nu[3], nd[3];
+    // the targets of the nudging
+    const R Tt = fma(g, (R)K.t_burnt_span, (R)K.t_in);
+    auto target = [&](int s) {
+        auto line = [&](R y, R slope) {
+            if constexpr (std::is_same<R, float>::value) return fma(slope, g, y);
+            else return y + slope * g;
+        };
+        if (s == C3H8) return (R)K.inletYk[C3H8] * (R(1.0) - g);
+        if (s == O2) return fmax(R(0.0), line((R)K.inletYk[O2], -(R)K.cons_o2));
+        if (s == CO2) return line((R)K.inletYk[CO2], (R)K.prod_co2);
+        if (s == H2O) return line((R)K.inletYk[H2O], (R)K.prod_h2o);
+        return (R)K.inletYk[N2];
+    };
+    if constexpr (std::is_same<R, float>::value) {
+        float n0, nu[3], nd[3];
         src.nu(n0, nu, nd);
+        Fl sp[3], sm[3], gp[3], gm[3];
 #pragma unroll
         for (int q = 0; q < 3; q++) {
-            const R c = K.d_sct2.r * ih2[q];
-            co.gu[q] = (nu[q] + n0) * c;
-            co.gd[q] = (nd[q] + n0) * c;
+            sp[q] = Fl(pos[q] ? nd[q] : nu[q]) + Fl(n0);
+            sm[q] = Fl(pos[q] ? nu[q] : nd[q]) + Fl(n0);
+            gp[q] = sp[q] * Fl(K.d_prt2.r);
+            gm[q] = sm[q] * Fl(K.d_prt2.r);
         }
-    }
-    {
-        Star<R> q;
+        Star<float> q;
         src.t(q);
-        const R Tt = fma(g, (R)K.t_burnt_span, (R)K.t_in);
-        kv[0] = star_rhs<R, false>(q, co, K.d_sct2.c * K.d_prt2.r, ld_stream(P.aT + id), ih2, relax * (Tt - q.c));
-    }
+        kv[0] = f32_scalar_rhs<true>(K, q, pos, band2, vel, gp, gm, ld_stream(P.aT + id), relax, Tt, 1.0f);
 #pragma unroll
-    for (int s = 0; s < NSP; s++) {
-        R tgt;
-        if (s == C3H8) tgt = (R)K.inletYk[C3H8] * (R(1.0) - g);
-        else if (s == O2) tgt = fmax(R(0.0), (R)K.inletYk[O2] - (R)K.cons_o2 * g);
-        else if (s == CO2) tgt = (R)K.inletYk[CO2] + (R)K.prod_co2 * g;
-        else if (s == H2O) tgt = (R)K.inletYk[H2O] + (R)K.prod_h2o * g;
-        else tgt = (R)K.inletYk[N2];
-        Star<R> q;
-        src.y(s, q);
-        kv[1 + s] = star_rhs<R, true>(q, co, R(1.0), ld_stream(P.D[s] + id), ih2, relax * (tgt - q.c));
+        for (int a = 0; a < 3; a++) {
+            gp[a] = sp[a] * Fl(K.d_sct2.r);
+            gm[a] = sm[a] * Fl(K.d_sct2.r);
+        }
+#pragma unroll
+        for (int s = 0; s < NSP; s++) {
+            src.y(s, q);
+            const Fl D = ld_stream(P.D[s] + id);
+            if (s == C3H8) kv[1] = f32_scalar_rhs<true>(K, q, pos, band2, vel, gp, gm, D, relax, K.inletYk[s], 1.0f - g);
+            else kv[1 + s] = f32_scalar_rhs<false>(K, q, pos, band2, vel, gp, gm, D, relax, target(s), 1.0f);
+        }
+    } else {
+        const R ih2[3] = {K.d_dxx.r, K.d_dyy.r, K.d_dzz.r};
+        StarCoef<R> co;
+        co.lim = band2 ? R(0.0) : R(1.0);
+        co.av[0] = fabs(vel[0]) * K.d_dx.r;
+        co.av[1] = fabs(vel[1]) * K.d_dy.r;
+        co.av[2] = fabs(vel[2]) * K.d_dz.r;
+        {
+            R n0, nu[3], nd[3];
+            src.nu(n0, nu, nd);
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const R c = K.d_sct2.r * ih2[q];
+                co.gu[q] = (nu[q] + n0) * c;
+                co.gd[q] = (nd[q] + n0) * c;
+            }
+        }
+        {
+            Star<R> q;
+            src.t(q);
+            kv[0] = star_rhs<R, false>(q, co, K.d_sct2.c * K.d_prt2.r, ld_stream(P.aT + id), ih2, relax * (Tt - q.c));
+        }
+#pragma unroll
+        for (int s = 0; s < NSP; s++) {
+            Star<R> q;
+            src.y(s, q);
+            kv[1 + s] = star_rhs<R, true>(q, co, R(1.0), ld_stream(P.D[s] + id), ih2, relax * (target(s) - q.c));
+        }
     }
     // ---- RK4 bookkeeping.  acc holds k1, k1 + 2k2, (k1 + 2k2) + 2k3: exactly the
     // left-to-right partial sums of k1 + 2.0*k2 + 2.0*k3 + k4 (:4520).  All loads come before the
@@ -1219,16 +1253,6 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
 // Everything is in differences across the six faces: a conservative flux m p with the face
 // value p = p0 + d/2 (first-order upwind next to the boundary: p0 or p0 + d by the sign of m),
 // so convection and diffusion of all three components are two coefficients a face.
-// What the flow pass loads of a cell before it knows its attribute.
-template <typename R>
-struct FlowCell {
-    R p0[3], r0, G0, n0, mu;
-    __device__ __forceinline__ void load(const F11<R>& F, const PropBuf<R>& P, int id) {
-        p0[0] = F.p[0][id]; p0[1] = F.p[1][id]; p0[2] = F.p[2][id];
-        r0 = F.p[5][id]; G0 = F.p[4][id]; n0 = P.nu_t[id]; mu = P.mu_eff[id];
-    }
-};
-
 // The right-hand sides of rho u, rho v, rho w and G of one fluid cell.
 template <typename R>
 __device__ __forceinline__ void flow_rhs(const Consts& C, const ModelK<R>& M, const F11<R>& F, const PropBuf<R>& P,
@@ -1282,8 +1306,7 @@ __device__ __forceinline__ void flow_rhs(const Consts& C, const ModelK<R>& M, co
             R d = f3;                                   // first-order upwind (:642-651)
             if (!band3) {
                 const R UU = G[id + 2 * o], U3 = G[id + 3 * o], DD = G[id - 2 * o];
-                if constexpr (std::is_same<R, float>::value) d = teno_faces(U3, UU, U, G0, Dn, DD);
-                else d = teno_faces<R>(UU - U3, U - UU, f3, f4, DD - Dn);
+                d = teno_faces<R>(UU - U3, U - UU, f3, f4, DD - Dn);
             } else if (!band2) {
                 // central faces (:652-677): the zero UW2 coefficient makes both upwind branches identical
                 d = R(0.5) * (f3 + f4);
@@ -1369,14 +1392,16 @@ __device__ __forceinline__ void flow_update(const F11<RS>& S0, const F11<R>& St,
     const RS rho = PART == RK_LAST ? fabs(left) : left;
     const double dt = Sc->dt;
     const RS cdt = PART == RK_LAST ? (RS)(dt / 6.0) : (RS)((PART == RK_MIDDLE && stage == 2 ? 1.0 : 0.5) * dt);
-    const RS irho = sdiv<R>(RS(1.0), rho);
+    const RS irho = srecip<R>(rho);
     RS out[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         const R incr = PART == RK_LAST ? ac[q] + kv[q] : kv[q];
         ac[q] = PART == RK_FIRST ? kv[q] : fma(R(2.0), kv[q], ac[q]);
         if (q < 3) {
-            const RS m = fma(cdt, (RS)incr, rho_n * sn[q]);             // rhou = rho*u after the BC (:3146)
+            // rhou = rho*u after the BC (:3146); the FP32 form has always rounded the other product
+            const RS m = std::is_same<R, float>::value ? fma(rho_n, sn[q], __dmul_rn(cdt, (RS)incr))
+                                                       : fma(cdt, (RS)incr, rho_n * sn[q]);
             out[q] = rho > RS(SMALL) ? cquot(m, rho, irho) : RS(0);
         } else {
             out[q] = fmax(RS(0.0), fmin(RS(1.0), fma(cdt, (RS)incr, sn[q])));
@@ -1443,7 +1468,8 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::flow, NTB))
         return;
     }
     R kv[4];
-    flow_rhs<R>(C, M, F, P, Sc, i, j, k, id, c, kv);
+    if constexpr (std::is_same<R, float>::value) f32_flow_rhs(C, M, F, P, Sc, i, j, k, id, c, kv);
+    else flow_rhs<R>(C, M, F, P, Sc, i, j, k, id, c, kv);
     flow_update<PART, R, RS>(S0, St, acc, kd, Sc, stage, id, kv, ld_stream(rn + id));
 }
 
@@ -1478,7 +1504,10 @@ __global__ void __launch_bounds__(2 * NT, 2)
         FlowCell<R> c;
         c.load(F, P, id);
         R kv[4];
-        if (a == 3) flow_rhs<R>(C, model_of<R>(C), F, P, Sc, i, j, k, id, c, kv);
+        if (a == 3) {
+            if constexpr (std::is_same<R, float>::value) f32_flow_rhs(C, model_of<R>(C), F, P, Sc, i, j, k, id, c, kv);
+            else flow_rhs<R>(C, model_of<R>(C), F, P, Sc, i, j, k, id, c, kv);
+        }
         __syncwarp();
         asm volatile("barrier.cta.sync 1, 512;" ::: "memory");
         if (a == 3) flow_update<PART, R, RS>(S0, St, acc, kd, Sc, stage, id, kv, rn[t]);
