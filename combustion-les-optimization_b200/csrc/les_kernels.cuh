@@ -211,6 +211,10 @@ __device__ __forceinline__ bool renormalise(double* Y, double least) {
 __device__ __forceinline__ bool off_faces(const Consts& C, int i, int j, int k) {
     return i >= 1 && i < C.nx - 1 && j >= 1 && j < C.ny - 1 && k >= 1 && k < C.nz - 1;
 }
+// A cell of a face or the one next to it, which the boundary conditions copy.
+__device__ __forceinline__ bool beside_face(const Consts& C, int i, int j, int k) {
+    return i < 2 || i >= C.nx - 2 || j < 2 || j >= C.ny - 2 || k < 2 || k >= C.nz - 2;
+}
 
 // Cell-local mixture properties of one fluid cell (attr == 3), general path: any temperature, any
 // composition, any fits, by the reference's own rules term by term.  Called, not inlined: ordinary
@@ -1043,7 +1047,7 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
             if (a == 2) St.p[5][id] = R(r);
         } else if (PART == RK_LAST && off_faces(C, i, j, k)) {
             hand(eos_rho_state<R>(C, T0, Y0, RS(1.2)));
-            if ((a == 2 || a == 5) && renormalise<R>(Y0, RS(1e-6))) {
+            if ((a == 2 || a == 5) && !beside_face(C, i, j, k) && renormalise<R>(Y0, RS(1e-6))) {
 #pragma unroll
                 for (int s = 0; s < NSP; s++) S0.p[6 + s][id] = Y0[s];
             }
@@ -1163,7 +1167,7 @@ __device__ __forceinline__ void rhs_scalar_cell(const Consts& C, const uint8_t* 
         // where there is none, which the sign bit tells the flow pass, of zero and NaN too) and
         // renormalises once more
         if (rho == RS(0.0)) rho = -fabs(rho_n);
-        renormalise<R>(up + 1, RS(1e-6));
+        if (!band2) renormalise<R>(up + 1, RS(1e-6));   // k_bc: beside a face, after the copies
     }
     if (kd.p[0]) {
 #pragma unroll
@@ -1518,9 +1522,11 @@ __global__ void __launch_bounds__(2 * NT, 2)
 // ------------------------------------------------------------------ boundary conditions
 // apply_boundary_conditions (:2967-3161): the i-faces (with the SEM + white-noise inflow), then for
 // every interior i the j-faces, then the k-faces, then the equation of state and mass-fraction
-// renormalisation.  Only the cells of the six faces change: the last stage's scalar and flow passes
-// leave every other cell as the reference's EOS sweep over the grid does, and take the maximum
-// of |u| over fluid cells, so no pass over the whole grid is needed here.
+// renormalisation.  Only the cells of the six faces and, in their mass fractions, the cells next to
+// them change: the last stage's scalar and flow passes leave every other cell as the reference's EOS
+// sweep over the grid does, and take the maximum of |u| over fluid cells, so no pass over the whole
+// grid is needed here.  The cells next to a face are renormalised for the second time here, as the
+// copies take their mass fractions before the sweep.
 
 template <typename R>
 __device__ __forceinline__ void copy_cell(F11<R>& S, size_t dst, size_t src) {
@@ -1595,6 +1601,19 @@ __device__ __forceinline__ void bc_eos_cell(const Consts& C, const uint8_t* __re
     if (a == 1 || a == 3) max_into(&Sc->umax, sqrt(u * u + v * v + w * w));
 }
 
+// The second renormalisation (:3150-3159) of a cell next to a face.
+template <typename R, typename Form>
+__device__ __forceinline__ void bc_renormalise(const uint8_t* __restrict__ attr, F11<R>& S, size_t id) {
+    const int a = attr[id];
+    R Y[NSP];
+#pragma unroll
+    for (int s = 0; s < NSP; s++) Y[s] = S.p[6 + s][id];
+    if ((a == 3 || a == 2 || a == 5) && renormalise<Form>(Y, R(1e-6))) {
+#pragma unroll
+        for (int s = 0; s < NSP; s++) S.p[6 + s][id] = Y[s];
+    }
+}
+
 // The q-th of the 2 (ny + nz) - 4 cells around a plane.
 __device__ __forceinline__ void ring_cell(int q, int ny, int nz, int& j, int& k) {
     if (q < 2 * nz) {
@@ -1609,15 +1628,16 @@ __device__ __forceinline__ void ring_cell(int q, int ny, int nz, int& j, int& k)
 
 // One launch for all of it.  Block b < nx - 2 takes the faces around plane i = b + 1 in the
 // reference's order, its own barriers between the steps; the blocks of the second and the last
-// but one plane also take the cells around planes 0 and nx - 1 first, which copy cells that the
-// j- and k-faces then overwrite.  The remaining blocks take the inner cells of planes 0 and
-// nx - 1, which copy cells that nothing here writes.
+// but one plane also take, first, the two outermost rings of planes 0 and nx - 1, which copy cells
+// that the j- and k-faces then overwrite or copy too.  The remaining blocks take the other cells of planes
+// 0 and nx - 1, each the only reader of the cell it copies.  A block writes to a cell next to a
+// face only after the last copy of it, which is always its own.
 template <typename R, typename Form = R>
 __global__ void __launch_bounds__(NT) k_bc(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> S,
                                            const double* __restrict__ plane, const double* __restrict__ noise,
                                            const int* __restrict__ inlet_pos, Scalars* __restrict__ Sc) {
     const int nx = C.nx, ny = C.ny, nz = C.nz, tid = threadIdx.x;
-    const int ring = 2 * (ny + nz) - 4;
+    const int ring = 2 * (ny + nz) - 4, rings = 2 * ring - 8;
     int j, k;
     pdl_wait();
     if ((int)blockIdx.x >= nx - 2) {
@@ -1625,16 +1645,28 @@ __global__ void __launch_bounds__(NT) k_bc(LES_KERNEL_CONSTS, const uint8_t* __r
         if (q >= (ny - 2) * (nz - 2)) return;
         j = 1 + q / (nz - 2);
         k = 1 + q % (nz - 2);
+        if (j == 1 || j == ny - 2 || k == 1 || k == nz - 2) return;
         bc_first_plane<R>(C, attr, S, plane, noise, inlet_pos, j, k);
         bc_last_plane<R>(C, attr, S, j, k);
         bc_eos_cell<R, Form>(C, attr, S, cid(0, j, k, ny, nz), Sc);
         bc_eos_cell<R, Form>(C, attr, S, cid(nx - 1, j, k, ny, nz), Sc);
+        bc_renormalise<R, Form>(attr, S, cid(1, j, k, ny, nz));
+        bc_renormalise<R, Form>(attr, S, cid(nx - 2, j, k, ny, nz));
         return;
     }
     const int i = (int)blockIdx.x + 1;
-    if (i == 1 || i == nx - 2) {
-        for (int q = tid; q < ring; q += NT) {
+    auto cell = [&](int q) {                        // of the outermost ring, then of the one inside it
+        if (q < ring) {
             ring_cell(q, ny, nz, j, k);
+        } else {
+            ring_cell(q - ring, ny - 2, nz - 2, j, k);
+            j++;
+            k++;
+        }
+    };
+    if (i == 1 || i == nx - 2) {
+        for (int q = tid; q < rings; q += NT) {
+            cell(q);
             if (i == 1) bc_first_plane<R>(C, attr, S, plane, noise, inlet_pos, j, k);
             else bc_last_plane<R>(C, attr, S, j, k);
         }
@@ -1666,9 +1698,10 @@ __global__ void __launch_bounds__(NT) k_bc(LES_KERNEL_CONSTS, const uint8_t* __r
         }
     }
     __syncthreads();
-    for (int q = tid; q < ring; q += NT) {
-        ring_cell(q, ny, nz, j, k);
-        bc_eos_cell<R, Form>(C, attr, S, cid(i, j, k, ny, nz), Sc);
+    for (int q = tid; q < rings; q += NT) {
+        cell(q);
+        if (q < ring) bc_eos_cell<R, Form>(C, attr, S, cid(i, j, k, ny, nz), Sc);
+        else bc_renormalise<R, Form>(attr, S, cid(i, j, k, ny, nz));
         if (i == 1) bc_eos_cell<R, Form>(C, attr, S, cid(0, j, k, ny, nz), Sc);
         if (i == nx - 2) bc_eos_cell<R, Form>(C, attr, S, cid(nx - 1, j, k, ny, nz), Sc);
     }

@@ -145,3 +145,34 @@ def test_density_of_cells_without_mass_fractions(N, oracle_mod, rho):
     np.testing.assert_allclose(got, want, rtol=1e-10)
     sol.close()
     orc.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(4, 4, 4), (5, 6, 7), (33, 7, 6), (12, 9, 40)])
+def test_faces_copy_mass_fractions_before_they_are_renormalised(N, nx, ny, nz):
+    """Open faces copy a cell's mass fractions as the last stage leaves them, and the sweep after the
+    boundary conditions divides the cell's own by their sum: an outflow cell of the k-faces, divided by
+    its sum, is its neighbour to the last bit."""
+    cfg = _grid(nx, ny, nz)
+    s = N.Solver(cfg)
+    st = s.state()
+    rng = np.random.default_rng(2)
+    for f, a in (("u", 3.0), ("v", 1.0), ("w", 4.0)):
+        st[f] = a * rng.standard_normal(st[f].shape)
+    y = rng.uniform(0.02, 1.0, (5,) + st["u"].shape)
+    for k in range(5):
+        st[f"Y{k}"] = y[k] / y.sum(0)
+    s.ctx.upload_state(st)
+    s.step(1)
+    st = s.state()
+    attr = s.attribute()
+    n = 0
+    for face, near, out in ((0, 1, st["w"][:, :, 1] <= 0), (nz - 1, nz - 2, st["w"][:, :, nz - 2] >= 0)):
+        m = out & (attr[:, :, face] == 4) & (attr[:, :, near] == 3)
+        m[[0, -1]] = m[:, [0, -1]] = False
+        Y = [st[f"Y{k}"][:, :, face][m] for k in range(5)]
+        total = (((Y[0] + Y[1]) + Y[2]) + Y[3]) + Y[4]
+        for k in range(5):
+            np.testing.assert_array_equal(Y[k] / total, st[f"Y{k}"][:, :, near][m])
+        n += int(m.sum())
+    assert n > 0
+    s.close()
