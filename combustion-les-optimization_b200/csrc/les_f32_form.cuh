@@ -175,6 +175,7 @@ __device__ __forceinline__ float f32_flame_speed(const ConstsF& K, float num, fl
 // two downstream (mirrored for a negative velocity the reference's two branches are this one): the
 // difference of the reconstructed values.  The faces share the second differences and one candidate.
 __device__ __forceinline__ Fl f32_smooth(Fl aa, Fl b) { return Fl(float(13.0 / 12.0)) * aa + Fl(0.25f) * (b * b); }
+__device__ __forceinline__ Fl f32_smooth_fused(Fl aa, Fl b) { return mad(float(13.0 / 12.0), aa, Fl(0.25f) * (b * b)); }
 __device__ __forceinline__ Fl f32_teno_face(Fl i0, Fl i1, Fl i2, Fl p0, Fl p1, Fl p2, Fl p0_alone) {
     const float cut = (float)TENO_CUT;
     const bool d0 = i0 < cut, d1 = i1 < cut, d2 = i2 < cut;
@@ -185,6 +186,7 @@ __device__ __forceinline__ Fl f32_teno_face(Fl i0, Fl i1, Fl i2, Fl p0, Fl p1, F
     const Fl best = (i0 <= i1 && i0 <= i2) ? p0_alone : ((i1 <= i0 && i1 <= i2) ? p1 : p2);
     return (d0 || d1 || d2) ? mad(w2, p2, mad(w0, p0, w1 * p1)) * r : best;
 }
+// Smoothness ties decide as well: the outermost stencil's sum of each face ends in a fused multiply-add.
 // Which products of the candidates are rounded before they are added depends on the face, the axis and the sign of
 // the velocity, for the first candidate also on whether it is weighted or taken alone.
 template <int AXIS>
@@ -196,14 +198,14 @@ __device__ __forceinline__ Fl f32_teno_diff(bool pos, Fl v0, Fl v1, Fl v2, Fl v3
     const Fl m0 = mad(11.0f, v2, mad(two, v0, -(Fl(7.0f) * v1))) * r6;
     const Fl m1 = (mad(5.0f, v2, -v1) + two * v3) * r6;
     const Fl m2 = ((pos ? two * v2 + Fl(5.0f) * v3 : mad(5.0f, v3, two * v2)) - v4) * r6;
-    const Fl m = f32_teno_face(f32_smooth(t1, v0 - four * v1 + m3), f32_smooth(t2, v1 - v3),
+    const Fl m = f32_teno_face(f32_smooth_fused(t1, v0 - four * v1 + m3), f32_smooth(t2, v1 - v3),
                                f32_smooth(t3, m3 - four * v3 + v4), m0, m1, m2, m0);
     const Fl p0a = mad(11.0f, v3, mad(-7.0f, v2, two * v1)) * r6;
     const Fl p0 = AXIS == 2 ? mad(11.0f, v3, mad(two, v1, -(Fl(7.0f) * v2))) * r6 : p0a;
     const Fl p1 = ((AXIS == 0 && pos ? Fl(5.0f) * v3 - v2 : mad(5.0f, v3, -v2)) + two * v4) * r6;
     const Fl p2 = (mad(5.0f, v4, two * v3) - v5) * r6;
     const Fl p = f32_teno_face(f32_smooth(t2, v1 - four * v2 + p3), f32_smooth(t3, v2 - v4),
-                               f32_smooth(t4, p3 - four * v4 + v5), p0, p1, p2, p0a);
+                               f32_smooth_fused(t4, p3 - four * v4 + v5), p0, p1, p2, p0a);
     return p - m;
 }
 
@@ -216,19 +218,18 @@ __device__ __forceinline__ Fl f32_weno_half(Fl i0, Fl i1, Fl i2, Fl g0, Fl g1, F
     return sum3(a0 * y, s0, a1 * y, s1, a2 * y, s2);
 }
 __device__ __forceinline__ Fl f32_weno_diff(Fl p0, Fl p1, Fl p2, Fl p3, Fl p4, Fl p5) {
-    const Fl r6 = float(1.0 / 6.0), two = 2.0f, four = 4.0f, c = float(13.0 / 12.0);
+    const Fl r6 = float(1.0 / 6.0), two = 2.0f, four = 4.0f;
     const Fl a1 = p0 - two * p1 + p2, a2 = p1 - two * p2 + p3, a3 = p2 - two * p3 + p4, a4 = p3 - two * p4 + p5;
     const Fl m3 = Fl(3.0f) * p2, h3 = Fl(3.0f) * p3;
-    auto fused = [&](Fl a, Fl b) { return mad(c, a * a, Fl(0.25f) * (b * b)); };
     const Fl s0 = mad(11.0f, p3, mad(-7.0f, p2, two * p1)) * r6;
     const Fl s1 = (mad(5.0f, p3, -p2) + two * p4) * r6;
     const Fl s2 = (mad(5.0f, p4, two * p3) - p5) * r6;
     const Fl h = f32_weno_half(f32_smooth(a2 * a2, p1 - four * p2 + h3), f32_smooth(a3 * a3, p2 - p4),
-                               fused(a4, h3 - four * p4 + p5), 3.0f / 10.0f, 6.0f / 10.0f, 1.0f / 10.0f, s0, s1, s2);
+                               f32_smooth_fused(a4 * a4, h3 - four * p4 + p5), 3.0f / 10.0f, 6.0f / 10.0f, 1.0f / 10.0f, s0, s1, s2);
     const Fl m0 = (mad(5.0f, p1, -p0) + two * p2) * r6;
     const Fl m1 = (mad(5.0f, p2, two * p1) - p3) * r6;
     const Fl m2 = (mad(-7.0f, p3, Fl(11.0f) * p2) + two * p4) * r6;
-    const Fl l = f32_weno_half(fused(a1, p0 - four * p1 + m3), f32_smooth(a2 * a2, p1 - p3), fused(a3, m3 - four * p3 + p4),
+    const Fl l = f32_weno_half(f32_smooth_fused(a1 * a1, p0 - four * p1 + m3), f32_smooth(a2 * a2, p1 - p3), f32_smooth_fused(a3 * a3, m3 - four * p3 + p4),
                                1.0f / 10.0f, 6.0f / 10.0f, 3.0f / 10.0f, m0, m1, m2);
     return h - l;
 }

@@ -14,7 +14,7 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, os.path.join(os.path.dirname(os.path.dirname(HERE)), "combustion-les-optimization_b200"))
 
-CASES = {"early": (22, 13, 17, 0), "late": (24, 12, 16, 600)}
+CASES = {"early": (22, 13, 17, 0), "late": (24, 12, 16, 600), "ties": (20, 14, 18, 0)}
 STEPS = 12
 
 
@@ -24,13 +24,16 @@ def config(nx, ny, nz):
                                   initial_flame_front_i=nx // 3, inlet_radius=0.001 * ny, seed=11)
 
 
-def state(nx, ny, nz):
+def state(nx, ny, nz, spikes=False):
     """A front through a swirling flow, formed with additions, products and quotients only, so that it
-    is the same to the last bit everywhere."""
+    is the same to the last bit everywhere; with `spikes`, single cells off a level G, whose stencils tie."""
     x, y, z = (np.arange(n).reshape([-1 if q == d else 1 for q in range(3)]) / n for d, n in enumerate((nx, ny, nz)))
     z = z - 0.5
     r = 9.0 * (y - 0.35 + 0.3 * x * x + 0.4 * z * z - 0.5 * x * z) + 0.0 * (x + y + z)
     g = np.clip(0.5 + 0.65 * r / (1.0 + np.abs(r)), 0.0, 1.0)
+    if spikes:
+        i, j, k = np.meshgrid(np.arange(nx), np.arange(ny), np.arange(nz), indexing="ij")
+        g = 0.5 + np.where((i % 5 == 2) & (j % 5 == 2) & (k % 5 == 2), ((7 * i + 3 * j + 5 * k) % 13 - 6) / 256.0, 0.0)
     st = {"u": 14.0 * (1.0 - 1.6 * y) + 20.0 * z * (x - 0.4), "v": 9.0 * (z * 2.0 - y + 0.3) * (1.2 - x),
           "w": 11.0 * (0.4 - y - z * x), "G": g, "T": 300.0 + 1900.0 * g}
     ys = [0.06 * (1.0 - g), 0.22 - 0.215 * g, 0.72 + 0.0 * g, 0.175 * g, 0.095 * g]
@@ -47,7 +50,7 @@ def main():
     out = {}
     for name, (nx, ny, nz, start) in CASES.items():
         s = N.Solver(config(nx, ny, nz), precision=N.FP32, start_step=start)
-        s.ctx.upload_state(state(nx, ny, nz))
+        s.ctx.upload_state(state(nx, ny, nz, name == "ties"))
         s.run(STEPS)
         for f, v in s.state().items():
             out[f"{name}_{f}"] = v.astype(np.float32)

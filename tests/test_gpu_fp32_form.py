@@ -18,10 +18,10 @@ def N(lesgpu_native, cuda_device):
     return lesgpu_native
 
 
-def _solver(N, case, precision=None):
+def _solver(N, case):
     nx, ny, nz, start = M.CASES[case]
-    s = N.Solver(M.config(nx, ny, nz), precision=N.FP32 if precision is None else precision, start_step=start)
-    s.ctx.upload_state(M.state(nx, ny, nz))
+    s = N.Solver(M.config(nx, ny, nz), precision=N.FP32, start_step=start)
+    s.ctx.upload_state(M.state(nx, ny, nz, case == "ties"))
     return s
 
 
