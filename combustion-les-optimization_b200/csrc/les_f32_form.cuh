@@ -155,12 +155,12 @@ __device__ __forceinline__ void f32_strain(const ConstsF& K, const ModelK<float>
 // whatever its value, and the exponential and the power are left out.
 __device__ __forceinline__ float f32_flame_speed(const ConstsF& K, float num, float div, float nu) {
     const Fl dx = K.dx, X = over(K.dx4, Fl(nu) * Fl(nu)) * Fl(num);
-    Fl d_eta = 1.0f;
+    Fl d_eta = Fl(1.0f) + Fl((float)SMALL);      // D / eta + SMALL
     if (!(X < Fl((float)SMALL))) {
         const Fl pX = qpow(X.v, 0.75f), arg = Fl((float)SSR_B) * pX;
-        d_eta = Fl((float)SSR_A) * pX * Fl(arg > Fl(1.0f) ? qlog(arg.v) : 0.0f);
+        d_eta = mad(Fl((float)SSR_A) * pX, arg > Fl(1.0f) ? qlog(arg.v) : 0.0f, (float)SMALL);
     }
-    const Fl eta = over(dx, d_eta + Fl((float)SMALL)), dce = Fl(8.0f) * eta;
+    const Fl eta = over(dx, d_eta), dce = Fl(8.0f) * eta;
     const float dl = fmaxf(0.0f, div);
     if (!(dl > 0.0f) && K.ssr_exp <= 0.0f && K.ssr_cdF >= 0.0f && dce.v >= 1.001f * K.dx) return K.s_l;
     const Fl asf = Fl(8.0f) * Fl(qexp(over(K.ssr_cdF, dce + Fl((float)SMALL)).v));

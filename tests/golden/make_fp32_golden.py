@@ -3,9 +3,10 @@
     LESGPU_LIB=<build>/liblesgpu.so python tests/golden/make_fp32_golden.py
 
 fp32_ref.npz holds what tests/test_gpu_fp32_form.py compares with: the fields after STEPS steps of
-each case, rounded to FP32.  It was written by the first FP32 build whose runs were compared with
+each case, rounded to FP32, and the SHA-256 of a field of flame speeds.  It was written by the first FP32 build whose runs were compared with
 the FP64 form's (the operations of csrc/les_f32_form.cuh, left to the compiler to contract).
 """
+import hashlib
 import os
 import sys
 
@@ -45,6 +46,25 @@ def state(nx, ny, nz, spikes=False):
     return {k: np.ascontiguousarray(v + np.zeros((nx, ny, nz))) for k, v in st.items()}
 
 
+SPEEDS = (128, 120, 128)
+
+
+def speeds(N):
+    """SHA-256 of the flame speeds of a sheared flow, in which the flame is wrinkled in one cell of seven."""
+    nx, ny, nz = SPEEDS
+    i, j, k = np.meshgrid(np.arange(nx), np.arange(ny), np.arange(nz), indexing="ij")
+    st = state(nx, ny, nz)
+    for f, q in (("u", 7 * i + 3 * j + 5 * k), ("v", 5 * i + 11 * j + 2 * k), ("w", 3 * i + 2 * j + 13 * k)):
+        st[f] = np.abs(q % 16 - 8.0) / 8.0
+    ctx = N.Context(config(nx, ny, nz), precision=N.FP32)
+    ctx.upload_attribute(N.initial_state(config(nx, ny, nz))[0])
+    ctx.upload_state(st)
+    ctx.eval_rhs(0)
+    h = hashlib.sha256(ctx.field("ST").astype(np.float32).tobytes()).hexdigest()
+    ctx.close()
+    return h
+
+
 def main():
     from lesgpu import native as N
     out = {}
@@ -56,6 +76,7 @@ def main():
             out[f"{name}_{f}"] = v.astype(np.float32)
         out[f"{name}_dt"] = np.float64(s.last_dt)
         s.close()
+    out["speeds"] = np.array(speeds(N))
     np.savez_compressed(sys.argv[1] if len(sys.argv) > 1 else os.path.join(HERE, "fp32_ref.npz"), **out)
 
 

@@ -37,6 +37,11 @@ def test_run_is_the_recorded_run(N, case):
     s.close()
 
 
+def test_flame_speeds_are_the_recorded_ones(N):
+    """2e6 cells: the constant that keeps eta's divisor from zero changes five of their speeds."""
+    assert M.speeds(N) == str(np.load(os.path.join(GOLDEN, "fp32_ref.npz"))["speeds"])
+
+
 @pytest.mark.parametrize("case", list(M.CASES))
 def test_every_instance_gives_the_same_bits(N, case):
     """Scalar and flow pass together and apart, 512-thread tiles, the staged scalar pass."""
