@@ -28,7 +28,7 @@ struct Fl {
     friend __device__ __forceinline__ bool operator>=(Fl a, Fl b) { return a.v >= b.v; }
 };
 __device__ __forceinline__ Fl mad(Fl a, Fl b, Fl c) { return __fmaf_rn(a.v, b.v, c.v); }
-__device__ __forceinline__ Fl over(Fl a, Fl b) { return qdiv(a.v, b.v); }
+__device__ __forceinline__ Fl over(Fl a, Fl b) { return qdiv_normal(a.v, b.v); }     // b not subnormal
 __device__ __forceinline__ Fl sum3(Fl a, Fl ra, Fl b, Fl rb, Fl c, Fl rc) { return mad(c, rc, mad(a, ra, b * rb)); }
 
 // ---------------------------------------------------------------------------- properties
@@ -121,8 +121,8 @@ __device__ __forceinline__ bool f32_cell_props(const Consts& C, float T, const f
     o.cp = Cp;
     o.mu_mix = fmaxf(1e-7f, mu.v);
     o.lam = fmaxf(1e-3f, lam.v);
-    o.nu = fmaxf(1e-7f, qdiv(o.mu_mix, rhof));
-    o.aT = qdiv(o.lam, (Fl(rhof) * Fl(Cp)).v);
+    o.nu = fmaxf(1e-7f, qdiv_normal(o.mu_mix, rhof));
+    o.aT = qdiv_normal(o.lam, (Fl(rhof) * Fl(Cp)).v);
     o.alpha = fmaxf(1e-7f, o.aT);
     return true;
 }
@@ -214,7 +214,7 @@ __device__ __forceinline__ Fl f32_weno_half(Fl i0, Fl i1, Fl i2, Fl g0, Fl g1, F
     const Fl eps = 1.0e-6f;
     const Fl e0 = eps + i0, e1 = eps + i1, e2 = eps + i2;
     const Fl a0 = over(g0, e0 * e0), a1 = over(g1, e1 * e1), a2 = over(g2, e2 * e2);
-    const Fl y = over(1.0f, a0 + a1 + a2);
+    const Fl y = qdiv(1.0f, (a0 + a1 + a2).v);
     return sum3(a0 * y, s0, a1 * y, s1, a2 * y, s2);
 }
 __device__ __forceinline__ Fl f32_weno_diff(Fl p0, Fl p1, Fl p2, Fl p3, Fl p4, Fl p5) {
@@ -364,16 +364,14 @@ __device__ __forceinline__ void f32_flow_rhs(const Consts& C, const ModelK<float
 
 // Half the limited slope of a face (:2017-2028, :2058-2094), 0.5 superbee(a / b), to be multiplied by b: a the
 // difference across the face behind, b across the face itself.  superbee takes 0, 1 or 2 over whole ranges
-// of the quotient, and there exact comparisons decide; where it is the quotient or its double, that is the
-// hardware's (__fdividef).
+// of the quotient, and there exact comparisons of |a| and |b| decide; where it is the quotient or its double,
+// that is the hardware's.  A NaN in a gives 2, as the reference's does, and |b| < SMALL too (it sets r = 1e9).
 __device__ __forceinline__ Fl f32_half_superbee(float a, float b) {
-    const float m = fabsf(a), n = fabsf(b), q = qdiv(a, b);
-    float s = fmaxf(fminf(2.0f * q, 1.0f), fminf(q, 2.0f));        // NaN gives 2, as the reference's
-    if (m >= 2.0f * n) s = 2.0f;
-    if (m <= n && m > 0.5f * n) s = 1.0f;
-    if (a == 0.0f || (m == m && signbit(a) != signbit(b))) s = 0.0f;
-    if (n < (float)SMALL) s = 2.0f;
-    return 0.5f * s;
+    const float m = fabsf(a), n = fabsf(b), q = qdiv_normal(a, b);
+    const float low = m > 0.5f * n ? 0.5f : fminf(q, 0.5f);
+    const float high = m >= 2.0f * n ? 1.0f : fmaxf(0.5f, fminf(0.5f * q, 1.0f));
+    const float h = m <= n ? low : high;
+    return n < (float)SMALL ? 1.0f : q < 0.0f ? 0.0f : h;
 }
 
 // One scalar of a cell (:2837-2962): target nudging - advection + molecular + SGS diffusion, c the cell,

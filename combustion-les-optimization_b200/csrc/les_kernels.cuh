@@ -108,9 +108,8 @@ __device__ __forceinline__ void shift_props(PropBuf<R>& P, long long d) {
 // Minimum resident blocks per SM requested from the register allocator (properties / flow /
 // scalar).  Swept on B200 at 256x128x128, ms per step (four launches): FP64 properties 1.13 at 5
 // blocks, 1.11 at 4, 1.16 at 3, 1.32 at 2; flow 0.95 at 5, 0.91 at 4, 1.01 at 3, 1.29 at 2; scalar
-// 1.40 at 5, 1.38 at 4, 1.51 at 3 and 2; FP32 properties 0.54 at 8, 0.505 at 6, 0.513 at 5, 0.536
-// at 4; flow 0.617 at 7, 0.610 at 6 and 5 (at 96x48x48 0.0775, 0.0729, 0.0705), 0.658 at 4; scalar
-// 1.06 at 7, 1.04 at 6, 0.91 at 5, 0.88 at 4.
+// 1.40 at 5, 1.38 at 4, 1.51 at 3 and 2; FP32 properties 0.530 at 6 and 5, 0.560 at 4; flow 0.916
+// at 6, 0.900 at 5, 0.906 at 4; scalar 1.11 at 6 (96x48x48 0.109), 1.14 at 5 (0.097), 1.33 at 3.
 #ifndef LES_MINB_PROPS
 #define LES_MINB_PROPS 4
 #endif
@@ -127,7 +126,7 @@ __device__ __forceinline__ void shift_props(PropBuf<R>& P, long long d) {
 #define LES_MINB_FLOW_F32 5
 #endif
 #ifndef LES_MINB_SCALAR_F32
-#define LES_MINB_SCALAR_F32 4
+#define LES_MINB_SCALAR_F32 5
 #endif
 template <typename R>
 struct MinBlocks {
