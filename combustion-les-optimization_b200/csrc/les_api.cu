@@ -1130,6 +1130,7 @@ int lesgpu_set_tiles(lesgpu_ctx* ctx, const int tiles[5]) {
     DevCtx& d = ctx->d;
     CK(cudaStreamSynchronize(d.stream));
     for (int q = 0; q < les::NSH_CLASSES; q++) d.shape[q] = tiles[q];
+    d.both_shape = -1;
     drop_graph(d);
     return LESGPU_OK;
 }
@@ -1163,6 +1164,7 @@ int lesgpu_autotune(lesgpu_ctx* ctx, int reps, int tiles_out[5], double* ms_out)
     const bool was_timing = d.timing;
     int old[les::NSH_CLASSES];
     for (int q = 0; q < les::NSH_CLASSES; q++) old[q] = d.shape[q];
+    const int old_both = d.both_shape;
     const int cls_of[4] = {LESGPU_K_FILTER, LESGPU_K_STRAIN, LESGPU_K_RHS_FLOW, LESGPU_K_RHS_SCALAR};
     static_assert(les::NSHAPES == LESGPU_NTILES, "tile table and ABI disagree");
     double ms[4][les::NSHAPES];
@@ -1181,6 +1183,23 @@ int lesgpu_autotune(lesgpu_ctx* ctx, int reps, int tiles_out[5], double* ms_out)
             ms[c][t] = (les::shape_allowed(c, t) && d.kcount[cls_of[c]] > 0)
                            ? d.kms[cls_of[c]] / (double)d.kcount[cls_of[c]] : 1e30;
     }
+    // a small grid's steps run the scalar and flow pass in one launch: that one is timed too
+    int both = -1;
+    d.timing = false;
+    if (les::both_passes(d)) {
+        double least = 1e30;
+        for (int t = 0; t < les::NSHAPES_256 && e == cudaSuccess; t++) {
+            d.both_shape = t;
+            d.timing = false;
+            e = (d.precision == LESGPU_FP64) ? les::rhs_only_f64(d, 0, true) : les::rhs_only_f32(d, 0, true);
+            d.timing = true;
+            d.kms[LESGPU_K_RHS_FLOW] = 0.0;
+            for (int r = 0; r < reps && e == cudaSuccess; r++)
+                e = (d.precision == LESGPU_FP64) ? les::rhs_only_f64(d, 0, true) : les::rhs_only_f32(d, 0, true);
+            if (d.kms[LESGPU_K_RHS_FLOW] < least) { least = d.kms[LESGPU_K_RHS_FLOW]; both = t; }
+        }
+    }
+    d.both_shape = both;
     d.timing = was_timing;
     for (int q = 0; q < 8; q++) { d.kms[q] = 0.0; d.kcount[q] = 0; }
     cudaError_t e2 = cudaStreamSynchronize(d.stream);
@@ -1188,6 +1207,7 @@ int lesgpu_autotune(lesgpu_ctx* ctx, int reps, int tiles_out[5], double* ms_out)
     if (e == cudaSuccess) e = cudaMemcpy(d.dS, &saved, sizeof(saved), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         for (int q = 0; q < les::NSH_CLASSES; q++) d.shape[q] = old[q];
+        d.both_shape = old_both;
         return cuda_fail(ctx, e, "autotune");
     }
     int best[les::NSH_CLASSES];

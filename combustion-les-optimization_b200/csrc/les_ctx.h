@@ -136,6 +136,7 @@ struct DevCtx {
     cudaGraphExec_t graph[2] = {};      // captured device-loop steps: one, and several of them
     long long steps_run = 0;            // steps of the session so far
     int shape[NSH_CLASSES] = {0, 0, 0, 0, 0};   // tile (index into kShapes) per kernel class
+    int both_shape = -1;                // autotuned tile of the scalar and flow pass in one launch (both_tile)
     // scalar pass with TMA-staged stencil fields (les_tma.cuh): tensor maps of the six
     // filtered scalars and nu_t (7 CUtensorMap, 128 bytes each), built at create time
     alignas(64) unsigned char tma_maps[7 * 128] = {};
@@ -165,6 +166,27 @@ struct DevCtx {
     std::string err;
 };
 
+// Scalar and flow pass in one launch (k_rhs_both).  On a small grid both passes are short latency
+// chains on a GPU they do not fill, and one launch runs them side by side; on a larger one the flow
+// half's wait for the scalar half costs more than a launch and a tail.  64 steps (32 of
+// 128x64x64), apart -> together: 64x32x32 FP64 9.16 -> 8.24 ms, FP32 7.73 -> 7.22; 80x40x40 FP64 15.1 -> 13.9,
+// FP32 12.7 -> 12.3; 96x48x48 (221k cells) FP64 20.0 -> 19.2, FP32 13.5 -> 13.3; 110x56x54 (333k) FP32 22.4 ->
+// 22.5; 128x64x64 (524k) FP64 21.0 -> 22.0; 191x95x97 66.3 -> 71.4.  The line is at 2^18 cells.  Members of
+// a group keep them apart whatever their size, as together they fill the GPU (six 64x32x32 members:
+// 20.9 -> 25.9).
+constexpr size_t BOTH_CELLS = (size_t)1 << 18;
+inline bool both_passes(const DevCtx& c) {
+    return !c.timing && !c.scalar_tma && !c.in_group && c.n <= BOTH_CELLS;
+}
+
+// Its tile: the autotuner's, which times this launch itself; else the flow or the scalar pass's, where that
+// has 256 threads, as a caller has set them; else the grid's default.
+inline int both_tile(const DevCtx& c) {
+    if (c.both_shape >= 0) return c.both_shape;
+    if (c.shape[SH_FLOW] < NSHAPES_256) return c.shape[SH_FLOW];
+    return c.shape[SH_SCALAR] < NSHAPES_256 ? c.shape[SH_SCALAR] : default_shape(c.nx, c.ny, c.nz);
+}
+
 // Storage size of the tensor maps (7 CUtensorMap of 128 bytes).
 struct TmaMapsStorage {
     unsigned char b[7 * 128];
@@ -188,7 +210,7 @@ cudaError_t umax_f64(DevCtx& c);
 cudaError_t monitor_f64(DevCtx& c);
 cudaError_t probe_f64(DevCtx& c, int n, int kline);
 cudaError_t check_f64(DevCtx& c, int field);
-cudaError_t rhs_only_f64(DevCtx& c, int t_loop);
+cudaError_t rhs_only_f64(DevCtx& c, int t_loop, bool one_launch = false);
 cudaError_t step_f32(DevCtx& c, double dt, int t_loop, bool device_mode);
 // Batched members (les_launch.cuh): step head and tail of one member, the RK stages of nmem
 // members of one shape in one launch per pass.
@@ -198,7 +220,7 @@ cudaError_t batch_stages_f64(DevCtx& c0, const MemberTab* mt, int nmem, cudaStre
 cudaError_t batch_head_f32(DevCtx& c);
 cudaError_t batch_tail_f32(DevCtx& c);
 cudaError_t batch_stages_f32(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t st);
-cudaError_t rhs_only_f32(DevCtx& c, int t_loop);
+cudaError_t rhs_only_f32(DevCtx& c, int t_loop, bool one_launch = false);
 cudaError_t umax_f32(DevCtx& c);
 cudaError_t monitor_f32(DevCtx& c);
 cudaError_t probe_f32(DevCtx& c, int n, int kline);

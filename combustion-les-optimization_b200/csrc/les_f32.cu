@@ -8,7 +8,7 @@ namespace les {
 cudaError_t step_f32(DevCtx& c, double dt, int t_loop, bool device_mode) {
     return step_impl<float>(c, dt, t_loop, device_mode);
 }
-cudaError_t rhs_only_f32(DevCtx& c, int t_loop) { return rhs_only_impl<float>(c, t_loop); }
+cudaError_t rhs_only_f32(DevCtx& c, int t_loop, bool one_launch) { return rhs_only_impl<float>(c, t_loop, one_launch); }
 cudaError_t batch_head_f32(DevCtx& c) { return batch_head<float>(c); }
 cudaError_t batch_tail_f32(DevCtx& c) { return batch_tail<float>(c); }
 cudaError_t batch_stages_f32(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t st) {

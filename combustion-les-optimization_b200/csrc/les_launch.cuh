@@ -143,23 +143,11 @@ static inline void launch_flow(bool pdl, dim3 g, dim3 b, cudaStream_t st, const 
     else launch_flow_part<RK_LAST, R, BATCH>(pdl, g, b, st, hC, attr, F, P, S, St, acc, rn, kd, dS, stage, B);
 }
 
-// Scalar and flow pass in one launch (k_rhs_both).  On a small grid both passes are short latency
-// chains on a GPU they do not fill, and one launch runs them side by side; on a larger one the flow
-// half's wait for the scalar half costs more than a launch and a tail.  64 steps (32 of
-// 128x64x64), apart -> together: 64x32x32 FP64 9.16 -> 8.24 ms, FP32 7.73 -> 7.22; 80x40x40 FP64 15.1 -> 13.9,
-// FP32 12.7 -> 12.3; 96x48x48 (221k cells) FP64 20.0 -> 19.2, FP32 13.5 -> 13.3; 110x56x54 (333k) FP32 22.4 ->
-// 22.5; 128x64x64 (524k) FP64 21.0 -> 22.0; 191x95x97 66.3 -> 71.4.  The line is at 2^18 cells.  Members of
-// a group keep them apart whatever their size, as together they fill the GPU (six 64x32x32 members:
-// 20.9 -> 25.9).
-constexpr size_t BOTH_CELLS = (size_t)1 << 18;
-static inline bool both_passes(const DevCtx& c) {
-    return !c.timing && !c.scalar_tma && !c.in_group && c.n <= BOTH_CELLS;
-}
+// The scalar and flow pass in one launch, where both_passes (les_ctx.h) has it so.
 template <typename R>
 static inline void launch_both(bool pdl, const DevCtx& c, cudaStream_t st, const F11<R>& F, const PropBuf<R>& P,
                                const F11<RS>& S, const F11<R>& St, const AccBuf<R>& acc, const KDbg<R>& kd, int stage) {
-    const int sh = c.shape[SH_FLOW] < NSHAPES_256 ? c.shape[SH_FLOW] : c.shape[SH_SCALAR] < NSHAPES_256 ? c.shape[SH_SCALAR] : 0;
-    const Shape t = kShapes[sh];
+    const Shape t = kShapes[both_tile(c)];
     const int3 tile = make_int3(t.bx, t.by, t.bz);
     const dim3 g((unsigned)((c.nz + t.bx - 1) / t.bx), (unsigned)((c.ny + t.by - 1) / t.by), (unsigned)((c.nx + t.bz - 1) / t.bz));
     if (stage == 0) chain(pdl, k_rhs_both<RK_FIRST, R, RS>, g, 2 * NT, st, c.hC, c.attr, F, P, S, St, acc, kd, c.dS, stage, tile);
@@ -328,9 +316,9 @@ cudaError_t batch_stages(DevCtx& c0, const MemberTab* mt, int nmem, cudaStream_t
 // Stage-1 right-hand side at the current state with the inspection buffers filled (when
 // debug buffers exist); the state itself is not advanced (dt = 0 leaves the stage state
 // equal to Phi_n).  The four kernels are bracketed by the kernel-timing marks, which the
-// tile autotuner reads.
+// tile autotuner reads; with `one_launch` the scalar and flow pass are one, under the flow pass's mark.
 template <typename R>
-cudaError_t rhs_only_impl(DevCtx& c, int t_loop) {
+cudaError_t rhs_only_impl(DevCtx& c, int t_loop, bool one_launch) {
     cudaStream_t st = c.stream;
     if (!part_fits(c, filter_blocks(c), 1)) return cudaErrorInvalidValue;
     F11<RS> S = f11<RS>(c.S);
@@ -351,6 +339,13 @@ cudaError_t rhs_only_impl(DevCtx& c, int t_loop) {
     tm = tmark_begin(c, 2);
     launch_props<R, false>(false, c, cell_grid(c, SH_STRAIN), cell_block(c, SH_STRAIN), st, F, P, 1, Batch{});
     tmark_end(c, tm);
+    if (one_launch) {
+        tm = tmark_begin(c, 3);
+        launch_both<R>(false, c, st, F, P, S, St, acc, kd, 0);
+        tmark_end(c, tm);
+        tmark_flush(c);
+        return cudaGetLastError();
+    }
     tm = tmark_begin(c, 5);
     if (c.scalar_tma && c.tma_ok)
         launch_scalar_tma<R, RS>(c, st, F, P, S, St, acc, rn, kd, 0);

@@ -176,3 +176,28 @@ def test_faces_copy_mass_fractions_before_they_are_renormalised(N, nx, ny, nz):
         n += int(m.sum())
     assert n > 0
     s.close()
+
+
+def test_wide_tiles_leave_a_small_grid_its_launch_shape(N):
+    """A small grid runs the scalar and flow pass in one launch of 256-thread tiles.  Where the tiles set
+    for the two passes have 512, it takes the grid's default, not the first of the table, whose padding
+    costs a fifth of the step on 60x20x40: no more than a tenth above the time without any tiles set."""
+    import time
+    from lesgpu.config import preset
+    cfg = preset("c1").replace(nx=60, ny=20, nz=40, num_vortices=50, initial_flame_front_i=15)
+    best = []
+    for tiles in (None, 9):
+        s = N.Solver(cfg)
+        if tiles:
+            d = s.ctx.get_tiles()
+            s.ctx.set_tiles([d[0], d[1], tiles, tiles, d[4]])
+        s.loop_begin(chunk=200)
+        s.loop_run(200)
+        t = []
+        for _ in range(7):
+            t0 = time.perf_counter()
+            s.loop_run(200)
+            t.append(time.perf_counter() - t0)
+        best.append(min(t))
+        s.close()
+    assert best[1] <= 1.1 * best[0], best
