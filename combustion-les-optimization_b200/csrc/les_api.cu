@@ -1110,6 +1110,11 @@ int lesgpu_selfcheck_division(const double* divisors, int nd, size_t n, unsigned
     return les::selfcheck_division(divisors, nd, n, seed, mismatches);
 }
 
+int lesgpu_selfcheck_math(size_t n, unsigned long long seed, double out[4]) {
+    if (!out || n == 0) return LESGPU_EINVAL;
+    return les::selfcheck_math(n, seed, out);
+}
+
 int lesgpu_sync(lesgpu_ctx* ctx) {
     if (!ctx) return LESGPU_EINVAL;
     CK(cudaStreamSynchronize(ctx->d.stream));

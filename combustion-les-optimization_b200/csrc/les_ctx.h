@@ -204,6 +204,7 @@ void tmark_flush(DevCtx& c);
 // Per-precision entry points (les_f64.cu / les_f32.cu).
 cudaError_t sem_inflow(DevCtx& c, cudaStream_t st);
 int selfcheck_division(const double* divisors, int nd, size_t n, unsigned long long seed, unsigned long long* bad);
+int selfcheck_math(size_t n, unsigned long long seed, double out[4]);
 cudaError_t loop_pre(DevCtx& c, cudaStream_t st);
 cudaError_t step_f64(DevCtx& c, double dt, int t_loop, bool device_mode);
 cudaError_t umax_f64(DevCtx& c);

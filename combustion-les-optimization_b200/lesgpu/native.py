@@ -129,6 +129,7 @@ def lib():
         _sig(L, "lesgpu_mark", C.c_int, [vp, C.c_int])
         _sig(L, "lesgpu_selfcheck_division", C.c_int, [dp, C.c_int, C.c_size_t, C.c_ulonglong,
                                                        C.POINTER(C.c_ulonglong)])
+        _sig(L, "lesgpu_selfcheck_math", C.c_int, [C.c_size_t, C.c_ulonglong, dp])
         _sig(L, "lesgpu_elapsed_ms", C.c_int, [vp, C.c_int, C.c_int, C.POINTER(C.c_double)])
         _sig(L, "lesgpu_device_bytes", C.c_size_t, [vp])
         _sig(L, "lesgpu_bytes_for_grid", C.c_size_t, [C.c_int, C.c_int, C.c_int, C.c_int])
@@ -238,6 +239,16 @@ def selfcheck_division(divisors: Sequence[float], n: int, seed: int = 12345) -> 
     if rc != 0:
         raise LesgpuError(rc, "selfcheck_division")
     return int(bad.value)
+
+
+def selfcheck_math(n: int, seed: int = 12345):
+    """Largest differences of the property pass's routines from CUDA's own functions
+    (lesgpu_selfcheck_math): reciprocal, exponential and quotient in last places, FP32 mismatches."""
+    out = np.zeros(4)
+    rc = lib().lesgpu_selfcheck_math(n, seed, out.ctypes.data)
+    if rc != 0:
+        raise LesgpuError(rc, "selfcheck_math")
+    return out.tolist()
 
 
 def initial_state(cfg: SolverConfig, species: Optional[LesgpuSpecies] = None):

@@ -276,6 +276,12 @@ int lesgpu_kernel_times(lesgpu_ctx* ctx, double* ms, long long* launches, int n)
  * IEEE division.  Runs on the current device; allocates a few bytes of device memory. */
 int lesgpu_selfcheck_division(const double* divisors, int nd, size_t n, unsigned long long seed,
                               unsigned long long* mismatches);
+/* The same for the property pass's routines, against CUDA's own functions on n pseudo-random arguments over the
+ * ranges they are used on.  out[0..2]: largest difference, in units of the result's last place, of the
+ * reciprocal (from 1/x, x of 2^-100..2^100), the table-driven exponential (from exp2(t/16), |t| < 16000)
+ * and the corrected quotient (from a/b); out[3]: FP32 quotients by normal denominators whose bits differ
+ * from the approximate division's. */
+int lesgpu_selfcheck_math(size_t n, unsigned long long seed, double out[4]);
 
 /* Keep |grad G| of every RHS evaluation in a field (grad_G_magnitude_for_debug, :2783,
  * :2820; written to the VTK files, :3579-3583), readable as LESGPU_F_GRAD_G.  Off by default:

@@ -201,3 +201,14 @@ def test_wide_tiles_leave_a_small_grid_its_launch_shape(N):
         best.append(min(t))
         s.close()
     assert best[1] <= 1.1 * best[0], best
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_property_routines_against_cudas_own(N, seed):
+    """The reciprocal (2^-60 and its rounding) and the corrected quotient (half a unit and a rounding) are at most
+    a last place from the correctly rounded ones; the exponential is within 1.1 last places and CUDA's
+    exp2 within one; FP32 quotients by normal denominators have the approximate division's bits."""
+    rcp, ex, quot, differ = N.selfcheck_math(1 << 26, seed)
+    assert rcp <= 1.0 and quot <= 1.0
+    assert ex <= 2.1
+    assert differ == 0
