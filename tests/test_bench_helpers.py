@@ -37,3 +37,15 @@ def test_committed_traffic_covers_the_stage_kernels():
         # a stage moves no more DRAM bytes than its passes' own field counts (halos from L1/L2,
         # no re-reads), within 1 % for the write-back of dirty lines across stages
         assert sum(got) <= 1.01 * sum(alg)
+
+
+def test_pass_bytes_are_what_the_passes_move():
+    """The own fields of each pass against the DRAM bytes ncu counted per launch: no more than them (in part
+    the next pass finds what one wrote in L2), and within a tenth of them."""
+    b = _bench()
+    t = b._traffic_table()
+    for prec, e in (("fp64", 8), ("fp32", 4)):
+        for k in ("filter_props", "strain", "rhs_flow", "rhs_scalar"):
+            own = b.pass_bytes_per_cell(k, e)
+            assert 0.9 * own <= t[(k, "c2", prec)] <= 1.01 * own, (k, prec, own)
+    assert b.pass_bytes_per_cell("rhs_scalar", 8) == 326 and b.pass_bytes_per_cell("rhs_flow", 8) == 194
