@@ -445,7 +445,7 @@ int lesgpu_create(const lesgpu_config* cfg, const lesgpu_species* sp, lesgpu_ctx
     if (cfg->nx < 4 || cfg->ny < 4 || cfg->nz < 4 || cfg->num_vortices < 0) return LESGPU_EINVAL;
     if (cfg->precision != LESGPU_FP64 && cfg->precision != LESGPU_FP32) return LESGPU_EINVAL;
     if ((size_t)cfg->ny * cfg->nz > (size_t)1 << 30 || (size_t)cfg->nx > 65535) return LESGPU_EINVAL;
-    // the kernels index cells in 32 bits and fields of the form's type, with a plane ahead of them, in
+    // the kernels index cells in 32 bits and fields of the form's type, with a plane behind them, in
     // 32 bits of bytes; a grid beyond that has 4/5 of 4 GiB a field at least, 200 GB (FP64) or 240 GB
     // (FP32) in all, so it could not be allocated either
     if (((size_t)cfg->nx + 1) * cfg->ny * cfg->nz > ((size_t)1 << 32) / (cfg->precision == LESGPU_FP32 ? 4 : 8))

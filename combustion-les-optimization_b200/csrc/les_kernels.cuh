@@ -950,25 +950,26 @@ __device__ __forceinline__ R star_rhs(const Star<R>& q, const StarCoef<R>& K, R 
 // Where the scalar pass reads its stencil fields (filtered T and Y_k, nu_t): global memory,
 // or the shared-memory tile of the staged kernel (les_tma.cuh).  Offsets are 32-bit bytes: ten
 // registers instead of twenty for the ten positions of a star (FP64 1.42 -> 1.37 ms per 256x128x128
-// step, FP32 0.87 -> 0.84 with the limiter in minima).  They count from one plane ahead of the
-// field, so that a fluid cell of the first plane, which a caller's attribute map may hold, reads what lies
-// in front of the field in the arena and not 4 GiB behind it.  Fields of 4 GiB less a plane do not
-// fit 59 times (lesgpu_create refuses them).
+// step).  A fluid cell of the first plane, which a caller's attribute map may hold, would be a negative offset
+// away from its neighbour, 4 GiB behind the field in 32 bits: it reads itself (offsets counted from a plane
+// ahead of the field instead: FP64 1.168 -> 1.211, FP32 1.128 -> 1.107).  Fields of 4 GiB less a
+// plane do not fit 59 times (lesgpu_create refuses them).
 template <typename R>
 struct GSrc {
-    const R* T;                         // the fields, less one plane
+    const R* T;
     const R* Y[NSP];
     const R* nut;
     int id, s[3];                       // the cell, the strides
     unsigned c0, up[3], dn[3], uu[3];   // byte offsets of the cell and its neighbours
     __device__ __forceinline__ void orient(const bool (&pos)[3], bool far) {
-        c0 = (unsigned)(id + s[0]) * (unsigned)sizeof(R);
+        c0 = (unsigned)id * (unsigned)sizeof(R);
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            const int o = (pos[a] ? -s[a] : s[a]) * (int)sizeof(R);
-            up[a] = c0 + (unsigned)o;
-            dn[a] = c0 - (unsigned)o;
-            uu[a] = c0 + (unsigned)(far ? 2 * o : o);    // the band's cells have no second neighbour
+            const unsigned b = (unsigned)s[a] * (unsigned)sizeof(R);
+            const unsigned lo = !far && c0 < b ? c0 : c0 - b, hi = c0 + b;
+            up[a] = pos[a] ? lo : hi;
+            dn[a] = pos[a] ? hi : lo;
+            uu[a] = far ? (pos[a] ? lo - b : hi + b) : up[a];    // the band's cells have no second neighbour
         }
     }
     static __device__ __forceinline__ R at(const R* p, unsigned o) {
@@ -999,10 +1000,10 @@ __device__ __forceinline__ GSrc<R> global_source(const F11<R>& F, const PropBuf<
     src.s[0] = ny * nz;
     src.s[1] = nz;
     src.s[2] = 1;
-    src.T = F.p[3] - src.s[0];
+    src.T = F.p[3];
 #pragma unroll
-    for (int s = 0; s < NSP; s++) src.Y[s] = F.p[6 + s] - src.s[0];
-    src.nut = P.nu_t - src.s[0];
+    for (int s = 0; s < NSP; s++) src.Y[s] = F.p[6 + s];
+    src.nut = P.nu_t;
     return src;
 }
 

@@ -37,3 +37,23 @@ def test_fluid_cells_on_every_face(N, nx, ny, nz, prec, staged):
     deep[4:-4, 4:-4, 4:-4] = True
     for k in out[0]:
         np.testing.assert_array_equal(out[0][k][deep], out[1][k][deep], err_msg=k)
+
+
+def test_a_first_plane_of_fluid_reads_within_its_field(N):
+    """Fields that are the same everywhere, all cells fluid: a cell of the first plane that reads beside its
+    field would find another's values there.  No neighbour differs, so nothing but the nudging is left
+    of the scalars' right-hand sides, the same on the first plane as inside."""
+    from lesgpu.config import preset
+    cfg = preset("tiny").replace(nx=8, ny=10, nz=12, lx=0.016, ly=0.02, lz=0.024, num_vortices=20,
+                                 initial_flame_front_i=3, inlet_radius=0.005, seed=11)
+    shape = (cfg.nx, cfg.ny, cfg.nz)
+    ctx = N.Context(cfg)
+    ctx.upload_attribute(np.full(shape, 3))
+    level = {"u": -2.0, "v": -1.0, "w": -1.0, "T": 900.0, "G": 0.0, "rho": 0.4, "Y0": 0.05, "Y1": 0.2, "Y2": 0.7,
+             "Y3": 0.03, "Y4": 0.02}
+    ctx.upload_state({k: np.full(shape, v) for k, v in level.items()})
+    ctx.eval_rhs(0)
+    for k in ["k_T"] + [f"k_Y{s}" for s in range(5)]:
+        x = ctx.field(k)[:-1, :-1, :-1]         # the last planes read what lies behind their field
+        np.testing.assert_array_equal(x[0], np.broadcast_to(x[3, 3, 3], x[0].shape), err_msg=k)
+    ctx.close()
