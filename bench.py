@@ -311,8 +311,8 @@ def run_ours(args):
     tiles = {k: "x".join(map(str, ctx.TILES[t])) for k, t in
              zip(["filter_props", "strain", "rhs_flow", "rhs_scalar", "eos"], ctx.get_tiles())}
     # per step: loop_pre, 2 SEM, 4 x 4 stage kernels, the faces, loop_end
-    # (up to 2^18 cells the scalar and the flow pass are one launch)
-    per_step_launches = 1 + 2 + (16 if cfg.cells > 1 << 18 else 12) + 1 + 1
+    # (up to 2^18 cells, 3 2^16 in FP32, the scalar and the flow pass are one launch)
+    per_step_launches = 1 + 2 + (16 if cfg.cells > (1 << 18 if esz == 8 else 3 << 16) else 12) + 1 + 1
 
     # ---- warm-up (device-resident loop session; graph capture happens here)
     sol.loop_begin(chunk=max(args.warmup, args.steps))

@@ -168,15 +168,15 @@ struct DevCtx {
 
 // Scalar and flow pass in one launch (k_rhs_both).  On a small grid both passes are short latency
 // chains on a GPU they do not fill, and one launch runs them side by side; on a larger one the flow
-// half's wait for the scalar half costs more than a launch and a tail.  64 steps (32 of
-// 128x64x64), apart -> together: 64x32x32 FP64 9.16 -> 8.24 ms, FP32 7.73 -> 7.22; 80x40x40 FP64 15.1 -> 13.9,
-// FP32 12.7 -> 12.3; 96x48x48 (221k cells) FP64 20.0 -> 19.2, FP32 13.5 -> 13.3; 110x56x54 (333k) FP32 22.4 ->
-// 22.5; 128x64x64 (524k) FP64 21.0 -> 22.0; 191x95x97 66.3 -> 71.4.  The line is at 2^18 cells.  Members of
-// a group keep them apart whatever their size, as together they fill the GPU (six 64x32x32 members:
-// 20.9 -> 25.9).
-constexpr size_t BOTH_CELLS = (size_t)1 << 18;
+// half's wait for the scalar half costs more than a launch and a tail.  64 autotuned steps past the
+// WENO switch, apart -> together, ms: 64x32x32 FP64 8.49 -> 7.74, FP32 7.47 -> 7.00; 80x40x40 (128k cells) FP64
+// 13.98 -> 13.86, FP32 11.53 -> 11.16; 96x48x48 (221k) FP64 18.51 -> 18.51, FP32 14.15 -> 14.54; 110x56x54
+// (333k) FP64 28.2 -> 29.3, FP32 22.7 -> 23.6; 128x64x64 (524k) FP64 38.0 -> 40.5, FP32 27.9 -> 30.1.
+// The lines are at 2^18 cells (FP64) and 3 2^16 (FP32).  Members of a group keep them apart whatever their
+// size, as together they fill the GPU (six 64x32x32 members: 20.9 -> 25.9).
 inline bool both_passes(const DevCtx& c) {
-    return !c.timing && !c.scalar_tma && !c.in_group && c.n <= BOTH_CELLS;
+    const size_t most = c.esz == 8 ? (size_t)1 << 18 : (size_t)3 << 16;
+    return !c.timing && !c.scalar_tma && !c.in_group && c.n <= most;
 }
 
 // Its tile: the autotuner's, which times this launch itself; else the flow or the scalar pass's, where that
