@@ -52,8 +52,8 @@ inline size_t max_cell_blocks(int nx, int ny, int nz) {
 
 // The tile of a context that sets none: 32x8x1, or the 256-thread shape that covers the grid with the
 // fewest blocks where that is at least 5 % fewer, since a block of mostly padding costs as much as
-// a full one.  Per step, 32x8x1 -> this choice: 60x20x40 FP64 208 -> 171 us (16x4x4), 70x35x38 FP64 220 -> 185,
-// 138x66x69 FP32 597 -> 538, 152x77x79 FP64 1236 -> 1146; 63x33x31 FP32 177 -> 183; ties (all powers of two)
+// a full one.  Per step, 32x8x1 -> this choice: 60x20x40 FP64 151 -> 122 us (16x4x4), 70x35x38 FP64 221 -> 184,
+// 138x66x69 FP32 699 -> 616, 152x77x79 FP64 1160 -> 1102, 63x33x31 FP32 123 -> 116; ties (all powers of two)
 // keep 32x8x1, which is as good there or better.
 inline int default_shape(int nx, int ny, int nz) {
     int best = 0;

@@ -1,6 +1,7 @@
 // les_f32.cu -- precision form of the solver step: fields stored and advanced in FP32
 // (advection, SGS, sources, properties); the stage <rho_f>, the dt maxima, the monitor
-// sums and the SEM inflow plane are accumulated in FP64.  Built with FMA contraction.
+// sums and the SEM inflow plane are accumulated in FP64.  Built with FMA contraction, which the
+// arithmetic of les_f32_form.cuh leaves no room for.
 #include "les_launch.cuh"
 
 namespace les {

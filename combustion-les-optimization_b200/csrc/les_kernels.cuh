@@ -18,9 +18,10 @@
 // (:2967-3161) in the reference's face order.
 //
 // Every kernel takes the constant table by value (__grid_constant__): divisors, their
-// reciprocals and the species data are read from the constant bank.  FP64 arithmetic is explicit
-// about contraction (the unit is built without it; fma() where it is wanted), so that every
-// instance of a kernel gives the same bits.
+// reciprocals and the species data are read from the constant bank.  The arithmetic is explicit
+// about contraction, so that every instance of a kernel gives the same bits: the FP64 unit is built
+// without it, with fma() where it is wanted, and the FP32 form's right-hand sides and properties are those of
+// les_f32_form.cuh.
 #pragma once
 
 #include <type_traits>
@@ -144,12 +145,10 @@ constexpr int lb_blocks(int minb, int ntb) { return (minb * NT) / ntb > 0 ? (min
 
 // ---------------------------------------------------------------------------- helpers
 
-// The scalar pass reads Phi_n, the RK running sum, the flow pass's right-hand sides and the
-// diffusivities once per stage and writes the running sum back for the next stage only:
-// these go through ld.global.cs / st.global.cs (evict first), so they do not push the
-// stencil fields' halo planes out of L2.  Measured at 256x128x128 on B200: DRAM traffic of
-// the FP64 scalar pass 414-494 B/cell per launch (plain loads 479-531; with an L2 prefetch
-// of these operands 530-622 at 3 % less time); FP32 scalar pass 1.73 -> 1.66 ms per step.
+// The scalar and flow passes read Phi_n and the RK running sum once per stage, the scalar pass the
+// diffusivities too, and write the running sum back for the next stage only: these go through
+// ld.global.cs / st.global.cs (evict first), so they do not push the stencil fields' halo planes out of
+// L2.  The FP64 scalar pass moves 318 bytes a cell per launch so, 326 of them its own fields.
 #ifndef LES_SCALAR_STREAM
 #define LES_SCALAR_STREAM 1
 #endif
@@ -1198,7 +1197,7 @@ __device__ __forceinline__ void touch_line(double* scratch, const double* p) {
 // into L1, where the threads around it find their neighbours.  Scalar pass per step, ms: 128x64x64
 // 0.213 -> 0.201, 191x95x97 0.629 -> 0.595, 256x128x128 1.355 -> 1.186; with the stars alone 1.270,
 // the diffusivities alone 1.300, Phi_n and the running sum as well 1.245, prefetch.global.L1 of the
-// stars 1.30.  The FP32 form, whose stars take half the registers, gains nothing (0.818 -> 0.828).
+// stars 1.30.  The FP32 form, whose stars take half the registers, gained nothing (0.818 -> 0.828).
 template <int PART, typename R, typename RS = R, bool BATCH = false, int NTB = NT>
 __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
     k_rhs_scalar(LES_KERNEL_CONSTS, const uint8_t* __restrict__ attr, F11<R> F, PropBuf<R> P, F11<RS> S0, F11<R> St,
@@ -1254,7 +1253,7 @@ __global__ void __launch_bounds__(NTB, lb_blocks(MinBlocks<R>::scalar, NTB))
 // (8 bytes a cell) instead of four right-hand sides, with this pass updating what it computes,
 // moves 48 bytes a cell less and takes the loads of half the update out of the scalar pass,
 // which waits for memory, into this one, which computes.
-// Everything is in differences across the six faces: a conservative flux m p with the face
+// In FP64 everything is in differences across the six faces: a conservative flux m p with the face
 // value p = p0 + d/2 (first-order upwind next to the boundary: p0 or p0 + d by the sign of m),
 // so convection and diffusion of all three components are two coefficients a face.
 // The right-hand sides of rho u, rho v, rho w and G of one fluid cell.

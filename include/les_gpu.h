@@ -322,8 +322,8 @@ int lesgpu_autotune(lesgpu_ctx* ctx, int reps, int tiles_out[5], double* ms_out)
  * (cp.async.bulk.tensor, a (32 x 8) tile marching through i-planes; the same arithmetic, so
  * the same bits).  Available when a grid row (NZ values) is a multiple of 16 bytes.  Off
  * by default and left alone by lesgpu_autotune: on B200 it is slower than the plain pass
- * (two resident blocks of 112.5 KB shared memory per SM instead of four; FP64 256x128x128 1.43
- * against 1.19 ms per step). */
+ * (two resident blocks of 112.5 KB shared memory per SM instead of four; FP64 256x128x128 1.46
+ * against 1.18 ms per step). */
 int lesgpu_set_scalar_staging(lesgpu_ctx* ctx, int enable);
 int lesgpu_get_scalar_staging(const lesgpu_ctx* ctx);
 
